@@ -1,5 +1,5 @@
-// algos.cu -- connectivity, PageRank and triangle counting over the shared
-// graph view (d_off / d_slots with kSentinel gaps / d_deg).
+// algos.cu -- connectivity and PageRank over the shared graph view (d_off /
+// d_slots with kSentinel gaps / d_deg).
 //
 // Connectivity (SimpleUnionAsync semantics, Connectivity.h:32-136): union-find
 // that always hooks the larger root under the smaller, so every root is the
@@ -13,12 +13,6 @@
 // FP32 state with compensated (TwoSum) per-vertex sums, FP64 L1 residual.
 // Bytes per iteration: 4 B per slot (ids) + 4 B per slot (p_div gather) +
 // 16 B offsets/degrees + 12 B state per vertex.
-//
-// Triangle counting (Triangle.h:167-204): rank by (degree, id) with the
-// device radix sort, keep u->v with rank[u] < rank[v], then count
-// |N+(u) cap N+(v)| per DAG edge with lane groups binary-searching the
-// shorter list in the longer (gbbs/intersect.h:72-151 uses a merge; the count
-// is the same).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -1023,273 +1017,6 @@ int pagerank_run(byo_graph *g, double eps, uint32_t max_iters, int precision, do
     case BYO_PR_FP32: return pagerank_impl<false, float>(g, eps, max_iters, d_p, iters, l1);
     default: return set_error(g->ctx, BYO_EINVAL, "pagerank: unknown precision");
   }
-}
-
-// ================================================================ triangle counting
-
-__global__ void k_tc_rank_keys(const uint32_t *__restrict__ deg, uint64_t n, uint64_t *keys) {
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n;
-       v += (uint64_t)gridDim.x * blockDim.x)
-    keys[v] = ((uint64_t)deg[v] << 32) | v;
-}
-
-__global__ void k_tc_rank_scatter(const uint64_t *__restrict__ sorted, uint64_t n, uint32_t *rank) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    rank[(uint32_t)sorted[i]] = (uint32_t)i;
-}
-
-// out-degree in the DAG: neighbours of higher rank
-__global__ void k_tc_count(const uint64_t *__restrict__ off, const uint32_t *__restrict__ slots,
-                           const uint32_t *__restrict__ rank, uint64_t n, uint32_t *dcnt) {
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t v = gw; v < n; v += nw) {
-    const uint32_t rv = rank[v];
-    const uint64_t b = off[v], e = off[v + 1];
-    uint32_t c = 0;
-    for (uint64_t j = b + lane_id(); j < e; j += 32) {
-      uint32_t u = slots[j];
-      c += (u != kSentinel && rank[u] > rv);
-    }
-    c = warp_sum(c);
-    if (lane_id() == 0) dcnt[v] = c;
-  }
-}
-
-__global__ void k_tc_fill(const uint64_t *__restrict__ off, const uint32_t *__restrict__ slots,
-                          const uint32_t *__restrict__ rank, uint64_t n,
-                          const uint64_t *__restrict__ doff, uint32_t *dn) {
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t v = gw; v < n; v += nw) {
-    const uint32_t rv = rank[v];
-    const uint64_t b = off[v], e = off[v + 1];
-    uint64_t w = doff[v];
-    for (uint64_t base = b; base < e; base += 32) {
-      uint64_t j = base + lane_id();
-      uint32_t u = j < e ? slots[j] : kSentinel;
-      bool keep = u != kSentinel && rank[u] > rv;
-      unsigned m = __ballot_sync(kFull, keep);
-      if (keep) dn[w + __popc(m & lanemask_lt())] = u;
-      w += __popc(m);
-    }
-  }
-}
-
-// Wedge counting over the DAG.  For a vertex u, A = N+(u) is staged in
-// shared memory; every w of N+(v) for v in A is looked up in A by binary
-// search, and each hit is one triangle (u, v, w) with rank(u) < rank(v) <
-// rank(w), so every triangle counts once (Triangle.h:99-150 counts the same
-// |N+(u) cap N+(v)| per DAG edge).  A warp enumerates the wedges of 32 v's at
-// a time flattened by a warp scan over their out-degrees, so lanes stay busy
-// whatever the degrees.
-constexpr uint32_t kTcWarpCap = 512;  // N+(u) a warp stages (2 KB per warp)
-
-__device__ __forceinline__ bool tc_member(const uint32_t *A, uint32_t na, uint32_t x) {
-  uint32_t lo = 0, hi = na;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (A[mid] < x) lo = mid + 1; else hi = mid;
-  }
-  return lo < na && A[lo] == x;
-}
-
-// N+(u) as a sorted array (binary search) or as an open-addressing hash set
-// in shared memory (linear probing, load <= 1/2: about two probes a lookup
-// against log2 |N+(u)| steps).
-struct TcSorted {
-  const uint32_t *A;
-  uint32_t na;
-  __device__ __forceinline__ bool has(uint32_t x) const { return tc_member(A, na, x); }
-};
-struct TcHash {
-  const uint32_t *t;
-  uint32_t mask, shift;
-  __device__ __forceinline__ bool has(uint32_t x) const {
-    uint32_t h = (x * 0x9E3779B1u) >> shift;
-    for (;;) {
-      const uint32_t y = t[h];
-      if (y == x) return true;
-      if (y == kSentinel) return false;
-      h = (h + 1) & mask;
-    }
-  }
-};
-constexpr uint32_t kTcHash = 2 * kTcWarpCap;  // table entries per warp
-
-// Wedges of the v's at positions c, c + stride, ... (chunks of 32) of V =
-// N+(u), each w of N+(v) looked up in S.  Warp-collective; pre/bas are this
-// warp's 32-entry scratch.
-template <class Set>
-__device__ __forceinline__ uint64_t tc_wedges(const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dn,
-                                              const uint32_t *A, uint32_t na, uint32_t c0, uint32_t stride,
-                                              uint32_t *pre, uint64_t *bas, const Set &S) {
-  const unsigned lane = lane_id();
-  uint64_t cnt = 0;
-  for (uint32_t c = c0; c < na; c += stride) {
-    const uint32_t i = c + lane;
-    uint32_t d = 0;
-    uint64_t b = 0;
-    if (i < na) {
-      const uint32_t v = A[i];
-      b = doff[v];
-      d = (uint32_t)(doff[v + 1] - b);
-    }
-    const uint32_t incl = warp_inclusive_scan(d);
-    pre[lane] = incl;
-    bas[lane] = b;
-    __syncwarp();
-    const uint32_t total = __shfl_sync(kFull, incl, 31);
-    uint32_t lo = 0;  // first lane whose inclusive prefix exceeds t: a binary search for
-    if (lane < total) {  // the lane's first t, then a forward walk as t rises by 32
-      uint32_t hi = 31;
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (pre[mid] <= lane) lo = mid + 1; else hi = mid;
-      }
-    }
-    for (uint32_t t = lane; t < total; t += 32) {
-      while (pre[lo] <= t) lo++;
-      const uint32_t start = lo ? pre[lo - 1] : 0;
-      const uint32_t w = dn[bas[lo] + (t - start)];
-      cnt += S.has(w);
-    }
-    __syncwarp();
-  }
-  return cnt;
-}
-
-// A warp per vertex with 2 <= |N+(u)| <= kTcWarpCap: N+(u) goes into a hash
-// set of the next power of two >= 4 |N+(u)| entries (at least 64, at most
-// kTcHash) in the warp's shared memory; the v's are read from the list itself.
-__global__ void __launch_bounds__(256) k_tc_warp(const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dn,
-                                                 uint64_t n, unsigned long long *total) {
-  __shared__ uint32_t Ht[8][kTcHash];
-  __shared__ uint32_t pre[8][32];
-  __shared__ uint64_t bas[8][32];
-  __shared__ unsigned long long sm[9];
-  const unsigned w = threadIdx.x >> 5, lane = lane_id();
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  uint32_t *tab = Ht[w];
-  uint64_t cnt = 0;
-  for (uint64_t u = gw; u < n; u += nw) {
-    const uint64_t ab = doff[u];
-    const uint32_t na = (uint32_t)(doff[u + 1] - ab);
-    if (na < 2 || na > kTcWarpCap) continue;
-    // 2^lg >= 4 na up to the table's kTcHash entries (>= 2 na): load <= 1/4
-    // for most vertices, so a miss (most lookups) ends after ~1.4 probes
-    const uint32_t lg = min(31 - __clz((int)kTcHash), max(6, 32 - __clz((int)(4 * na - 1))));
-    const uint32_t size = 1u << lg, mask = size - 1, shift = 32 - lg;
-    for (uint32_t i = lane; i < size; i += 32) tab[i] = kSentinel;
-    __syncwarp();
-    for (uint32_t i = lane; i < na; i += 32) {
-      const uint32_t x = dn[ab + i];
-      uint32_t h = (x * 0x9E3779B1u) >> shift;
-      while (atomicCAS(tab + h, kSentinel, x) != kSentinel) h = (h + 1) & mask;
-    }
-    __syncwarp();
-    cnt += tc_wedges(doff, dn, dn + ab, na, 0, 32, pre[w], bas[w], TcHash{tab, mask, shift});
-    __syncwarp();
-  }
-  const unsigned long long tot = block_sum((unsigned long long)cnt, sm);
-  if (threadIdx.x == 0 && tot) atomicAdd(total, tot);
-}
-
-// A CTA per vertex with |N+(u)| > kTcWarpCap (listed in big[]); N+(u) is
-// staged in dynamic shared memory when it fits `stage` entries, else read in
-// place.  The CTA's warps take interleaved chunks of 32 v's.
-__global__ void __launch_bounds__(256) k_tc_block(const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dn,
-                                                  const uint32_t *__restrict__ big, const unsigned long long *nbig,
-                                                  uint32_t stage, unsigned long long *total) {
-  extern __shared__ uint32_t Ablk[];
-  __shared__ uint32_t pre[8][32];
-  __shared__ uint64_t bas[8][32];
-  __shared__ unsigned long long sm[9];
-  const unsigned w = threadIdx.x >> 5, nwb = blockDim.x >> 5;
-  const uint64_t nb = *nbig;
-  uint64_t cnt = 0;
-  for (uint64_t k = blockIdx.x; k < nb; k += gridDim.x) {
-    const uint32_t u = big[k];
-    const uint64_t ab = doff[u];
-    const uint32_t na = (uint32_t)(doff[u + 1] - ab);
-    const uint32_t *A = dn + ab;
-    if (na <= stage) {
-      for (uint32_t i = threadIdx.x; i < na; i += blockDim.x) Ablk[i] = dn[ab + i];
-      A = Ablk;
-    }
-    __syncthreads();
-    cnt += tc_wedges(doff, dn, A, na, w * 32, nwb * 32, pre[w], bas[w], TcSorted{A, na});
-    __syncthreads();
-  }
-  const unsigned long long tot = block_sum((unsigned long long)cnt, sm);
-  if (threadIdx.x == 0 && tot) atomicAdd(total, tot);
-}
-
-__global__ void k_tc_big(const uint64_t *__restrict__ doff, uint64_t n, uint32_t *big, unsigned long long *nbig) {
-  for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < n;
-       base += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t u = base + lane_id();
-    const bool b = u < n && doff[u + 1] - doff[u] > kTcWarpCap;
-    const uint64_t at = warp_append(b, nbig);
-    if (b) big[at] = (uint32_t)u;
-  }
-}
-
-int tc_run(byo_graph *g, uint64_t *count) {
-  byo_ctx *ctx = g->ctx;
-  const uint64_t n = g->n;
-  *count = 0;
-  if (n == 0) return BYO_OK;
-  uint64_t *keys = nullptr, *tmp = nullptr;
-  BYO_TRY(ws(g, WS_TC_OFF, 2 * n + 2, &keys));
-  tmp = keys + n + 1;
-  launch(ctx, k_tc_rank_keys, dim3(grid_for(ctx, n, 256)), dim3(256), 0, (const uint32_t *)g->d_deg, n, keys);
-  uint64_t maxdeg_mask = 0xFFFFFFFFull;  // degree bits
-  uint64_t id_mask = sig_mask_for(n) & 0xFFFFFFFFull;
-  uint64_t *sorted = nullptr;
-  BYO_TRY(sort_u64(ctx, keys, tmp, n, (maxdeg_mask << 32) | id_mask, &sorted));
-  uint32_t *rank = nullptr;
-  BYO_TRY(ws(g, WS_TC_RANK, n, &rank));
-  launch(ctx, k_tc_rank_scatter, dim3(grid_for(ctx, n, 256)), dim3(256), 0, (const uint64_t *)sorted, n,
-         rank);
-  uint32_t *dcnt = nullptr;
-  BYO_TRY(ws(g, WS_TC_CNT, n, &dcnt));
-  launch(ctx, k_tc_count, dim3(grid_for(ctx, n * 32, 256, 16)), dim3(256), 0, (const uint64_t *)g->d_off,
-         (const uint32_t *)g->d_slots, (const uint32_t *)rank, n, dcnt);
-  uint64_t *doff = keys;  // reuse: sorted keys no longer needed
-  BYO_TRY(scan_u32_to_u64(ctx, dcnt, n, doff));
-  uint64_t *h = nullptr;
-  BYO_TRY(pinned(ctx, 4096, (void **)&h));
-  BYO_CU(ctx, cudaMemcpyAsync(h, doff + n, 8, cudaMemcpyDeviceToHost, ctx->stream));
-  BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
-  const uint64_t md = h[0];
-  uint32_t *dn = nullptr;
-  BYO_TRY(ws(g, WS_TC_NBR, md + 1, &dn));
-  launch(ctx, k_tc_fill, dim3(grid_for(ctx, n * 32, 256, 16)), dim3(256), 0, (const uint64_t *)g->d_off,
-         (const uint32_t *)g->d_slots, (const uint32_t *)rank, n, (const uint64_t *)doff, dn);
-  unsigned long long *d_total = nullptr;
-  BYO_TRY(ws(g, WS_MISC, 4, (uint32_t **)&d_total));
-  BYO_CU(ctx, cudaMemsetAsync(d_total, 0, 16, ctx->stream));  // total, big count
-  uint32_t *big = dcnt;  // reuse: the counts are in doff now
-  launch(ctx, k_tc_big, dim3(grid_for(ctx, n, 256)), dim3(256), 0, (const uint64_t *)doff, n, big, d_total + 1);
-  launch_t(ctx, "tc_intersect", k_tc_warp, dim3(grid_for(ctx, n * 32, 256, 8)), dim3(256), 0,
-           (const uint64_t *)doff, (const uint32_t *)dn, n, d_total);
-  const byo_tuning tn = effective_tuning(g);
-  const uint32_t stage = tn.tc_stage;
-  static int configured = 0;
-  const int smem = (int)(stage * 4);
-  if (smem > 48 * 1024 && configured < smem) {
-    BYO_CU(ctx, cudaFuncSetAttribute(k_tc_block, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    configured = smem;
-  }
-  launch_t(ctx, "tc_intersect", k_tc_block, dim3(ctx->num_sms), dim3(256), (size_t)smem, (const uint64_t *)doff,
-           (const uint32_t *)dn, (const uint32_t *)big, (const unsigned long long *)(d_total + 1), stage, d_total);
-  BYO_CU(ctx, cudaMemcpyAsync(h, d_total, 8, cudaMemcpyDeviceToHost, ctx->stream));
-  BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
-  *count = h[0];
-  return check_launch(ctx, "triangle_count");
 }
 
 }  // namespace byo

@@ -255,8 +255,9 @@ typedef struct byo_tuning {
   uint32_t ms_push_div;  /* 64-source: push while the frontier's slots < all slots / ms_push_div */
   uint32_t pull_stage_words; /* single-source pull: frontier bitmap words staged in shared memory
                                 (256..49152; fewer words let two CTAs share an SM) */
-  uint32_t tc_stage;     /* triangle counting: DAG out-lists up to this many entries are staged in
-                            a CTA's shared memory, longer ones are searched in place (512..49152) */
+  uint32_t tc_stage;     /* triangle counting: words of shared memory a CTA's map of one out-list may
+                            take (longer maps are counted in parts), and the longest out-list sorted
+                            (512..49152; at most 28672 and 16384 are used) */
   uint32_t reserved;     /* zero */
 } byo_tuning;
 int byo_graph_get_tuning(byo_graph *g, byo_tuning *out);
