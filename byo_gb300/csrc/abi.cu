@@ -80,6 +80,13 @@ void byo_gpu_shutdown(byo_ctx *ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+  for (int i = 0; i < 3; i++) {
+    if (ctx->side[i]) {
+      cudaStreamSynchronize(ctx->side[i]);
+      cudaStreamDestroy(ctx->side[i]);
+    }
+    if (ctx->side_ev[i]) cudaEventDestroy(ctx->side_ev[i]);
+  }
   for (auto &b : ctx->scratch) free_buf(b);
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   for (int i = 0; i < 64; i++)
@@ -890,6 +897,10 @@ int byo_edge_map(byo_graph *g, byo_vertex_subset *vs, byo_functor *f, int64_t th
     o->f.has_list = o->f.has_bits = true;
   }
   if (rc == BYO_OK) rc = check_launch(ctx, "edge_map");
+  // the caller's arrays are written when the call returns (a round with an
+  // output has waited for its counts)
+  if (rc == BYO_OK && (flags & BYO_FL_NO_OUTPUT) && cudaStreamSynchronize(ctx->stream) != cudaSuccess)
+    rc = set_error(ctx, BYO_EDEVICE, "edge_map: synchronise", cudaGetLastError());
   if (rc != BYO_OK) {
     byo_vs_destroy(o);
     return rc;

@@ -20,8 +20,8 @@
 //     per vertex) to those in the frontier, leaving at the first !cond.  A
 //     lane takes a vertex of <= kDenseShort slots; longer runs go to a warp
 //     that loads and tests 32 neighbours at a time and applies the updates in
-//     order (for PR_F / PR_Delta_F: lanes gather the values, one lane adds them
-//     left to right, so sums are bit-identical to a sequential scan).
+//     order.  PR_F and PR_Delta_F have kernels of their own (k_em_sum_lanes,
+//     k_em_sum_warps, k_em_sum_ctas), whose sums are bit-identical to a sequential scan.
 //   dense forward (edgeMapDenseForward, gbbs/edge_map_data.h:180-247): the
 //     frontier's members push with updateAtomic, as the sparse round does.
 // The output is a list and a bitmap kept together (the engine's Frontier).
@@ -32,6 +32,7 @@
 #include "device.cuh"
 #include "engine.h"
 #include "internal.h"
+#include "seqsum.cuh"
 
 namespace byo {
 
@@ -203,46 +204,6 @@ __device__ __forceinline__ bool warp_pull_run(const F &f, uint32_t v, const uint
   return marked;
 }
 
-// Sums (PR_F, PR_Delta_F): lanes gather 32 values, lane 0 adds them in order.
-template <class F>
-__device__ __forceinline__ bool warp_pull_sum(double *acc_at, bool zero_marks, const F &f, const uint32_t *slots,
-                                              uint64_t b, uint64_t e, const uint32_t *fb) {
-  double acc = 0.0;
-  bool marked = false;
-  if (lane_id() == 0) acc = *acc_at;
-  for (uint64_t base = b; base < e; base += 32) {
-    const uint64_t j = base + lane_id();
-    const uint32_t u = j < e ? slots[j] : kSentinel;
-    const bool in = u != kSentinel && test_bit(fb, u);
-    const double x = in ? f.value(u) : 0.0;
-    unsigned m = __ballot_sync(kFull, in);
-    while (m) {
-      const int k = __ffs(m) - 1;
-      m &= m - 1;
-      const double xk = __shfl_sync(kFull, x, k);
-      if (lane_id() == 0) {
-        marked |= zero_marks ? acc == 0.0 : true;
-        acc = __dadd_rn(acc, xk);
-      }
-    }
-  }
-  if (lane_id() == 0) *acc_at = acc;
-  return __shfl_sync(kFull, marked ? 1 : 0, 0) != 0;
-}
-
-__device__ __forceinline__ bool warp_pull(const LabelF &f, uint32_t v, const uint32_t *slots, uint64_t b, uint64_t e,
-                                          const uint32_t *fb) {
-  return warp_pull_run(f, v, slots, b, e, fb);
-}
-__device__ __forceinline__ bool warp_pull(const PrF &f, uint32_t v, const uint32_t *slots, uint64_t b, uint64_t e,
-                                          const uint32_t *fb) {
-  return warp_pull_sum(f.pn + v, false, f, slots, b, e, fb);
-}
-__device__ __forceinline__ bool warp_pull(const PrDeltaF &f, uint32_t v, const uint32_t *slots, uint64_t b,
-                                          uint64_t e, const uint32_t *fb) {
-  return warp_pull_sum(f.ngh + v, true, f, slots, b, e, fb);
-}
-
 template <class F>
 __global__ void __launch_bounds__(256) k_em_pull_long(const uint64_t *__restrict__ off,
                                                       const uint32_t *__restrict__ slots,
@@ -257,12 +218,296 @@ __global__ void __launch_bounds__(256) k_em_pull_long(const uint64_t *__restrict
   for (uint64_t i = gw; i < nd; i += nw) {
     const uint32_t v = defer[i];
     bool marked = false;
-    if (__shfl_sync(kFull, f.cond(v) ? 1 : 0, 0)) marked = warp_pull(f, v, slots, off[v], off[v + 1], fb);
+    if (__shfl_sync(kFull, f.cond(v) ? 1 : 0, 0)) marked = warp_pull_run(f, v, slots, off[v], off[v + 1], fb);
     const bool want = lane_id() == 0 && marked && output;
     emit_out(want, v, out_list, out_bits, deg, cnt, outdeg);
   }
   outdeg = warp_sum(outdeg);
   if (lane_id() == 0 && outdeg) atomicAdd(cnt + 1, (unsigned long long)outdeg);
+}
+
+// ---------------------------------------------------------------- dense rounds of the sums
+// Runs in classes of similar length, each a list of vertices: a lane takes a
+// run of the first ones, a warp one of the next to last and a CTA one of the
+// last.  A warp's FP64 addition takes the pipe 19 cycles however many lanes
+// add, so 32 runs of one length cost a warp what a single one would.
+constexpr uint32_t kSumLaneMax = 128;
+constexpr int kSumLanes = 11, kSumWarp = kSumLanes, kSumCta = kSumLanes + 1, kSumClasses = kSumLanes + 2;
+__device__ __forceinline__ int sum_class(uint64_t len) {  // 1..2, 3..4, ..8, ..12, ..16, 24, 32, .. kSumLaneMax
+  if (len <= 8) return len <= 2 ? 0 : len <= 4 ? 1 : 2;
+  if (len > kSumLaneMax) return len <= 4096 ? kSumWarp : kSumCta;
+  const int lg = 31 - __clz((int)len - 1);  // 8 < len: len - 1 in [2^lg, 2^(lg+1))
+  return 3 + 2 * (lg - 3) + (int)(((len - 1) >> (lg - 1)) & 1);
+}
+struct SumPlan {
+  uint32_t *list;             // the classes' vertices, one class after the other
+  unsigned long long *count;  // [kSumClasses] vertices, [kSumClasses] cursors, [1] next warp run
+};
+
+// What one neighbour adds: a value computed once per vertex (PR_F: n divisions
+// instead of one an edge; FP64 division is slow here), or read in place.
+struct SumArgs {
+  const uint64_t *off;
+  const uint32_t *slots;
+  const uint32_t *deg;
+  const uint32_t *fb;    // the frontier; null: every vertex
+  const double *val;     // value of vertex u at val[u * stride + at]
+  uint32_t stride, at;
+  uint64_t n;
+  double *sum;
+  int zero_marks, output;
+  uint32_t *out_list, *out_bits;
+  unsigned long long *cnt;  // members out, their degrees
+  SumPlan plan;
+  __device__ double value(uint32_t u) const { return __ldg(val + (uint64_t)u * stride + at); }
+  __device__ bool member(uint32_t u) const { return u != kSentinel && (!fb || test_bit(fb, u)); }
+};
+
+// kPlace = false counts the classes, true writes the lists: a CTA counts its
+// 4096 vertices in shared memory and takes a place in each list at once.
+template <bool kPlace>
+__global__ void __launch_bounds__(1024) k_sum_plan(const uint64_t *__restrict__ off, uint64_t n, SumPlan p) {
+  __shared__ unsigned int cnt[kSumClasses];
+  __shared__ unsigned long long at[kSumClasses];
+  for (uint64_t base = blockIdx.x * 4096ull; base < n; base += gridDim.x * 4096ull) {
+    if (threadIdx.x < kSumClasses) cnt[threadIdx.x] = 0;
+    __syncthreads();
+    int c[4];
+    unsigned int slot[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const uint64_t v = base + q * 1024 + threadIdx.x;
+      const uint64_t len = v < n ? off[v + 1] - off[v] : 0;
+      c[q] = len ? sum_class(len) : -1;
+      const unsigned peers = __match_any_sync(kFull, c[q]);
+      const int leader = __ffs(peers) - 1;
+      unsigned int b = 0;
+      if (c[q] >= 0 && (int)lane_id() == leader) b = atomicAdd(cnt + c[q], (unsigned)__popc(peers));
+      slot[q] = __shfl_sync(kFull, b, leader) + __popc(peers & lanemask_lt());
+    }
+    __syncthreads();
+    if (threadIdx.x < kSumClasses && cnt[threadIdx.x]) {
+      unsigned long long start = 0;
+      if (kPlace)
+        for (int k = 0; k < (int)threadIdx.x; k++) start += p.count[k];
+      at[threadIdx.x] = start + atomicAdd(p.count + (kPlace ? kSumClasses : 0) + threadIdx.x,
+                                          (unsigned long long)cnt[threadIdx.x]);
+    }
+    __syncthreads();
+    if (kPlace) {
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (c[q] >= 0) p.list[at[c[q]] + slot[q]] = (uint32_t)(base + q * 1024 + threadIdx.x);
+    }
+    __syncthreads();
+  }
+}
+
+__global__ void k_em_values(PrF f, uint64_t n, double *val) {
+  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
+    val[v] = f.value((uint32_t)v);
+}
+
+// A lane per run: 32 runs of one class, kWin terms of each at a time gathered
+// by the whole warp (the runs' ids in pieces of kWin) and staged, then added
+// by the runs' lanes.  Bound by a warp's own chain (64 cycles an FP64 addition,
+// two gathers a window), so longer runs than kSumLaneMax are composed by a warp
+// instead: with lanes up to 512 slots, one warp's 32 windows took 285 us.
+// Chung-Lu n = 10^6, 16 M edges: 90 us a round; a lane that walked its own run
+// of up to 64 slots with a division for every term took 270.
+template <int kWin>
+__device__ __forceinline__ void sum_lane_runs(const SumArgs &a, const uint32_t *list, uint64_t runs, uint64_t group,
+                                              double *stage, uint64_t &outdeg) {
+  const unsigned lane = lane_id();
+  const uint64_t i = group * 32 + lane;
+  uint32_t v = 0;
+  uint64_t b = 0;
+  uint32_t len = 0;
+  if (i < runs) {
+    v = list[i];
+    b = a.off[v];
+    len = (uint32_t)(a.off[v + 1] - b);
+  }
+  double acc = len ? a.sum[v] : 0.0;
+  bool any = false, zero = false;
+  for (uint32_t w0 = 0; __ballot_sync(kFull, w0 < len); w0 += kWin) {
+    uint32_t u[kWin];
+#pragma unroll
+    for (int q = 0; q < kWin; q++) {  // position q * 32 + lane: run / kWin, term % kWin
+      const int run = q * (32 / kWin) + lane / kWin;
+      const uint32_t k = w0 + lane % kWin;
+      const uint64_t rb = __shfl_sync(kFull, b, run);
+      const uint32_t rl = __shfl_sync(kFull, len, run);
+      u[q] = k < rl ? a.slots[rb + k] : kSentinel;
+    }
+    uint32_t has = 0;
+#pragma unroll
+    for (int q = 0; q < kWin; q++) {
+      const bool in = a.member(u[q]);
+      if (in) stage[(q * (32 / kWin) + lane / kWin) * (kWin + 1) + lane % kWin] = a.value(u[q]);
+      const unsigned m = __ballot_sync(kFull, in);
+      if ((int)(lane / (32 / kWin)) == q) has = m >> (lane % (32 / kWin) * kWin);
+    }
+    __syncwarp();
+    has &= (1u << kWin) - 1u;
+    any |= has != 0;
+#pragma unroll
+    for (int k = 0; k < kWin; k++)
+      if ((has >> k) & 1u) {
+        zero |= seq_zero(acc);
+        acc = __dadd_rn(acc, stage[lane * (kWin + 1) + k]);
+      }
+    __syncwarp();
+  }
+  if (any) a.sum[v] = acc;
+  emit_out(a.output && (a.zero_marks ? zero : any), v, a.out_list, a.out_bits, a.deg, a.cnt, outdeg);
+}
+
+__global__ void __launch_bounds__(256) k_em_sum_lanes(SumArgs a) {
+  __shared__ double stage[8][32 * 17];
+  __shared__ uint64_t first[kSumLanes + 1], vert[kSumLanes + 1];  // groups and vertices before each class
+  if (threadIdx.x == 0) {
+    uint64_t g = 0, v = 0;
+    for (int c = 0; c < kSumLanes; c++) {
+      first[c] = g;
+      vert[c] = v;
+      g += (a.plan.count[c] + 31) / 32;
+      v += a.plan.count[c];
+    }
+    first[kSumLanes] = g;
+    vert[kSumLanes] = v;
+  }
+  __syncthreads();
+  // neighbouring groups, which are of one length, on different SMs
+  const uint64_t gw = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  double *st = stage[threadIdx.x >> 5];
+  uint64_t outdeg = 0;
+  int c = kSumLanes - 1;  // the longest runs first
+  for (uint64_t t = gw; t < first[kSumLanes]; t += nw) {
+    const uint64_t g = first[kSumLanes] - 1 - t;
+    while (g < first[c]) c--;
+    const uint32_t *list = a.plan.list + vert[c];
+    const uint64_t runs = vert[c + 1] - vert[c];
+    if (c <= 1)
+      sum_lane_runs<4>(a, list, runs, g - first[c], st, outdeg);
+    else if (c == 2)
+      sum_lane_runs<8>(a, list, runs, g - first[c], st, outdeg);
+    else
+      sum_lane_runs<16>(a, list, runs, g - first[c], st, outdeg);
+  }
+  outdeg = warp_sum(outdeg);
+  if (lane_id() == 0 && outdeg) atomicAdd(a.cnt + 1, (unsigned long long)outdeg);
+}
+
+// Runs above 4096 slots, a CTA each (seqsum.cuh), 4096 neighbours a step: bound by
+// the largest hub's steps (1.4 us each).  Chung-Lu n = 10^6, whose hub has 500 K
+// neighbours: 172 us a round; one lane adding a warp's values in turn took 20 ms.
+// 64 registers instead of 128 spill the loads in flight: 364 us.
+constexpr int kSumBlock = 512, kSumTerms = 8;
+__global__ void __launch_bounds__(kSumBlock, 1) k_em_sum_ctas(SumArgs a) {
+  __shared__ double stage[seq_at<kSumTerms>(kSumTerms * kSumBlock)];
+  __shared__ uint32_t mask[kSumTerms * kSumBlock / 32];
+  __shared__ uint64_t sums[2][32];
+  __shared__ SeqSum shared;
+  const SeqBlockMem mem{stage, mask, sums, &shared};
+  uint64_t start = 0;
+  for (int c = 0; c < kSumCta; c++) start += a.plan.count[c];
+  const uint32_t *runs = a.plan.list + start;
+  const uint64_t ncta = a.plan.count[kSumCta];
+  uint64_t outdeg = 0;
+  unsigned turn = 0;
+  for (uint64_t i = blockIdx.x; i < ncta; i += gridDim.x) {
+    const uint32_t v = runs[i];
+    const uint64_t b = a.off[v], e = a.off[v + 1];
+    SeqSum s{a.sum[v], false, false};
+    // the values of the next step and the ids of the one after it load while
+    // a step is added
+    uint32_t u[kSumTerms];
+    double x[kSumTerms];
+    unsigned in = 0;
+    auto ids = [&](uint64_t j0) {
+#pragma unroll
+      for (int r = 0; r < kSumTerms; r++) {
+        const uint64_t j = j0 + r * kSumBlock + threadIdx.x;
+        u[r] = j < e ? a.slots[j] : kSentinel;
+      }
+    };
+    auto values = [&]() {
+      in = 0;
+#pragma unroll
+      for (int r = 0; r < kSumTerms; r++) {
+        const bool has = a.member(u[r]);
+        in |= (has ? 1u : 0u) << r;
+        x[r] = has ? a.value(u[r]) : 0.0;
+      }
+    };
+    constexpr uint64_t kStep = kSumTerms * kSumBlock;
+    ids(b);
+    values();
+    ids(b + kStep);
+    for (uint64_t j = b; j < e; j += kStep) {
+      double y[kSumTerms];
+#pragma unroll
+      for (int r = 0; r < kSumTerms; r++) y[r] = x[r];
+      const unsigned had = in;
+      values();
+      ids(j + 2 * kStep);
+      seq_block(s, y, had, mem, turn++);
+    }
+    if (threadIdx.x < 32) {
+      if (threadIdx.x == 0 && s.any) a.sum[v] = s.acc;
+      emit_out(threadIdx.x == 0 && a.output && (a.zero_marks ? s.zero : s.any), v, a.out_list, a.out_bits, a.deg,
+               a.cnt, outdeg);
+    }
+  }
+  if (threadIdx.x == 0 && outdeg) atomicAdd(a.cnt + 1, (unsigned long long)outdeg);
+}
+
+// Runs of kSumLaneMax to 4096 slots, a warp each, 256 neighbours a step: 108 us a
+// round on the same graph (with the lanes' and the CTAs' runs side by side).
+__global__ void __launch_bounds__(256) k_em_sum_warps(SumArgs a) {
+  __shared__ double stages[8][seq_at<8>(256)];
+  __shared__ uint32_t masks[8][8];
+  const unsigned lane = lane_id();
+  double *stage = stages[threadIdx.x >> 5];
+  uint32_t *mask = masks[threadIdx.x >> 5];
+  uint64_t start = 0;
+  for (int c = 0; c < kSumWarp; c++) start += a.plan.count[c];
+  const uint32_t *runs = a.plan.list + start;
+  const uint64_t nwarp = a.plan.count[kSumWarp];
+  uint64_t outdeg = 0;
+  for (;;) {
+    unsigned long long i = 0;
+    if (lane == 0) i = atomicAdd(a.plan.count + 2 * kSumClasses, 1ull);
+    i = __shfl_sync(kFull, i, 0);
+    if (i >= nwarp) break;
+    const uint32_t v = runs[i];
+    const uint64_t b = a.off[v], e = a.off[v + 1];
+    SeqSum s{a.sum[v], false, false};
+    for (uint64_t j0 = b; j0 < e; j0 += 256) {
+      uint32_t u[8];
+#pragma unroll
+      for (int r = 0; r < 8; r++) u[r] = j0 + r * 32 + lane < e ? a.slots[j0 + r * 32 + lane] : kSentinel;
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        const bool has = a.member(u[r]);
+        const unsigned word = __ballot_sync(kFull, has);
+        stage[seq_at<8>(r * 32 + lane)] = has ? a.value(u[r]) : 0.0;
+        if (lane == 0) mask[r] = word;
+      }
+      __syncwarp();
+      double x[8];
+#pragma unroll
+      for (int r = 0; r < 8; r++) x[r] = stage[seq_at<8>(8 * lane + r)];
+      seq_warp(s, x, reinterpret_cast<const unsigned char *>(mask)[lane]);
+      __syncwarp();
+    }
+    if (lane == 0 && s.any) a.sum[v] = s.acc;
+    emit_out(lane == 0 && a.output && (a.zero_marks ? s.zero : s.any), v, a.out_list, a.out_bits, a.deg, a.cnt, outdeg);
+  }
+  outdeg = warp_sum(outdeg);
+  if (lane == 0 && outdeg) atomicAdd(a.cnt + 1, (unsigned long long)outdeg);
 }
 
 // ---------------------------------------------------------------- frontier forms
@@ -370,22 +615,45 @@ __global__ void __launch_bounds__(256) k_vertex_op(VOp o, const uint32_t *__rest
 
 // Sum of |a[i] - b[i]| in 4096-vertex chunks (each summed in order), then
 // the chunks in order: the oracle's reduction order, so the value is the
-// oracle's to the last bit on the same inputs.
+// oracle's to the last bit on the same inputs.  A CTA per chunk (seqsum.cuh);
+// a thread per chunk took 800 us at n = 10^6, 51 here.
 constexpr uint64_t kL1Chunk = 4096;
-__global__ void k_l1_chunks(const double *__restrict__ a, const double *__restrict__ b, uint64_t n, double *part) {
+constexpr int kL1Block = 512, kL1Terms = 8;
+template <class Term>
+__device__ __forceinline__ double block_seq_sum(Term term, uint64_t lo, uint64_t hi) {
+  __shared__ double stage[seq_at<kL1Terms>(kL1Terms * kL1Block)];
+  __shared__ uint32_t mask[kL1Terms * kL1Block / 32];
+  __shared__ uint64_t sums[2][32];
+  __shared__ SeqSum shared;
+  const SeqBlockMem mem{stage, mask, sums, &shared};
+  SeqSum s{0.0, false, false};
+  unsigned turn = 0;
+  for (uint64_t i0 = lo; i0 < hi; i0 += kL1Terms * kL1Block) {
+    double x[kL1Terms];
+    unsigned in = 0;
+#pragma unroll
+    for (int r = 0; r < kL1Terms; r++) {
+      const uint64_t i = i0 + r * kL1Block + threadIdx.x;
+      in |= (i < hi ? 1u : 0u) << r;
+      x[r] = i < hi ? term(i) : 0.0;
+    }
+    seq_block(s, x, in, mem, turn++);
+  }
+  __syncthreads();
+  return s.acc;
+}
+__global__ void __launch_bounds__(kL1Block, 2) k_l1_chunks(const double *__restrict__ a, const double *__restrict__ b,
+                                                        uint64_t n, double *part) {
   const uint64_t nch = (n + kL1Chunk - 1) / kL1Chunk;
-  for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < nch; c += (uint64_t)gridDim.x * blockDim.x) {
-    double acc = 0.0;
-    const uint64_t hi = (c + 1) * kL1Chunk < n ? (c + 1) * kL1Chunk : n;
-    for (uint64_t i = c * kL1Chunk; i < hi; i++) acc = __dadd_rn(acc, fabs(__dsub_rn(a[i], b[i])));
-    part[c] = acc;
+  for (uint64_t c = blockIdx.x; c < nch; c += gridDim.x) {
+    const double s = block_seq_sum([&](uint64_t i) { return fabs(__dsub_rn(a[i], b[i])); }, c * kL1Chunk,
+                                   min((c + 1) * kL1Chunk, n));
+    if (threadIdx.x == 0) part[c] = s;
   }
 }
-__global__ void k_l1_total(const double *__restrict__ part, uint64_t nch, double *out) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  double s = 0.0;
-  for (uint64_t c = 0; c < nch; c++) s = __dadd_rn(s, part[c]);
-  *out = s;
+__global__ void __launch_bounds__(kL1Block) k_l1_total(const double *__restrict__ part, uint64_t nch, double *out) {
+  const double s = block_seq_sum([&](uint64_t c) { return part[c]; }, 0, nch);
+  if (threadIdx.x == 0) *out = s;
 }
 
 __global__ void k_fill_f64(double *a, uint64_t n, double x) {
@@ -393,22 +661,96 @@ __global__ void k_fill_f64(double *a, uint64_t n, double x) {
     a[i] = x;
 }
 
+// The runs of g in classes, for any number of rounds while g stays as it is.
+int sum_plan(byo_graph *g, SumPlan *p) {
+  byo_ctx *ctx = g->ctx;
+  BYO_TRY(ws(g, WS_DEFER, g->n + 1, &p->list));
+  BYO_TRY(ws(g, WS_BUCKETS, 2 * kSumClasses + 1, &p->count));
+  BYO_CU(ctx, cudaMemsetAsync(p->count, 0, (2 * kSumClasses + 1) * 8, ctx->stream));
+  const dim3 grid(grid_for(ctx, (g->n + 3) / 4, 1024, 2));
+  launch(ctx, k_sum_plan<false>, grid, dim3(1024), 0, (const uint64_t *)g->d_off, g->n, *p);
+  launch(ctx, k_sum_plan<true>, grid, dim3(1024), 0, (const uint64_t *)g->d_off, g->n, *p);
+  return check_launch(ctx, "edge_map plan");
+}
+
+// A dense round of a functor that sums (PR_F, PR_Delta_F).
+int sum_round(byo_graph *g, SumArgs a, Frontier &in, Frontier &out, bool output, unsigned long long *cnt,
+              const SumPlan *plan) {
+  byo_ctx *ctx = g->ctx;
+  a.fb = nullptr;
+  if (!in.all) {  // (a list may hold an id twice, so its size does not tell)
+    BYO_TRY(ensure_bits(g, in));
+    a.fb = in.bits;
+  }
+  if (plan) a.plan = *plan; else BYO_TRY(sum_plan(g, &a.plan));
+  BYO_CU(ctx, cudaMemsetAsync(a.plan.count + 2 * kSumClasses, 0, 8, ctx->stream));
+  a.off = g->d_off;
+  a.slots = g->d_slots;
+  a.deg = g->d_deg;
+  a.n = g->n;
+  a.output = output ? 1 : 0;
+  a.out_list = out.list;
+  a.out_bits = out.bits;
+  a.cnt = cnt;
+  // the three take vertices of their own: side by side, the longest runs' few
+  // CTAs leave room for the rest
+  BYO_TRY(side_fork(ctx, 0));
+  BYO_TRY(side_fork(ctx, 1));
+  k_em_sum_ctas<<<ctx->num_sms, kSumBlock, 0, ctx->side[0]>>>(a);
+  k_em_sum_warps<<<grid_for(ctx, g->nslots / kSumLaneMax * 32, 256), 256, 0, ctx->side[1]>>>(a);
+  ctx->launches += 2;
+  launch(ctx, k_em_sum_lanes, dim3(grid_for(ctx, g->n, 256)), dim3(256), 0, a);
+  BYO_TRY(side_join(ctx, 0));
+  BYO_TRY(side_join(ctx, 1));
+  return check_launch(ctx, "edge_map");
+}
+
+int pull_round(byo_graph *g, const PrF &f, Frontier &in, Frontier &out, bool output, unsigned long long *cnt,
+               const SumPlan *plan) {
+  SumArgs a{};
+  double *val = nullptr;
+  BYO_TRY(ws(g, WS_PR_D, g->n + 1, &val));
+  launch(g->ctx, k_em_values, dim3(grid_for(g->ctx, g->n, 256)), dim3(256), 0, f, g->n, val);
+  a.val = val;
+  a.stride = 1;
+  a.sum = f.pn;
+  return sum_round(g, a, in, out, output, cnt, plan);
+}
+
+int pull_round(byo_graph *g, const PrDeltaF &f, Frontier &in, Frontier &out, bool output, unsigned long long *cnt,
+               const SumPlan *plan) {
+  SumArgs a{};
+  a.val = f.delta;
+  a.stride = 2;
+  a.at = 1;
+  a.sum = f.ngh;
+  a.zero_marks = 1;
+  return sum_round(g, a, in, out, output, cnt, plan);
+}
+
+int pull_round(byo_graph *g, const LabelF &f, Frontier &in, Frontier &out, bool output, unsigned long long *cnt,
+               const SumPlan *) {
+  byo_ctx *ctx = g->ctx;
+  BYO_TRY(ensure_bits(g, in));
+  uint32_t *defer = nullptr;
+  BYO_TRY(ws(g, WS_DEFER, g->n + 1, &defer));
+  const dim3 grid(grid_for(ctx, (g->n + 31) / 32 * 32, 256));
+  launch(ctx, k_em_pull<LabelF>, grid, dim3(256), 0, (const uint64_t *)g->d_off, (const uint32_t *)g->d_slots,
+         (const uint32_t *)g->d_deg, f, (const uint32_t *)in.bits, g->n, output ? 1 : 0, out.list, out.bits, cnt,
+         defer);
+  launch(ctx, k_em_pull_long<LabelF>, grid, dim3(256), 0, (const uint64_t *)g->d_off, (const uint32_t *)g->d_slots,
+         (const uint32_t *)g->d_deg, f, (const uint32_t *)in.bits, output ? 1 : 0, out.list, out.bits, cnt,
+         (const uint32_t *)defer);
+  return check_launch(ctx, "edge_map");
+}
+
 template <class F>
 int run_round(byo_graph *g, const F &f, Frontier &in, Frontier &out, int mode, bool output,
-              unsigned long long *cnt) {
+              unsigned long long *cnt, const SumPlan *plan) {
   byo_ctx *ctx = g->ctx;
   const int block = 256;
   if (mode == MODE_PULL) {
-    BYO_TRY(ensure_bits(g, in));
-    uint32_t *defer = nullptr;
-    BYO_TRY(ws(g, WS_DEFER, g->n + 1, &defer));
-    const uint64_t W = (g->n + 31) / 32;
-    launch(ctx, k_em_pull<F>, dim3(grid_for(ctx, W * 32, block)), dim3(block), 0, (const uint64_t *)g->d_off,
-           (const uint32_t *)g->d_slots, (const uint32_t *)g->d_deg, f, (const uint32_t *)in.bits, g->n,
-           output ? 1 : 0, out.list, out.bits, cnt, defer);
-    launch(ctx, k_em_pull_long<F>, dim3(grid_for(ctx, W * 32, block)), dim3(block), 0, (const uint64_t *)g->d_off,
-           (const uint32_t *)g->d_slots, (const uint32_t *)g->d_deg, f, (const uint32_t *)in.bits, output ? 1 : 0,
-           out.list, out.bits, cnt, (const uint32_t *)defer);
+    BYO_TRY(pull_round(g, f, in, out, output, cnt, plan));
   } else {  // sparse, blocked and dense forward: updateAtomic from the members
     BYO_TRY(ensure_list(g, in));
     if (in.size)
@@ -446,29 +788,37 @@ int frontier_from_bits(byo_graph *g, const uint32_t *d_bits, Frontier &f) {
   f.has_bits = true;
   f.has_list = false;
   f.dense = true;
+  f.all = d_bits == nullptr;
   BYO_TRY(ensure_list(g, f));
   return BYO_OK;
 }
 
-int generic_edge_map(byo_graph *g, const FunctorArgs &fa, Frontier &in, Frontier &out, int mode, bool output) {
+static int edge_map_planned(byo_graph *g, const FunctorArgs &fa, Frontier &in, Frontier &out, int mode, bool output,
+                            const SumPlan *plan) {
   byo_ctx *ctx = g->ctx;
   unsigned long long *cnt = nullptr;
-  BYO_TRY(ws(g, WS_STATS, 4, (uint64_t **)&cnt));
-  BYO_CU(ctx, cudaMemsetAsync(cnt, 0, 32, ctx->stream));
+  BYO_TRY(ws(g, WS_STATS, 8, (uint64_t **)&cnt));
+  BYO_CU(ctx, cudaMemsetAsync(cnt, 0, 64, ctx->stream));
   switch (fa.kind) {
-    case BYO_F_BFS_LABEL: BYO_TRY(run_round(g, LabelF{fa.parents, fa.src}, in, out, mode, output, cnt)); break;
-    case BYO_F_PR: BYO_TRY(run_round(g, PrF{fa.p_curr, fa.p_next, g->d_deg}, in, out, mode, output, cnt)); break;
-    case BYO_F_PR_DELTA: BYO_TRY(run_round(g, PrDeltaF{fa.delta, fa.ngh}, in, out, mode, output, cnt)); break;
+    case BYO_F_BFS_LABEL: BYO_TRY(run_round(g, LabelF{fa.parents, fa.src}, in, out, mode, output, cnt, plan)); break;
+    case BYO_F_PR: BYO_TRY(run_round(g, PrF{fa.p_curr, fa.p_next, g->d_deg}, in, out, mode, output, cnt, plan)); break;
+    case BYO_F_PR_DELTA: BYO_TRY(run_round(g, PrDeltaF{fa.delta, fa.ngh}, in, out, mode, output, cnt, plan)); break;
     default: return set_error(ctx, BYO_EINVAL, "edge_map: unknown functor kind");
   }
   unsigned long long h[2] = {0, 0};
-  BYO_CU(ctx, cudaMemcpyAsync(h, cnt, 16, cudaMemcpyDeviceToHost, ctx->stream));
-  BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
-  out.size = output ? h[0] : 0;
-  out.outdeg = output ? h[1] : 0;
+  if (output) {  // no output: the host waits for nothing
+    BYO_CU(ctx, cudaMemcpyAsync(h, cnt, 16, cudaMemcpyDeviceToHost, ctx->stream));
+    BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
+  }
+  out.size = h[0];
+  out.outdeg = h[1];
   out.has_list = out.has_bits = true;
   out.dense = mode == MODE_PULL || mode == MODE_DENSE_FWD;
   return BYO_OK;
+}
+
+int generic_edge_map(byo_graph *g, const FunctorArgs &fa, Frontier &in, Frontier &out, int mode, bool output) {
+  return edge_map_planned(g, fa, in, out, mode, output, nullptr);
 }
 
 int vertex_op_run(byo_graph *g, const VertexOpArgs &op, Frontier &in, Frontier *out) {
@@ -503,13 +853,18 @@ int vertex_op_run(byo_graph *g, const VertexOpArgs &op, Frontier &in, Frontier *
   return BYO_OK;
 }
 
-int l1_diff(byo_graph *g, const double *a, const double *b, double *d_part, double *h_out) {
+// The L1 distance of a and b on ctx->side[2], into h_out (pinned) when `done`
+// has happened.
+static int l1_diff(byo_graph *g, const double *a, const double *b, double *d_part, double *h_out, cudaEvent_t done) {
   byo_ctx *ctx = g->ctx;
   const uint64_t nch = (g->n + kL1Chunk - 1) / kL1Chunk;
-  launch(ctx, k_l1_chunks, dim3(grid_for(ctx, nch, 128)), dim3(128), 0, a, b, g->n, d_part);
-  launch(ctx, k_l1_total, dim3(1), dim3(32), 0, (const double *)d_part, nch, d_part + nch);
-  BYO_CU(ctx, cudaMemcpyAsync(h_out, d_part + nch, 8, cudaMemcpyDeviceToHost, ctx->stream));
-  BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
+  BYO_TRY(side_fork(ctx, 2));
+  cudaStream_t st = ctx->side[2];
+  k_l1_chunks<<<grid_for(ctx, nch * kL1Block, kL1Block, 4), kL1Block, 0, st>>>(a, b, g->n, d_part);
+  k_l1_total<<<1, kL1Block, 0, st>>>(d_part, nch, d_part + nch);
+  ctx->launches += 2;
+  BYO_CU(ctx, cudaMemcpyAsync(h_out, d_part + nch, 8, cudaMemcpyDeviceToHost, st));
+  BYO_CU(ctx, cudaEventRecord(done, st));
   return check_launch(ctx, "l1");
 }
 
@@ -519,16 +874,23 @@ int l1_diff(byo_graph *g, const double *a, const double *b, double *d_part, doub
 // L1 between the iterates, stop below eps; reset p_curr and swap.  Returns
 // the last computed iterate (the reference's final swap would hand back the
 // zeroed one when max_iters ends the loop).
+//
+// The L1 distance of an iteration is computed beside the next one, which writes
+// the third of three buffers: when the distance ends the loop, that iteration
+// is left unread.  So the host's wait and the L1 kernels (60 us, few CTAs) leave
+// the chain of iterations.
 int pagerank_edgemap_run(byo_graph *g, double eps, uint32_t max_iters, double *d_p, uint32_t *iters_out,
                          double *l1_out) {
   byo_ctx *ctx = g->ctx;
   const uint64_t n = g->n;
   const uint64_t W = (n + 31) / 32;
   const uint64_t nch = (n + kL1Chunk - 1) / kL1Chunk;
-  double *pa = nullptr, *pb = nullptr, *part = nullptr;
-  BYO_TRY(ws(g, WS_PR_A, n + 1, &pa));
-  BYO_TRY(ws(g, WS_PR_B, n + 1, &pb));
+  double *p[3] = {}, *part = nullptr, *h = nullptr;
+  BYO_TRY(ws(g, WS_PR_A, n + 1, &p[0]));
+  BYO_TRY(ws(g, WS_PR_B, n + 1, &p[1]));
+  BYO_TRY(ws(g, WS_LP, n + 1, &p[2]));
   BYO_TRY(ws(g, WS_PR_C, nch + 2, &part));
+  BYO_TRY(pinned(ctx, 4096, (void **)&h));
   uint32_t *flist = nullptr, *fbits = nullptr;
   BYO_TRY(ws(g, WS_FRONT_LIST_A, n + 1, &flist));
   BYO_TRY(ws(g, WS_FRONT_BITS_A, W + 1, &fbits));
@@ -537,30 +899,40 @@ int pagerank_edgemap_run(byo_graph *g, double eps, uint32_t max_iters, double *d
   all.bits = fbits;
   BYO_TRY(frontier_from_bits(g, nullptr, all));
   Frontier none;  // no_output rounds write nothing
-  launch(ctx, k_fill_f64, dim3(grid_for(ctx, n, 256)), dim3(256), 0, pa, n, 1.0 / (double)n);
-  BYO_CU(ctx, cudaMemsetAsync(pb, 0, n * 8, ctx->stream));
-  double *pc = pa, *pn = pb;
-  uint32_t it = 0;
+  SumPlan plan;   // of the view, which stays as it is
+  BYO_TRY(sum_plan(g, &plan));
+  launch(ctx, k_fill_f64, dim3(grid_for(ctx, n, 256)), dim3(256), 0, p[0], n, 1.0 / (double)n);
+  uint32_t it = 0;  // iterations whose distance is known
   double L1 = 0.0;
-  while (it++ < max_iters) {
-    FunctorArgs f{};
-    f.kind = BYO_F_PR;
-    f.p_curr = pc;
-    f.p_next = pn;
-    BYO_TRY(generic_edge_map(g, f, all, none, MODE_PULL, false));
-    VertexOpArgs vf{BYO_VOP_PR_UPDATE, pn, nullptr, nullptr, 0.85, 0.0};
-    BYO_TRY(vertex_op_run(g, vf, all, nullptr));
-    BYO_TRY(l1_diff(g, pc, pn, part, &L1));
-    if (L1 < eps) break;
-    VertexOpArgs rz{BYO_VOP_ZERO, pc, nullptr, nullptr, 0.0, 0.0};
-    BYO_TRY(vertex_op_run(g, rz, all, nullptr));
-    std::swap(pc, pn);
-  }
-  if (it > max_iters) {
-    it = max_iters;
-    std::swap(pc, pn);  // the last computed iterate, not the zeroed one
-  }
-  BYO_CU(ctx, cudaMemcpyAsync(d_p, pn, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
+  auto wait = [&](uint32_t t) -> int {  // for iteration t's distance
+    BYO_CU(ctx, cudaEventSynchronize(ctx->ev[2 + (t & 1)]));
+    L1 = h[t & 1];
+    it = t + 1;
+    return BYO_OK;
+  };
+  auto loop = [&]() -> int {
+    for (uint32_t t = 0; t < max_iters; t++) {
+      double *pc = p[t % 3], *pn = p[(t + 1) % 3];
+      BYO_TRY(memset_async(ctx, pn, 0, n * 8));
+      FunctorArgs f{};
+      f.kind = BYO_F_PR;
+      f.p_curr = pc;
+      f.p_next = pn;
+      BYO_TRY(edge_map_planned(g, f, all, none, MODE_PULL, false, &plan));
+      VertexOpArgs vf{BYO_VOP_PR_UPDATE, pn, nullptr, nullptr, 0.85, 0.0};
+      BYO_TRY(vertex_op_run(g, vf, all, nullptr));
+      BYO_TRY(l1_diff(g, pc, pn, part, h + (t & 1), ctx->ev[2 + (t & 1)]));
+      if (t) {
+        BYO_TRY(wait(t - 1));
+        if (L1 < eps) return BYO_OK;
+      }
+    }
+    return max_iters ? wait(max_iters - 1) : BYO_OK;
+  };
+  const int rc = loop();
+  if (max_iters) BYO_TRY(side_join(ctx, 2));
+  BYO_TRY(rc);
+  BYO_CU(ctx, cudaMemcpyAsync(d_p, p[it % 3], n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
   if (iters_out) *iters_out = it;
   if (l1_out) *l1_out = L1;
   return check_launch(ctx, "pagerank_edgemap");

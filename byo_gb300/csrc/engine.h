@@ -44,6 +44,7 @@ struct Frontier {
   uint64_t outdeg = 0;
   bool dense = false;        // produced by a dense round
   bool has_list = false, has_bits = false;
+  bool all = false;          // made as every vertex: membership needs no test
   unsigned long long hist[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   int next_mode = 0;    // policy kernel's choice for the round consuming this frontier
   float feat[16] = {0}; // its features

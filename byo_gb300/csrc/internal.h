@@ -40,6 +40,10 @@ struct byo_ctx {
   int device = 0;
   int num_sms = 0;
   cudaStream_t stream = nullptr;
+  // streams beside it, made on first use: work forked from it and joined again
+  // within one call (side_fork, side_join)
+  cudaStream_t side[3] = {};
+  cudaEvent_t side_ev[3] = {};
   std::string err;
   uint64_t launches = 0;
   void *pinned = nullptr;  // small pinned host staging area
@@ -138,6 +142,11 @@ int set_error(byo_ctx *ctx, int code, const char *what, cudaError_t e = cudaSucc
     if (rc_ != BYO_OK) return rc_; \
   } while (0)
 int check_launch(byo_ctx *ctx, const char *what);
+
+// ctx->side[i] continues from ctx->stream's work so far; ctx->stream waits for
+// ctx->side[i]'s.  Every fork is joined before the call that made it returns.
+int side_fork(byo_ctx *ctx, int i);
+int side_join(byo_ctx *ctx, int i);
 
 // Launch on the context's stream and count it.
 template <typename Kern, typename... Args>

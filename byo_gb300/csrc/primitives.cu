@@ -53,6 +53,20 @@ int check_launch(byo_ctx *ctx, const char *what) {
   return BYO_OK;
 }
 
+int side_fork(byo_ctx *ctx, int i) {
+  if (!ctx->side[i]) BYO_CU(ctx, cudaStreamCreateWithFlags(&ctx->side[i], cudaStreamNonBlocking));
+  if (!ctx->side_ev[i]) BYO_CU(ctx, cudaEventCreateWithFlags(&ctx->side_ev[i], cudaEventDisableTiming));
+  BYO_CU(ctx, cudaEventRecord(ctx->side_ev[i], ctx->stream));
+  BYO_CU(ctx, cudaStreamWaitEvent(ctx->side[i], ctx->side_ev[i], 0));
+  return BYO_OK;
+}
+
+int side_join(byo_ctx *ctx, int i) {
+  BYO_CU(ctx, cudaEventRecord(ctx->side_ev[i], ctx->side[i]));
+  BYO_CU(ctx, cudaStreamWaitEvent(ctx->stream, ctx->side_ev[i], 0));
+  return BYO_OK;
+}
+
 void free_buf(DevBuf &b) {
   if (b.p) cudaFree(b.p);
   b.p = nullptr;
