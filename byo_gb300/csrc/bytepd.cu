@@ -407,10 +407,10 @@ int graph_from_bytepd_host(byo_ctx *ctx, uint64_t n, const uint64_t *h_bo, const
   if (!h_bo || (n && !h_deg) || (nbytes && !h_bytes)) return set_error(ctx, BYO_EINVAL, "null byte-PD array");
   if (h_bo[0] != 0 || h_bo[n] > nbytes) return set_error(ctx, BYO_EINVAL, "byte-PD offsets outside the bytes");
   uint64_t m = 0;
-  for (uint64_t v = 0; v < n; v++) {
-    if (h_bo[v + 1] < h_bo[v]) return set_error(ctx, BYO_EINVAL, "byte-PD offsets decrease");
-    m += h_deg[v];
-  }
+  bool drops = false;
+  for (uint64_t v = 0; v < n; v++) drops |= h_bo[v + 1] < h_bo[v];
+  for (uint64_t v = 0; v < n; v++) m += h_deg[v];
+  if (drops) return set_error(ctx, BYO_EINVAL, "byte-PD offsets decrease");
   uint64_t *d_bo = nullptr, *d_off = nullptr;
   uint32_t *d_deg = nullptr, *d_nbrs = nullptr;
   unsigned char *d_bytes = nullptr;
@@ -419,7 +419,7 @@ int graph_from_bytepd_host(byo_ctx *ctx, uint64_t n, const uint64_t *h_bo, const
   if (e == cudaSuccess) e = cudaMalloc(&d_deg, (n ? n : 1) * 4);
   if (e == cudaSuccess) e = cudaMalloc(&d_bytes, nbytes ? nbytes : 1);
   if (e == cudaSuccess) e = cudaMalloc(&d_off, (n + 1) * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&d_nbrs, (m ? m : 1) * 4);
+  if (e == cudaSuccess) e = cudaMalloc(&d_nbrs, (m + 16) * 4);
   if (e != cudaSuccess) rc = set_error(ctx, BYO_ENOMEM, "cudaMalloc", e);
   if (rc == BYO_OK) {
     cudaMemcpyAsync(d_bo, h_bo, (n + 1) * 8, cudaMemcpyHostToDevice, ctx->stream);
@@ -427,7 +427,7 @@ int graph_from_bytepd_host(byo_ctx *ctx, uint64_t n, const uint64_t *h_bo, const
     if (nbytes) cudaMemcpyAsync(d_bytes, h_bytes, nbytes, cudaMemcpyHostToDevice, ctx->stream);
     rc = bytepd_decode(ctx, n, d_bo, d_deg, d_bytes, P, d_off, d_nbrs);
   }
-  if (rc == BYO_OK) rc = graph_from_device_csr(ctx, container, n, m, d_off, d_nbrs, out);
+  if (rc == BYO_OK) rc = graph_from_device_csr(ctx, container, n, m, &d_off, &d_nbrs, &d_deg, out);
   for (void *p : {(void *)d_bo, (void *)d_deg, (void *)d_bytes, (void *)d_off, (void *)d_nbrs})
     if (p) cudaFree(p);
   return rc;
