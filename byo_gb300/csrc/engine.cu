@@ -76,6 +76,10 @@ __device__ __forceinline__ bool visit(uint32_t u, uint32_t v, uint64_t lvl, uint
 }
 
 // ---------------------------------------------------------------- push
+// Slots of a hub a CTA takes (hub, chunk).  One CTA for a whole hub held the
+// round of a 2^22-vertex RMAT graph's largest hubs up for 1.3 ms; 0.19 in chunks.
+constexpr uint32_t kHubChunk = 2048;
+
 template <int GS>
 __global__ void __launch_bounds__(256) k_push(const uint64_t *__restrict__ off,
                                               const uint32_t *__restrict__ slots,
@@ -83,7 +87,7 @@ __global__ void __launch_bounds__(256) k_push(const uint64_t *__restrict__ off,
                                               const uint32_t *__restrict__ F, uint64_t fsize,
                                               uint64_t *lp, const uint32_t *__restrict__ visited,
                                               uint32_t *out_list, uint32_t *out_bits,
-                                              RoundStats *st, uint64_t lvl, uint32_t *hubs,
+                                              RoundStats *st, uint64_t lvl, uint2 *hubs, uint64_t hub_cap,
                                               uint32_t hub_min) {
   __shared__ unsigned long long s_hist[8];
   hist_init(s_hist);
@@ -100,10 +104,17 @@ __global__ void __launch_bounds__(256) k_push(const uint64_t *__restrict__ off,
       u = F[i];
       b = off[u];
       e = off[u + 1];
-      if (e - b >= hub_min) {
-        if (gl == 0) hubs[atomicAdd(&st->ndefer, 1ull)] = u;
-        e = b;
-      }
+    }
+    // a hub's lanes list its chunks; where the list is full (a frontier that
+    // holds ids twice) the places left say so and the group walks the hub itself
+    const uint32_t nc = e - b >= hub_min ? (uint32_t)((e - b + kHubChunk - 1) / kHubChunk) : 0;
+    unsigned long long at = 0;
+    if (nc && gl == 0) at = atomicAdd(&st->ndefer, (unsigned long long)nc);
+    at = __shfl_sync(kFull, at, g * GS);
+    if (nc) {
+      const bool fits = at + nc <= hub_cap;
+      for (uint32_t c = gl; c < nc && at + c < hub_cap; c += GS) hubs[at + c] = make_uint2(fits ? u : kSentinel, c);
+      if (fits) e = b;
     }
     uint64_t chunks = (e - b + GS - 1) / GS;
 #pragma unroll
@@ -165,21 +176,23 @@ __global__ void __launch_bounds__(256) k_push_dense_fwd(const uint64_t *__restri
   flush_dsum(dsum, st);
 }
 
-// One CTA per hub vertex (degree >= hub_min).
+// A CTA per chunk of a hub (degree >= hub_min).
 __global__ void __launch_bounds__(256) k_push_hubs(const uint64_t *__restrict__ off,
                                                    const uint32_t *__restrict__ slots,
                                                    const uint32_t *__restrict__ deg,
-                                                   const uint32_t *__restrict__ hubs,
+                                                   const uint2 *__restrict__ hubs, uint64_t hub_cap,
                                                    uint64_t *lp, const uint32_t *__restrict__ visited,
                                                    uint32_t *out_list, uint32_t *out_bits,
                                                    RoundStats *st, uint64_t lvl) {
   __shared__ unsigned long long s_hist[8];
   hist_init(s_hist);
-  const uint64_t nh = *(volatile unsigned long long *)&st->ndefer;
+  const uint64_t nd = *(volatile unsigned long long *)&st->ndefer, nh = nd < hub_cap ? nd : hub_cap;
   uint64_t dsum = 0;
   for (uint64_t h = blockIdx.x; h < nh; h += gridDim.x) {
-    const uint32_t u = hubs[h];
-    const uint64_t b = off[u], e = off[u + 1];
+    const uint32_t u = hubs[h].x;
+    if (u == kSentinel) continue;
+    const uint64_t b = off[u] + (uint64_t)hubs[h].y * kHubChunk, end = off[u + 1];
+    const uint64_t e = b + kHubChunk < end ? b + kHubChunk : end;
     for (uint64_t base = b; base < e; base += blockDim.x) {
       uint64_t j = base + threadIdx.x;
       bool em = false;
@@ -417,6 +430,22 @@ __global__ void k_trav_init(uint64_t *lp, uint32_t *visited, uint64_t n, uint32_
   }
 }
 
+// Everything a BFS from src starts from: lp, visited, both frontier bitmaps and
+// the first frontier.
+__global__ void k_bfs_start(uint64_t *lp, uint32_t *visited, uint32_t *list, uint32_t *bits, uint32_t *next_bits,
+                            uint64_t n, uint32_t src) {
+  const uint64_t W = (n + 31) >> 5;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+       i += (uint64_t)gridDim.x * blockDim.x) {
+    lp[i] = (i == src) ? (uint64_t)src : kNone64;
+    if (i < W) {
+      visited[i] = bits[i] = (i == (src >> 5)) ? (1u << (src & 31)) : 0u;
+      next_bits[i] = 0;
+    }
+    if (i == 0) list[0] = src;
+  }
+}
+
 __global__ void k_trav_extract(const uint64_t *__restrict__ lp, uint64_t n, uint32_t *parent,
                                uint32_t *level) {
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
@@ -550,8 +579,11 @@ int edge_map_round(byo_graph *g, TravState &st, Frontier &in, Frontier &out, int
   // the policy for the next round runs as the epilogue of this round's last kernel
   PolicyTail pt;
   if (run_policy) BYO_TRY(policy_tail_args(g, (unsigned int *)(d_st + 1), st.reached, mode == MODE_PULL, &pt));
+  // pull: deferred vertices; push: hub chunks (a frontier without repeats holds
+  // at most so many)
   uint32_t *defer = nullptr;
-  BYO_TRY(ws(g, WS_DEFER, g->n + 1, &defer));
+  const uint64_t hub_cap = g->nslots / kHubChunk + g->nslots / tune.hub_min + 1;
+  BYO_TRY(ws(g, WS_DEFER, std::max<uint64_t>(g->n + 1, 2 * hub_cap), &defer));
   const uint64_t lvl = (uint64_t)st.round << 32;
   if (mode == MODE_PULL) {
     BYO_TRY(ensure_bits(g, in));
@@ -590,8 +622,8 @@ int edge_map_round(byo_graph *g, TravState &st, Frontier &in, Frontier &out, int
   case GS:                                                                                       \
     launch_t(ctx, "bfs_push", k_push<GS>, dim3(grid), dim3(256), 0, (const uint64_t *)g->d_off,                \
            (const uint32_t *)g->d_slots, (const uint32_t *)g->d_deg, (const uint32_t *)in.list,  \
-           in.size, st.lp, (const uint32_t *)st.visited, out.list, out.bits, d_st, lvl, defer,   \
-           tune.hub_min);                                                                        \
+           in.size, st.lp, (const uint32_t *)st.visited, out.list, out.bits, d_st, lvl,          \
+           (uint2 *)defer, hub_cap, tune.hub_min);                                                                     \
     break;
         PUSH_CASE(4)
         PUSH_CASE(8)
@@ -602,7 +634,7 @@ int edge_map_round(byo_graph *g, TravState &st, Frontier &in, Frontier &out, int
           return set_error(ctx, BYO_EINVAL, "push group must be 4, 8, 16 or 32");
       }
       launch(ctx, k_push_hubs, dim3(ctx->num_sms * 2), dim3(256), 0, (const uint64_t *)g->d_off,
-             (const uint32_t *)g->d_slots, (const uint32_t *)g->d_deg, (const uint32_t *)defer, st.lp,
+             (const uint32_t *)g->d_slots, (const uint32_t *)g->d_deg, (const uint2 *)defer, hub_cap, st.lp,
              (const uint32_t *)st.visited, out.list, out.bits, d_st, lvl);
     } else {
       uint64_t *pre = nullptr;
@@ -656,18 +688,12 @@ int bfs_run(byo_graph *g, uint32_t src, uint32_t *d_parent, uint32_t *d_level, i
   BYO_TRY(ws(g, WS_FRONT_LIST_B, n, &fb.list));
   BYO_TRY(ws(g, WS_FRONT_BITS_A, W, &fa.bits));
   BYO_TRY(ws(g, WS_FRONT_BITS_B, W, &fb.bits));
-  BYO_TRY(trav_init(g, st, src));
-  BYO_CU(ctx, cudaMemcpyAsync(fa.list, &src, sizeof(uint32_t), cudaMemcpyHostToDevice, ctx->stream));
-  BYO_TRY(memset_async(ctx, fa.bits, 0, W * 4));
-  BYO_TRY(memset_async(ctx, fb.bits, 0, W * 4));
-  uint32_t word = 1u << (src & 31);
-  BYO_CU(ctx, cudaMemcpyAsync(fa.bits + (src >> 5), &word, 4, cudaMemcpyHostToDevice, ctx->stream));
-  uint32_t dsrc = 0;
-  BYO_CU(ctx, cudaMemcpyAsync(&dsrc, g->d_deg + src, 4, cudaMemcpyDeviceToHost, ctx->stream));
-  BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
+  launch(ctx, k_bfs_start, dim3(grid_for(ctx, n, 256)), dim3(256), 0, st.lp, st.visited, fa.list, fa.bits, fb.bits, n,
+         src);
+  BYO_TRY(check_launch(ctx, "bfs_start"));
+  st.round = 1;
+  st.reached = 1;
   fa.size = 1;
-  fa.outdeg = dsrc;
-  fa.hist[log4_bin(dsrc)] = 1;
   fa.has_list = fa.has_bits = true;
   fb.size = 0;
   fb.has_list = true;  // empty list: its bitmap is all zero
@@ -676,32 +702,44 @@ int bfs_run(byo_graph *g, uint32_t src, uint32_t *d_parent, uint32_t *d_level, i
   // features (and the learned choice) are computed on the device after every
   // round when the learned policy runs or rounds are being logged
   const bool run_policy = policy == BYO_POLICY_LEARNED || ctx->time_rounds;
-  if (run_policy) {
-    RoundStats *d_st = nullptr, *h = nullptr;
-    BYO_TRY(ws(g, WS_STATS, sizeof(RoundStats) / sizeof(uint64_t) + 2, (uint64_t **)&d_st));
-    BYO_TRY(pinned(ctx, 4096, (void **)&h));
-    std::memset(h, 0, sizeof(RoundStats));
-    h->count = 1;
-    h->outdeg = dsrc;
-    int bin = dsrc ? (31 - __builtin_clz(dsrc)) / 2 : 0;
-    h->hist[bin > 7 ? 7 : bin] = 1;
-    BYO_CU(ctx, cudaMemcpyAsync(d_st, h, sizeof(RoundStats), cudaMemcpyHostToDevice, ctx->stream));
-    BYO_TRY(round_policy(g, d_st, 0, false));
-    BYO_CU(ctx, cudaMemcpyAsync(h, d_st, sizeof(RoundStats), cudaMemcpyDeviceToHost, ctx->stream));
-    BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
-    fa.next_mode = (int)h->mode;
-    for (int i = 0; i < 16; i++) fa.feat[i] = h->feat[i];
-  }
   Frontier *cur = &fa, *nxt = &fb;
   uint32_t nr = 0;
   // small push rounds run back to back in one persistent kernel (not while
   // rounds are timed one by one for the policy's training samples)
   const bool small_ok = !ctx->time_rounds &&
                         (policy == BYO_POLICY_M20 || policy == BYO_POLICY_LEARNED || policy == BYO_POLICY_PUSH);
-  const uint64_t small_limit = std::max<uint64_t>(4096, g->m / 20 / 64);
-  // a frontier holding a vertex of degree >= 4^5 goes to the round kernels,
-  // which give such vertices whole CTAs (and which the learned policy inspects)
-  const bool gate_hub = true;
+  // The learned policy inspects frontiers near the m/20 threshold and those
+  // holding a vertex of degree >= 4^5; a rule does not, and up to kSmallEdges
+  // edges a round costs less there (under 10 us) than any round driven from the
+  // host (~30 us).
+  const bool gate_hub = policy == BYO_POLICY_LEARNED;
+  const uint64_t small_limit = gate_hub ? std::max<uint64_t>(4096, g->m / 20 / 64) : kSmallEdges;
+  if (small_ok && !gate_hub) {
+    // start there without asking the host for the source's degree
+    BYO_TRY(bfs_small_rounds(g, st, cur, nxt, small_limit, false, nullptr, &nr));
+  } else {
+    uint32_t dsrc = 0;
+    BYO_CU(ctx, cudaMemcpyAsync(&dsrc, g->d_deg + src, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
+    fa.outdeg = dsrc;
+    fa.hist[log4_bin(dsrc)] = 1;
+    if (run_policy) {
+      RoundStats *d_st = nullptr, *h = nullptr;
+      BYO_TRY(ws(g, WS_STATS, sizeof(RoundStats) / sizeof(uint64_t) + 2, (uint64_t **)&d_st));
+      BYO_TRY(pinned(ctx, 4096, (void **)&h));
+      std::memset(h, 0, sizeof(RoundStats));
+      h->count = 1;
+      h->outdeg = dsrc;
+      int bin = dsrc ? (31 - __builtin_clz(dsrc)) / 2 : 0;
+      h->hist[bin > 7 ? 7 : bin] = 1;
+      BYO_CU(ctx, cudaMemcpyAsync(d_st, h, sizeof(RoundStats), cudaMemcpyHostToDevice, ctx->stream));
+      BYO_TRY(round_policy(g, d_st, 0, false));
+      BYO_CU(ctx, cudaMemcpyAsync(h, d_st, sizeof(RoundStats), cudaMemcpyDeviceToHost, ctx->stream));
+      BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
+      fa.next_mode = (int)h->mode;
+      for (int i = 0; i < 16; i++) fa.feat[i] = h->feat[i];
+    }
+  }
   while (cur->size > 0) {
     int mode;
     switch (policy) {
@@ -717,13 +755,14 @@ int bfs_run(byo_graph *g, uint32_t src, uint32_t *d_parent, uint32_t *d_level, i
     BYO_TRY(clear_frontier_bits(g, *nxt));
     bool hub = false;
     for (int q = 5; q < 8; q++) hub |= cur->hist[q] != 0;
-    if (small_ok && mode == MODE_PUSH && cur->has_list && cur->size + cur->outdeg <= small_limit &&
-        !(gate_hub && hub)) {
+    if (small_ok && mode != MODE_BLOCKED && (mode == MODE_PUSH || !gate_hub) && cur->has_list &&
+        cur->outdeg && cur->size + cur->outdeg <= std::min(small_limit, kSmallEdges) && !(gate_hub && hub)) {
       RoundStats *d_st = nullptr;
       BYO_TRY(ws(g, WS_STATS, sizeof(RoundStats) / sizeof(uint64_t) + 2, (uint64_t **)&d_st));
       uint32_t R = 0;
       BYO_TRY(bfs_small_rounds(g, st, cur, nxt, small_limit, gate_hub, run_policy ? d_st : nullptr, &R));
       nr += R;
+      if (R == 0) return set_error(ctx, BYO_EDEVICE, "bfs: small rounds did not run");
       if (run_policy && cur->size > 0) {
         // the policy for the frontier the kernel stopped at
         RoundStats *h = nullptr;

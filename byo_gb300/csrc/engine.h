@@ -9,7 +9,8 @@
 //
 //   push     (edgeMapSparse, edge_map_blocked.h:18-92): groups of lanes per
 //            frontier vertex, coalesced neighbour loads, atomicMin on lp so the
-//            smallest-id parent of this level wins; hubs go to one CTA each.
+//            smallest-id parent of this level wins; hubs are cut into chunks, a
+//            CTA each.
 //   blocked  (edgeMapBlocked, edge_map_blocked.h:130-246): edge-balanced tiles
 //            over the exclusive scan of frontier degrees (merge-path split).
 //   pull     (edgeMapDense, edge_map_data.h:47-175): one thread per unvisited
@@ -30,7 +31,7 @@ enum Mode { MODE_PUSH = 0, MODE_PULL = 1, MODE_BLOCKED = 2, MODE_DENSE_FWD = 3 }
 struct RoundStats {
   unsigned long long count;   // |next frontier|
   unsigned long long outdeg;  // sum of degrees of the next frontier
-  unsigned long long ndefer;  // pull: deferred long scans; push: hubs
+  unsigned long long ndefer;  // pull: deferred long scans; push: hub chunks
   unsigned long long edges;   // edges examined (diagnostic)
   unsigned long long hist[8]; // degree sketch of the next frontier (log4 bins)
   unsigned long long mode;    // next round's mode chosen by the policy kernel
@@ -78,11 +79,13 @@ int ensure_bits(byo_graph *g, Frontier &f);
 int trav_init(byo_graph *g, TravState &st, uint32_t src);
 int trav_extract(byo_graph *g, const TravState &st, uint32_t *d_parent, uint32_t *d_level);
 EngineTuning default_tuning(const byo_graph *g);
-// Runs push rounds from *cur in one persistent kernel while the frontier
-// stays within `limit` edges (and, with gate_hub, holds no vertex of degree
-// >= 4^5); on return *cur is the frontier reached and *nxt a clean buffer
-// (bfs_small.cu).  With d_st, the final frontier's statistics are written
-// there for the policy.
+// Runs push rounds from *cur in one kernel while the frontier stays within
+// `limit` (at most kSmallEdges) edges and, with gate_hub, holds no vertex of
+// degree >= 4^5; on return *cur is the frontier reached (with its size,
+// out-degree and sketch; the one it came with when no round could run) and *nxt,
+// whose bitmap is zero, stays empty (bfs_small.cu).  With d_st, the final frontier's statistics are
+// written there for the policy.
+constexpr uint64_t kSmallEdges = 1u << 16;
 int bfs_small_rounds(byo_graph *g, TravState &st, Frontier *&cur, Frontier *&nxt, uint64_t limit, bool gate_hub,
                      RoundStats *d_st, uint32_t *rounds_run);
 
