@@ -48,12 +48,11 @@ __device__ __forceinline__ void hist_flush(unsigned long long *sh, RoundStats *s
 __device__ __forceinline__ void emit_next(bool emit, uint32_t v, uint32_t *out_list,
                                           uint32_t *out_bits, RoundStats *st,
                                           const uint32_t *__restrict__ deg, uint64_t &dsum,
-                                          bool set_bits, unsigned long long *sh) {
-  uint64_t slot = warp_append(emit, &st->count);
+                                          WarpList &wl, unsigned long long *sh) {
+  wl.add(emit, v, out_list, &st->count);
   uint32_t d = 0;
   if (emit) {
-    out_list[slot] = v;
-    if (set_bits) atomicOr(out_bits + (v >> 5), 1u << (v & 31));
+    atomicOr(out_bits + (v >> 5), 1u << (v & 31));
     d = deg[v];
     dsum += d;
   }
@@ -75,9 +74,26 @@ __device__ __forceinline__ bool visit(uint32_t u, uint32_t v, uint64_t lvl, uint
   return old == kNone64;
 }
 
+// R edges u[q] -> v[q] a lane (v kSentinel: none): their bits, then their atomics, then
+// the emissions, so R edges wait for each access once.  Warp-collective.
+template <int R>
+__device__ __forceinline__ void visit_emit(const uint32_t (&u)[R], const uint32_t (&v)[R], uint64_t lvl, uint64_t *lp,
+                                           const uint32_t *__restrict__ visited, uint32_t *out_list,
+                                           uint32_t *out_bits, RoundStats *st, const uint32_t *__restrict__ deg,
+                                           uint64_t &dsum, WarpList &wl, unsigned long long *sh) {
+  bool open[R];
+#pragma unroll
+  for (int q = 0; q < R; q++) open[q] = v[q] != kSentinel && !test_bit_cg(visited, v[q]);
+#pragma unroll
+  for (int q = 0; q < R; q++)
+    if (open[q]) open[q] = atomicMin((unsigned long long *)(lp + v[q]), (unsigned long long)(lvl | u[q])) == kNone64;
+#pragma unroll
+  for (int q = 0; q < R; q++) emit_next(open[q], v[q], out_list, out_bits, st, deg, dsum, wl, sh);
+}
+
 // ---------------------------------------------------------------- push
 // Slots of a hub a CTA takes (hub, chunk).  One CTA for a whole hub held the
-// round of a 2^22-vertex RMAT graph's largest hubs up for 1.3 ms; 0.19 in chunks.
+// round of a 2^22-vertex RMAT graph's largest hubs up for 1.3 ms; 0.11 in chunks.
 constexpr uint32_t kHubChunk = 2048;
 
 template <int GS>
@@ -91,6 +107,8 @@ __global__ void __launch_bounds__(256) k_push(const uint64_t *__restrict__ off,
                                               uint32_t hub_min) {
   __shared__ unsigned long long s_hist[8];
   hist_init(s_hist);
+  __shared__ uint32_t s_list[8][kWarpListCap];
+  WarpList wl{s_list[threadIdx.x >> 5]};
   constexpr int PER_WARP = 32 / GS;
   const unsigned lane = lane_id(), g = lane / GS, gl = lane % GS;
   const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -123,16 +141,12 @@ __global__ void __launch_bounds__(256) k_push(const uint64_t *__restrict__ off,
       chunks = t > chunks ? t : chunks;
     }
     for (uint64_t c = 0; c < chunks; c++) {
-      uint64_t j = b + c * GS + gl;
-      bool em = false;
-      uint32_t v = kSentinel;
-      if (j < e) {
-        v = slots[j];
-        em = visit(u, v, lvl, lp, visited);
-      }
-      emit_next(em, v, out_list, out_bits, st, deg, dsum, true, s_hist);
+      const uint64_t j = b + c * GS + gl;
+      const uint32_t us[1] = {u}, v[1] = {j < e ? slots[j] : kSentinel};
+      visit_emit(us, v, lvl, lp, visited, out_list, out_bits, st, deg, dsum, wl, s_hist);
     }
   }
+  wl.flush(out_list, &st->count);
   hist_flush(s_hist, st);
   flush_dsum(dsum, st);
 }
@@ -149,6 +163,8 @@ __global__ void __launch_bounds__(256) k_push_dense_fwd(const uint64_t *__restri
                                                         uint64_t lvl) {
   __shared__ unsigned long long s_hist[8];
   hist_init(s_hist);
+  __shared__ uint32_t s_list[8][kWarpListCap];
+  WarpList wl{s_list[threadIdx.x >> 5]};
   const unsigned lane = lane_id();
   const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -168,10 +184,11 @@ __global__ void __launch_bounds__(256) k_push_dense_fwd(const uint64_t *__restri
           v = slots[j];
           em = visit(u, v, lvl, lp, visited);
         }
-        emit_next(em, v, out_list, out_bits, st, deg, dsum, true, s_hist);
+        emit_next(em, v, out_list, out_bits, st, deg, dsum, wl, s_hist);
       }
     }
   }
+  wl.flush(out_list, &st->count);
   hist_flush(s_hist, st);
   flush_dsum(dsum, st);
 }
@@ -186,6 +203,8 @@ __global__ void __launch_bounds__(256) k_push_hubs(const uint64_t *__restrict__ 
                                                    RoundStats *st, uint64_t lvl) {
   __shared__ unsigned long long s_hist[8];
   hist_init(s_hist);
+  __shared__ uint32_t s_list[8][kWarpListCap];
+  WarpList wl{s_list[threadIdx.x >> 5]};
   const uint64_t nd = *(volatile unsigned long long *)&st->ndefer, nh = nd < hub_cap ? nd : hub_cap;
   uint64_t dsum = 0;
   for (uint64_t h = blockIdx.x; h < nh; h += gridDim.x) {
@@ -193,25 +212,44 @@ __global__ void __launch_bounds__(256) k_push_hubs(const uint64_t *__restrict__ 
     if (u == kSentinel) continue;
     const uint64_t b = off[u] + (uint64_t)hubs[h].y * kHubChunk, end = off[u + 1];
     const uint64_t e = b + kHubChunk < end ? b + kHubChunk : end;
-    for (uint64_t base = b; base < e; base += blockDim.x) {
-      uint64_t j = base + threadIdx.x;
-      bool em = false;
-      uint32_t v = kSentinel;
-      if (j < e) {
-        v = slots[j];
-        em = visit(u, v, lvl, lp, visited);
+    for (uint64_t base = b; base < e; base += 4 * blockDim.x) {
+      uint32_t v[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const uint64_t j = base + q * blockDim.x + threadIdx.x;
+        v[q] = j < e ? slots[j] : kSentinel;
       }
-      emit_next(em, v, out_list, out_bits, st, deg, dsum, true, s_hist);
+      const uint32_t us[4] = {u, u, u, u};
+      visit_emit(us, v, lvl, lp, visited, out_list, out_bits, st, deg, dsum, wl, s_hist);
     }
   }
+  wl.flush(out_list, &st->count);
   hist_flush(s_hist, st);
   flush_dsum(dsum, st);
 }
 
 // ---------------------------------------------------------------- blocked
+// The last i in [0, n) with pre[i] <= x (pre[0] <= x), by a warp: 32 probes a
+// step, so 2^20 entries take four waits for memory.
+__device__ __forceinline__ uint64_t warp_last_le(const uint64_t *__restrict__ pre, uint64_t n, uint64_t x) {
+  uint64_t lo = 0, len = n;  // the answer is in [lo, lo + len)
+  while (len > 1) {
+    const uint64_t step = (len + 31) / 32, at = lo + lane_id() * step;
+    const unsigned m = __ballot_sync(kFull, lane_id() * step < len && pre[at] <= x);
+    const int k = 31 - __clz((int)m);
+    lo += (uint64_t)k * step;
+    len = len - (uint64_t)k * step < step ? len - (uint64_t)k * step : step;
+  }
+  return lo;
+}
+
 // Edge-balanced: tile t covers frontier-edge ranks [t*TILE, (t+1)*TILE) of
 // the exclusive degree prefix `pre`; each rank is mapped to its frontier
-// vertex by binary search (the merge-path split of rank space).
+// vertex by binary search (the merge-path split of rank space).  The tile's
+// part of the prefix and the vertices' slots are staged in shared memory, so an
+// edge's search waits for no global memory, and a thread has 4 edges in flight
+// (RMAT 2^20, a round over half the graph: 420 -> 375 us).
+constexpr uint32_t kBlockedStage = 2048;
 __global__ void __launch_bounds__(256) k_push_blocked(const uint64_t *__restrict__ off,
                                                       const uint32_t *__restrict__ slots,
                                                       const uint32_t *__restrict__ deg,
@@ -223,48 +261,68 @@ __global__ void __launch_bounds__(256) k_push_blocked(const uint64_t *__restrict
                                                       RoundStats *st, uint64_t lvl, int tile) {
   __shared__ unsigned long long s_hist[8];
   hist_init(s_hist);
+  __shared__ uint32_t s_list[8][kWarpListCap];
+  WarpList wl{s_list[threadIdx.x >> 5]};
+  __shared__ uint64_t s_slot[kBlockedStage];  // slot of a rank: rank + s_slot
+  __shared__ uint32_t s_pre[kBlockedStage], s_u[kBlockedStage];
+  __shared__ uint64_t s_lo, s_hi;
   const uint64_t total = pre[fsize];
   const uint64_t ntiles = (total + tile - 1) / tile;
-  __shared__ uint64_t s_lo, s_hi;
   uint64_t dsum = 0;
   for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const uint64_t e0 = t * tile;
     const uint64_t e1 = e0 + tile < total ? e0 + tile : total;
-    if (threadIdx.x == 0) {
-      // last index with pre[i] <= e0, and with pre[i] <= e1-1
-      uint64_t lo = 0, hi = fsize;  // search in [0, fsize)
-      while (hi - lo > 1) {
-        uint64_t mid = (lo + hi) >> 1;
-        if (pre[mid] <= e0) lo = mid; else hi = mid;
-      }
-      s_lo = lo;
-      uint64_t lo2 = lo, hi2 = fsize;
-      while (hi2 - lo2 > 1) {
-        uint64_t mid = (lo2 + hi2) >> 1;
-        if (pre[mid] <= e1 - 1) lo2 = mid; else hi2 = mid;
-      }
-      s_hi = lo2;
+    if (threadIdx.x < 64) {  // the first and the last vertex, a warp each
+      const uint64_t i = warp_last_le(pre, fsize, threadIdx.x < 32 ? e0 : e1 - 1);
+      if (threadIdx.x == 0) s_lo = i;
+      if (threadIdx.x == 32) s_hi = i;
     }
     __syncthreads();
     const uint64_t vlo = s_lo, vhi = s_hi;
-    for (uint64_t base = e0; base < e1; base += blockDim.x) {
-      const uint64_t e = base + threadIdx.x;
-      bool em = false;
-      uint32_t v = kSentinel;
-      if (e < e1) {
-        uint64_t lo = vlo, hi = vhi + 1;
-        while (hi - lo > 1) {
-          uint64_t mid = (lo + hi) >> 1;
-          if (pre[mid] <= e) lo = mid; else hi = mid;
-        }
-        const uint32_t u = F[lo];
-        v = slots[off[u] + (e - pre[lo])];
-        em = visit(u, v, lvl, lp, visited);
+    // (a frontier may hold any number of vertices without slots)
+    const bool staged = vhi - vlo < kBlockedStage;
+    const uint32_t nv = (uint32_t)(vhi - vlo + 1);
+    if (staged) {
+      for (uint32_t i = threadIdx.x; i < nv; i += blockDim.x) {
+        const uint32_t u = F[vlo + i];
+        const uint64_t p = pre[vlo + i];
+        s_u[i] = u;
+        s_pre[i] = p > e0 ? (uint32_t)(p - e0) : 0;
+        s_slot[i] = off[u] - p;
       }
-      emit_next(em, v, out_list, out_bits, st, deg, dsum, true, s_hist);
+      __syncthreads();
+    }
+    for (uint64_t base = e0; base < e1; base += 4 * blockDim.x) {
+      uint32_t u[4], v[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const uint64_t e = base + q * blockDim.x + threadIdx.x;
+        u[q] = 0;
+        v[q] = kSentinel;
+        if (e >= e1) continue;
+        if (staged) {
+          uint32_t lo = 0, hi = nv;
+          while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (s_pre[mid] <= (uint32_t)(e - e0)) lo = mid; else hi = mid;
+          }
+          u[q] = s_u[lo];
+          v[q] = slots[e + s_slot[lo]];
+        } else {
+          uint64_t lo = vlo, hi = vhi + 1;
+          while (hi - lo > 1) {
+            const uint64_t mid = (lo + hi) >> 1;
+            if (pre[mid] <= e) lo = mid; else hi = mid;
+          }
+          u[q] = F[lo];
+          v[q] = slots[off[u[q]] + (e - pre[lo])];
+        }
+      }
+      visit_emit(u, v, lvl, lp, visited, out_list, out_bits, st, deg, dsum, wl, s_hist);
     }
     __syncthreads();
   }
+  wl.flush(out_list, &st->count);
   hist_flush(s_hist, st);
   flush_dsum(dsum, st);
 }
@@ -277,6 +335,9 @@ __device__ __forceinline__ bool in_frontier(const uint32_t *s_bits, int stage_wo
   return (word >> (u & 31)) & 1u;
 }
 
+// A thread per unvisited vertex.  Found and deferred vertices go out through
+// WarpLists: an add to the two counters from every warp held the first dense
+// round at RMAT 2^22 up by a third (138 us, 96 now).
 __global__ void __launch_bounds__(1024, 2) k_pull(const uint64_t *__restrict__ off,
                                                const uint32_t *__restrict__ slots,
                                                const uint32_t *__restrict__ deg,
@@ -287,6 +348,8 @@ __global__ void __launch_bounds__(1024, 2) k_pull(const uint64_t *__restrict__ o
                                                int cap, int stage_words) {
   extern __shared__ uint32_t s_bits[];
   __shared__ unsigned long long s_hist[8];
+  __shared__ uint32_t s_list[2][32][kWarpListCap];
+  WarpList wl{s_list[0][threadIdx.x >> 5]}, wdefer{s_list[1][threadIdx.x >> 5]};
   for (int i = threadIdx.x; i < stage_words; i += blockDim.x) s_bits[i] = Fbits[i];
   if (threadIdx.x < 8) s_hist[threadIdx.x] = 0;
   __syncthreads();
@@ -329,17 +392,17 @@ __global__ void __launch_bounds__(1024, 2) k_pull(const uint64_t *__restrict__ o
       out_bits[w] = fb;
       visited[w] = vword | fb;
     }
-    uint64_t slot = warp_append(found, &st->count);
+    wl.add(found, (uint32_t)v, out_list, &st->count);
     uint32_t d = 0;
     if (found) {
-      out_list[slot] = (uint32_t)v;
       d = deg[v];
       dsum += d;
     }
     hist_warp_add(s_hist, found, d);
-    uint64_t ds = warp_append(deferred, &st->ndefer);
-    if (deferred) defer[ds] = (uint32_t)v;
+    wdefer.add(deferred, (uint32_t)v, defer, &st->ndefer);
   }
+  wl.flush(out_list, &st->count);
+  wdefer.flush(defer, &st->ndefer);
   hist_flush(s_hist, st);
   flush_dsum(dsum, st);
 }
@@ -561,8 +624,8 @@ int ensure_bits(byo_graph *g, Frontier &f) {
 }
 
 static int pull_smem_ok(int bytes) {
-  static int configured = 0;
-  if (bytes > 48 * 1024 && configured < bytes) {
+  static int configured = 0;  // (24 KB more are static)
+  if (configured < bytes) {
     if (cudaFuncSetAttribute(k_pull, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
       return 0;
     configured = bytes;

@@ -246,7 +246,7 @@ int byo_bfs_multi_device(byo_graph *g, const uint32_t *h_srcs, uint32_t k, uint3
  * vertex_ops::kBlockSize gbbs/vertex.h:35). */
 typedef struct byo_tuning {
   uint32_t push_group;   /* single-source push: lanes per frontier vertex (4, 8, 16 or 32) */
-  uint32_t hub_min;      /* single-source push: degree from which one CTA takes a vertex (>= 32) */
+  uint32_t hub_min;      /* single-source push: degree from which CTAs take a vertex, in chunks (>= 32) */
   uint32_t pull_cap;     /* single-source pull: slots a thread scans before a warp takes over (1..4096) */
   uint32_t blocked_tile; /* blocked push: slots per tile (64..65536) */
   uint32_t ms_heavy_deg; /* 64-source pull: slots above which a warp takes a vertex (1..65536) */
