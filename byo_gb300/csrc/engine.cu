@@ -528,8 +528,8 @@ byo_tuning effective_tuning(const byo_graph *g) {
   if (!t.hub_min) t.hub_min = 4096;
   if (!t.pull_cap) t.pull_cap = 32;
   if (!t.blocked_tile) t.blocked_tile = 2048;
-  if (!t.ms_heavy_deg) t.ms_heavy_deg = 32;
-  if (!t.ms_hub_deg) t.ms_hub_deg = 2048;
+  if (!t.ms_heavy_deg) t.ms_heavy_deg = 48;
+  if (!t.ms_hub_deg) t.ms_hub_deg = 1024;
   if (!t.ms_push_div) t.ms_push_div = 20;
   if (!t.tc_stage) t.tc_stage = 40960;
   t.reserved = 0;

@@ -42,7 +42,7 @@
 
 namespace byo {
 
-__global__ void __launch_bounds__(kMsBlock, 5) k_ms_bfs(MsArgs a) { ms_bfs_body(a, &a.ctl->bar); }
+__global__ void __launch_bounds__(kMsBlock, 2) k_ms_bfs(MsArgs a) { ms_bfs_body(a, &a.ctl->bar); }
 
 __global__ void __launch_bounds__(256) k_ms_levels(const MsArgs a) {
   if (a.ctl->bar.err) return;

@@ -11,7 +11,9 @@
 
 namespace byo {
 
-constexpr int kMsBlock = 256;
+// Two CTAs of 20 warps an SM: as many warps as five of 8 hold (48 registers), and
+// 304 arrivals at a grid barrier instead of 760.
+constexpr int kMsBlock = 640;
 constexpr int kLevelBits = 16;                   // bit planes of the levels (rounds < 2^16)
 constexpr int kMsLog = 64;                       // rounds recorded for byo_last_rounds
 
@@ -84,53 +86,110 @@ __device__ __forceinline__ void ms_levels(const MsArgs &a, uint32_t v, uint64_t 
   }
 }
 
-// Appends lanes' vertices to frontier list `slot` (non-hubs front, hubs back
-// with their chunks in C[par]).  Warp-uniform call.
-__device__ __forceinline__ void ms_list(const MsArgs &a, int slot, int par, bool has, uint32_t v, uint64_t d) {
+// Places for the lanes' items, Q a lane, in a list (has[q]: the lane has item q):
+// the value returned plus at[q], with one add to the counter for all of them.  An
+// add of every warp for 32 items would take the L2 ~1 ns each.
+template <int Q>
+__device__ __forceinline__ uint64_t ms_places(const bool (&has)[Q], unsigned long long *counter, uint32_t (&at)[Q]) {
+  uint32_t total = 0;
+#pragma unroll
+  for (int q = 0; q < Q; q++) {
+    const unsigned m = __ballot_sync(kFull, has[q]);
+    at[q] = total + __popc(m & lanemask_lt());
+    total += __popc(m);
+  }
+  if (!total) return 0;
+  unsigned long long base = 0;
+  if (lane_id() == 0) base = atomicAdd(counter, (unsigned long long)total);
+  return __shfl_sync(kFull, base, 0);
+}
+
+// Lists a hub v of d slots in the back of `list` (its place from `count`) and its
+// chunks in `chunks` (from `nchunks`).
+__device__ __forceinline__ void ms_hub(const MsArgs &a, uint32_t *list, unsigned long long *count, uint64_t *chunks,
+                                       unsigned long long *nchunks, uint32_t v, uint64_t d) {
+  list[a.n - 1 - atomicAdd(count, 1ull)] = v;
+  const uint64_t nch = (d + a.hub_deg - 1) / a.hub_deg;
+  const uint64_t cb = atomicAdd(nchunks, (unsigned long long)nch);
+  if (cb + nch <= a.ccap)
+    for (uint64_t t = 0; t < nch; t++) chunks[cb + t] = (uint64_t)v << 32 | t;
+  else
+    atomicOr(&a.ctl->bar.err, 2u);
+}
+
+// Appends lanes' vertices, Q a lane, to frontier list `slot` (non-hubs front,
+// hubs back with their chunks in C[par]).  Warp-uniform call.
+template <int Q>
+__device__ __forceinline__ void ms_list(const MsArgs &a, int slot, int par, const bool (&has)[Q],
+                                        const uint32_t (&v)[Q], const uint32_t (&d)[Q]) {
   MsCtl *c = a.ctl;
-  const bool hub = has && d > a.hub_deg;
-  const uint64_t s1 = warp_append(has && !hub, &c->lc[slot]);
-  if (has && !hub) a.L[slot][s1] = v;
-  if (__ballot_sync(kFull, hub)) {
-    const uint64_t s2 = warp_append(hub, &c->hc[slot]);
-    if (hub) {
-      a.L[slot][a.n - 1 - s2] = v;
-      const uint64_t nch = (d + a.hub_deg - 1) / a.hub_deg;
-      const uint64_t cb = atomicAdd(&c->cc[par], (unsigned long long)nch);
-      if (cb + nch <= a.ccap)
-        for (uint64_t t = 0; t < nch; t++) a.C[par][cb + t] = (uint64_t)v << 32 | t;
+  bool plain[Q];
+  uint32_t at[Q];
+#pragma unroll
+  for (int q = 0; q < Q; q++) plain[q] = has[q] && d[q] <= a.hub_deg;
+  uint32_t *const to = a.L[slot] + ms_places(plain, &c->lc[slot], at);
+#pragma unroll
+  for (int q = 0; q < Q; q++) {
+    if (plain[q]) to[at[q]] = v[q];
+    else if (has[q]) ms_hub(a, a.L[slot], &c->hc[slot], a.C[par], &c->cc[par], v[q], d[q]);
+  }
+}
+
+// One warp pushes F[u] over slots [b, e) of u, 128 at a time (each access is
+// waited for once for four edges a lane); with `track`, the first writer of
+// X[v] appends v to the touched list.  Warp-uniform call.
+__device__ __forceinline__ void ms_push_range(const MsArgs &a, uint64_t mu, uint64_t b, uint64_t e, int par,
+                                              bool track) {
+  const unsigned lane = threadIdx.x & 31;
+  for (uint64_t base = b; base < e; base += 128) {
+    uint32_t v[4], at[4];
+    uint64_t add[4];
+    bool first[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) v[q] = base + q * 32 + lane < e ? __ldg(a.slots + base + q * 32 + lane) : kSentinel;
+#pragma unroll
+    for (int q = 0; q < 4; q++) add[q] = v[q] != kSentinel ? mu & ~ldm(a.seen, v[q]) : 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      first[q] = false;
+      if (!add[q]) continue;
+      if (track)
+        first[q] = atomicOr((unsigned long long *)a.X + v[q], (unsigned long long)add[q]) == 0;
       else
-        atomicOr(&c->bar.err, 2u);
+        atomicOr((unsigned long long *)a.X + v[q], (unsigned long long)add[q]);
+    }
+    if (track) {
+      uint32_t *const to = a.T + ms_places(first, &a.ctl->tc[par], at);
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (first[q]) to[at[q]] = v[q];
     }
   }
 }
 
-// One warp pushes F[u] over slots [b, e) of u; with `track`, the first
-// writer of X[v] appends v to the touched list.  Warp-uniform call.
-__device__ __forceinline__ void ms_push_range(const MsArgs &a, uint64_t mu, uint64_t b, uint64_t e, int par,
-                                              bool track) {
+// The OR of F over slots [b, e), a warp's lanes together: 32 slots first (a
+// dense frontier ends most searches there), then 128 at a time, until all of
+// `need` is found or done(got) says so after a step (the same in every lane).
+template <class Done>
+__device__ __forceinline__ uint64_t ms_pull_range(const MsArgs &a, const uint64_t *F, uint64_t b, uint64_t e,
+                                                  uint64_t need, const Done &done) {
   const unsigned lane = threadIdx.x & 31;
-  for (uint64_t base = b; base < e; base += 32) {
-    const uint64_t j = base + lane;
-    uint32_t v = kSentinel;
-    bool first = false;
-    if (j < e) {
-      v = __ldg(a.slots + j);
-      if (v != kSentinel) {
-        const uint64_t add = mu & ~ldm(a.seen, v);
-        if (add) {
-          if (track)
-            first = atomicOr((unsigned long long *)a.X + v, (unsigned long long)add) == 0;
-          else
-            atomicOr((unsigned long long *)a.X + v, (unsigned long long)add);
-        }
-      }
-    }
-    if (track) {
-      const uint64_t slot = warp_append(first, &a.ctl->tc[par]);
-      if (first) a.T[slot] = v;
-    }
+  uint64_t x = 0;
+  if (b + lane < e) {
+    const uint32_t u = __ldg(a.slots + b + lane);
+    if (u != kSentinel) x = ldm(F, u);
   }
+  uint64_t got = warp_or64(x);
+  for (uint64_t base = b + 32; base < e && (got & need) != need && !done(got); base += 128) {
+    uint32_t u[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) u[q] = base + q * 32 + lane < e ? __ldg(a.slots + base + q * 32 + lane) : kSentinel;
+    x = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) x |= u[q] != kSentinel ? ldm(F, u[q]) : 0;
+    got |= warp_or64(x);
+  }
+  return got & need;
 }
 
 // Adds per-thread counts of a round's frontier to slot `cur`, one atomic pair
@@ -177,23 +236,21 @@ __device__ inline void ms_bfs_body(const MsArgs &a, GridBar *bar) {
     stm(a.X, i, 0);
     stm(a.planes, i, 0);  // plane 0; plane b is cleared before round 2^b
   }
-  for (uint64_t base = warp * 32; base < n; base += nwarps * 32) {
-    const uint64_t v = base + lane;
-    const uint64_t d = v < n ? a.off[v + 1] - a.off[v] : 0;
-    const bool heavy = d > a.heavy_deg && d <= a.hub_deg, mega = d > a.hub_deg;
-    const uint64_t s1 = warp_append(heavy, &c->nheavy);
-    if (heavy) a.H[s1] = (uint32_t)v;
-    if (__ballot_sync(kFull, mega)) {
-      const uint64_t s2 = warp_append(mega, &c->nmega);
-      if (mega) {
-        a.H[n - 1 - s2] = (uint32_t)v;
-        const uint64_t nch = (d + a.hub_deg - 1) / a.hub_deg;
-        const uint64_t cb = atomicAdd(&c->nmc, (unsigned long long)nch);
-        if (cb + nch <= a.ccap)
-          for (uint64_t t = 0; t < nch; t++) a.MC[cb + t] = v << 32 | t;
-        else
-          atomicOr(&c->bar.err, 2u);
-      }
+  for (uint64_t base = warp * 128; base < n; base += nwarps * 128) {
+    bool heavy[4];
+    uint32_t d[4], at[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const uint64_t v = base + q * 32 + lane;
+      d[q] = v < n ? (uint32_t)(a.off[v + 1] - a.off[v]) : 0;
+      heavy[q] = d[q] > a.heavy_deg && d[q] <= a.hub_deg;
+    }
+    uint32_t *const to = a.H + ms_places(heavy, &c->nheavy, at);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const uint32_t v = (uint32_t)(base + q * 32 + lane);
+      if (heavy[q]) to[at[q]] = v;
+      else if (d[q] > a.hub_deg) ms_hub(a, a.H, &c->nmega, a.MC, &c->nmc, v, d[q]);
     }
   }
   if (!grid_sync(bar, nb)) return;
@@ -238,10 +295,18 @@ __device__ inline void ms_bfs_body(const MsArgs &a, GridBar *bar) {
       const bool dense = fdeg + fcnt >= n / 64;
       // phase A: a round that left no list of its frontier; collect it from F
       if (!vload(&c->lvalid[prv])) {
-        for (uint64_t base = warp * 32; base < n; base += nwarps * 32) {
-          const uint64_t v = base + lane;
-          const bool has = v < n && ldm(F, v) != 0;
-          ms_list(a, prv, ppar, has, (uint32_t)v, has ? a.off[v + 1] - a.off[v] : 0);
+        for (uint64_t base = warp * 128; base < n; base += nwarps * 128) {
+          bool has[4];
+          uint32_t v[4], d[4];
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const uint64_t w = base + q * 32 + lane;
+            v[q] = (uint32_t)w;
+            has[q] = w < n && ldm(F, w) != 0;
+          }
+#pragma unroll
+          for (int q = 0; q < 4; q++) d[q] = has[q] ? (uint32_t)(a.off[v[q] + 1] - a.off[v[q]]) : 0;
+          ms_list(a, prv, ppar, has, v, d);
         }
         if (!grid_sync(bar, nb)) return;
       }
@@ -307,7 +372,10 @@ __device__ inline void ms_bfs_body(const MsArgs &a, GridBar *bar) {
             my_cnt++;
             my_deg += d;
           }
-          ms_list(a, cur, par, i < tcount, v, d);
+          const bool has1[1] = {i < tcount};
+          const uint32_t v1[1] = {v};
+          const uint32_t d1[1] = {(uint32_t)d};
+          ms_list(a, cur, par, has1, v1, d1);
           ms_levels(a, v, got, r);
         }
       }
@@ -319,30 +387,22 @@ __device__ inline void ms_bfs_body(const MsArgs &a, GridBar *bar) {
         c->tc[ppar] = 0;
       }
       uint64_t my_cnt = 0, my_deg = 0;
-      // light vertices: a thread each
+      // light vertices: a thread each, 8 neighbours in flight
       for (uint64_t base = warp * 32; base < n; base += nwarps * 32) {
         const uint64_t v = base + lane;
         uint64_t got = 0;
         if (v < n) {
           const uint64_t b = a.off[v], e = a.off[v + 1];
-          if (e - b <= a.heavy_deg) {
+          if (e - b <= a.heavy_deg) {  // (a longer one's seen and N are its warp's to write)
             const uint64_t sv = ldm(a.seen, v);
             const uint64_t need = a.full & ~sv;
             if (need) {
-              uint64_t j = b;
-              for (; j + 4 <= e; j += 4) {
-                const uint32_t u0 = __ldg(a.slots + j), u1 = __ldg(a.slots + j + 1);
-                const uint32_t u2 = __ldg(a.slots + j + 2), u3 = __ldg(a.slots + j + 3);
-                uint64_t f = u0 != kSentinel ? ldm(F, u0) : 0;
-                f |= u1 != kSentinel ? ldm(F, u1) : 0;
-                f |= u2 != kSentinel ? ldm(F, u2) : 0;
-                f |= u3 != kSentinel ? ldm(F, u3) : 0;
-                got |= f;
-                if ((got & need) == need) break;
-              }
-              for (; j < e && (got & need) != need; j++) {
-                const uint32_t u = __ldg(a.slots + j);
-                if (u != kSentinel) got |= ldm(F, u);
+              for (uint64_t j = b; j < e && (got & need) != need; j += 8) {
+                uint32_t u[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) u[q] = j + q < e ? __ldg(a.slots + j + q) : kSentinel;
+#pragma unroll
+                for (int q = 0; q < 8; q++) got |= u[q] != kSentinel ? ldm(F, u[q]) : 0;
               }
               got &= need;
               if (got) {
@@ -357,25 +417,14 @@ __device__ inline void ms_bfs_body(const MsArgs &a, GridBar *bar) {
         ms_levels(a, (uint32_t)v, got, r);
       }
       // warp vertices
+      uint64_t hv = warp < nheavy ? __ldcg(a.H + warp) : 0;  // the next vertex, loaded ahead
       for (uint64_t i = warp; i < nheavy; i += nwarps) {
-        const uint32_t v = __ldcg(a.H + i);
+        const uint32_t v = (uint32_t)hv;
+        if (i + nwarps < nheavy) hv = __ldcg(a.H + i + nwarps);
         const uint64_t sv = ldm(a.seen, v);
         const uint64_t need = a.full & ~sv;
         const uint64_t b = a.off[v], e = a.off[v + 1];
-        uint64_t got = 0;
-        if (need) {
-          for (uint64_t base = b; base < e; base += 32) {
-            const uint64_t j = base + lane;
-            uint64_t x = 0;
-            if (j < e) {
-              const uint32_t u = __ldg(a.slots + j);
-              if (u != kSentinel) x = ldm(F, u);
-            }
-            got |= warp_or64(x);
-            if ((got & need) == need) break;
-          }
-          got &= need;
-        }
+        const uint64_t got = need ? ms_pull_range(a, F, b, e, need, [](uint64_t) { return false; }) : 0;
         if (lane == 0) {
           stm(N, v, got);
           if (got) {
@@ -394,20 +443,12 @@ __device__ inline void ms_bfs_body(const MsArgs &a, GridBar *bar) {
         if (!need) continue;
         const uint64_t b = a.off[v] + (uint64_t)(uint32_t)ch * a.hub_deg;
         const uint64_t e = min(b + a.hub_deg, a.off[v + 1]);
-        uint64_t got = 0;
-        uint32_t it = 0;
-        for (uint64_t base = b; base < e; base += 32, it++) {
-          const uint64_t j = base + lane;
-          uint64_t x = 0;
-          if (j < e) {
-            const uint32_t u = __ldg(a.slots + j);
-            if (u != kSentinel) x = ldm(F, u);
-          }
-          got |= warp_or64(x);
-          if ((got & need) == need) break;
-          if ((it & 7) == 7 && ((got | ldm(a.X, v)) & need) == need) break;
-        }
-        got &= need;
+        const uint64_t got = ms_pull_range(a, F, b, e, need, [&](uint64_t x) {
+          // with what other chunks found: they may be writing it, so one lane's
+          // view decides for all (the lanes go on together)
+          x |= ldm(a.X, v);
+          return (__shfl_sync(kFull, x, 0) & need) == need;
+        });
         if (lane == 0 && (got & ~ldm(a.X, v))) atomicOr((unsigned long long *)a.X + v, (unsigned long long)got);
       }
       if (nmega) {
@@ -471,19 +512,52 @@ __device__ __forceinline__ void ms_store_level(const MsArgs &a, uint32_t s, uint
   __stcs(a.levels + (uint64_t)s * a.n + v, lv);
 }
 
-// The levels from the bit planes, a thread per vertex: level of (s, v) =
-// sum over planes b of bit s of plane b, << b.  Up to 8 planes (levels below
-// 256) the levels of 8 sources at a time are assembled as bytes of one word,
-// a spread8 per plane; deeper traversals take them bit by bit.  Per source a
-// warp stores 32 consecutive words.
+// The levels from the bit planes: level of (s, v) = sum over planes b of bit s
+// of plane b, << b.  Up to 8 planes (levels below 256) the levels of 8 sources
+// at a time are assembled as bytes of one word, a spread8 per plane; deeper
+// traversals take them bit by bit.  Per source a warp stores 128 (or 32)
+// consecutive words.
 __device__ inline void ms_levels_body(const MsArgs &a, uint64_t tid, uint64_t nthr) {
   const uint32_t last = a.ctl->rounds;
   const int used = last ? min(32 - __clz((int)last), kLevelBits) : 0;
   const uint64_t n = a.n;
   const uint32_t k = a.k;
-  for (uint64_t v = tid; v < n; v += nthr) {
-    const uint64_t sv = __ldcs(a.seen + v);
-    if (used <= 8) {
+  if (used <= 8) {
+    // Levels below 256: the levels of 8 sources at a time as the bytes of one
+    // word, for 4 vertices a thread where 16-byte stores fit.  `seen` tells the
+    // pairs that were reached (a source reaches itself, at level 0).
+    const bool wide = n % 4 == 0 && (reinterpret_cast<uintptr_t>(a.levels) & 15) == 0;
+    if (wide) {
+      for (uint64_t v = 4 * tid; v < n; v += 4 * nthr) {
+        uint64_t sv[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) sv[j] = __ldcs(a.seen + v + j);
+        for (uint32_t s0 = 0; s0 < k; s0 += 8) {
+          uint64_t packed[4] = {0, 0, 0, 0};
+          for (int b = 0; b < used; b++) {
+            const ulonglong2 *pl = reinterpret_cast<const ulonglong2 *>(a.planes + (uint64_t)b * n + v);
+            const ulonglong2 x = __ldcg(pl), y = __ldcg(pl + 1);
+            packed[0] |= spread8(x.x >> s0) << b;
+            packed[1] |= spread8(x.y >> s0) << b;
+            packed[2] |= spread8(y.x >> s0) << b;
+            packed[3] |= spread8(y.y >> s0) << b;
+          }
+#pragma unroll
+          for (uint32_t i = 0; i < 8; i++) {
+            uint32_t lv[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)  // all ones where the bit is off (then the level is 0)
+              lv[j] = ((uint32_t)(packed[j] >> (8 * i)) & 0xFFu) | (((uint32_t)(sv[j] >> (s0 + i)) & 1u) - 1u);
+            if (s0 + i < k)
+              __stcs(reinterpret_cast<uint4 *>(a.levels + (uint64_t)(s0 + i) * n + v),
+                     make_uint4(lv[0], lv[1], lv[2], lv[3]));
+          }
+        }
+      }
+      return;
+    }
+    for (uint64_t v = tid; v < n; v += nthr) {
+      const uint64_t sv = __ldcs(a.seen + v);
       uint64_t pl[8];
 #pragma unroll
       for (int b = 0; b < 8; b++) pl[b] = b < used ? __ldcs(a.planes + (uint64_t)b * n + v) : 0;
@@ -493,14 +567,19 @@ __device__ inline void ms_levels_body(const MsArgs &a, uint64_t tid, uint64_t nt
         for (int b = 0; b < 8; b++) packed |= spread8(pl[b] >> s0) << b;
 #pragma unroll
         for (uint32_t i = 0; i < 8; i++)
-          if (s0 + i < k) ms_store_level(a, s0 + i, v, (uint32_t)(packed >> (8 * i)) & 0xFFu, sv);
+          if (s0 + i < k)
+            __stcs(a.levels + (uint64_t)(s0 + i) * n + v,
+                   ((uint32_t)(packed >> (8 * i)) & 0xFFu) | (((uint32_t)(sv >> (s0 + i)) & 1u) - 1u));
       }
-    } else {
-      for (uint32_t s = 0; s < k; s++) {
-        uint32_t lv = 0;
-        for (int b = 0; b < used; b++) lv |= (uint32_t)((__ldg(a.planes + (uint64_t)b * n + v) >> s) & 1) << b;
-        ms_store_level(a, s, v, lv, sv);
-      }
+    }
+    return;
+  }
+  for (uint64_t v = tid; v < n; v += nthr) {
+    const uint64_t sv = __ldcs(a.seen + v);
+    for (uint32_t s = 0; s < k; s++) {
+      uint32_t lv = 0;
+      for (int b = 0; b < used; b++) lv |= (uint32_t)((ldm(a.planes, (uint64_t)b * n + v) >> s) & 1) << b;
+      ms_store_level(a, s, v, lv, sv);
     }
   }
 }
