@@ -445,7 +445,7 @@ __device__ __forceinline__ T group_total(T s, T c) {
 // Work units of at most kPrTile + kPrLightMax slots, all processed by one
 // kernel so every CTA streams the same amount:
 //   light tile   consecutive vertices with runs <= kPrLightMax; one run of
-//                slots; per-vertex sums written directly
+//                slots; FP32 finishes its vertices, FP64 writes their sums
 //   heavy chunk  kPrTile consecutive slots of one heavier vertex; its
 //                compensated partial goes to part[chunk] and k_pr_combine sums
 //                a vertex's chunks in order
@@ -555,20 +555,102 @@ __global__ void k_pr_desc_chunks(const uint64_t *__restrict__ off, const uint32_
       d.v0 = v;
       d.v1 = kNoVertex;
       d.chunk = (uint32_t)(cbase[h] + k);
-      d.pad = cbase[h + 1] - cbase[h] == 1;  // the vertex's only chunk: its unit finishes it
+      d.pad = cbase[h + 1] - cbase[h] == 1;  // the vertex's only chunk
       desc[base + cbase[h] + k] = d;
     }
   }
 }
 
-template <bool kComp, typename T>
-__device__ __forceinline__ void pr_finish(uint64_t v, T tot, const uint32_t *__restrict__ deg,
-                                          const T *__restrict__ p_curr, T *__restrict__ p_next,
-                                          T *__restrict__ pdiv_out, T damping, T added, double &l1loc) {
-  T p = damping * tot + added;
-  p_next[v] = p;
-  pdiv_out[v] = p / (T)deg[v];
-  l1loc += fabs((double)p_curr[v] - (double)p);
+// State of the iteration loop (device side).
+struct PrLoop {
+  double l1;
+  uint32_t iters;
+  int32_t last;  // -1: no iteration ran; 0: the last iterate is in pb; 1: in pa
+};
+
+// One iteration: what its three kernels read and write.
+template <typename T>
+struct PrIter {
+  const uint64_t *off;
+  const uint32_t *slots, *deg;
+  const PrDesc *desc;
+  const uint64_t *counts;  // light tiles, heavy chunks
+  const uint32_t *heavy;
+  const uint64_t *cbase;
+  uint64_t nheavy, n;
+  const T *pdiv_in, *p_curr, *rdeg;  // rdeg: 1 / degree (FP64 only)
+  T *p_next, *pdiv_out;
+  T *part, *sum;  // chunk partials; every vertex's sum over its neighbours
+  T damping, added;
+  double *l1;          // the iteration's L1 distance, 0 between iterations
+  unsigned int *done;  // blocks of the last kernel that are done
+  PrLoop *loop;
+  double eps;
+  uint32_t max_iters;
+  int half, in_graph;
+  cudaGraphConditionalHandle h_if, h_while;
+};
+
+// Where vertices are finished (their iterate, shares and L1 distance, from their
+// sums).  An FP64 instruction takes the SM's FP64 pipe 19 cycles however many
+// lanes are active, and finishing takes ~30 of them in FP64 and 4 in FP32 (the L1
+// norm is FP64 in every precision).  FP32: by the warp that has the sum, hidden
+// behind its gathers (a kernel of its own takes 45 us an iteration at RMAT 2^22
+// and saves the units 4).  FP64: by k_pr_finish with full warps; the units, with one
+// heavy vertex or a tile's few at a time, kept the pipe 57% busy with it.  At RMAT
+// 2^20 with 2^24 draws, an iteration: units 322 -> 157 us, combining 19, finishing
+// 22; 20 iterations 6.9 -> 4.3 ms.
+template <typename T>
+constexpr bool kPrInPlace = sizeof(T) == 4;
+
+// p / d from r = 1 / d: the quotient's error is computed exactly by a fused
+// multiply-add and corrected (Markstein, IBM J. Res. Dev. 34, 1990: correctly
+// rounded when r is, away from the ends of the exponent range).  3 FP64
+// instructions where a division takes about 12.
+__device__ __forceinline__ double pr_divide(double p, double d, double r) {
+  const double q = __dmul_rn(p, r);
+  if ((__double2hiint(q) & 0x7FF00000) == 0x7FF00000) return q;  // infinite or NaN
+  return __fma_rn(__fma_rn(-q, d, p), r, q);
+}
+__device__ __forceinline__ float pr_divide(float p, float d, float) { return p / d; }
+
+template <typename T>
+__device__ __forceinline__ void pr_finish(const PrIter<T> &a, uint64_t v, T tot, double &l1loc) {
+  const T p = a.damping * tot + a.added;
+  const uint32_t d = __ldg(a.deg + v);
+  const T before = __ldg(a.p_curr + v);
+  const T r = sizeof(T) == 8 ? __ldg(a.rdeg + v) : T(0);
+  a.p_next[v] = p;
+  a.pdiv_out[v] = d ? pr_divide(p, (T)d, r) : (T)INFINITY;
+  l1loc += fabs((double)before - (double)p);
+}
+
+// The end of an iteration's last kernel: the last block to finish records the
+// distance, clears the accumulators and, in a graph, tells the loop whether
+// another iteration runs (PageRank.h:176-190: stop when L1 < eps or after
+// max_iters).  half 0 ends the first iteration of a loop body (pa -> pb) and
+// sets both conditions; half 1 ends the second (pb -> pa) and sets the loop's.
+template <typename T>
+__device__ __forceinline__ void pr_end(const PrIter<T> &a, double l1loc, double *sm) {
+  if (__syncthreads_or(l1loc != 0.0)) l1loc = block_sum(l1loc, sm);  // FP64 adds: 64 cycles each, in a row
+  if (threadIdx.x) return;
+  if (gridDim.x > 1) {
+    if (l1loc != 0.0) atomicAdd(a.l1, l1loc);
+    __threadfence();
+    if (atomicAdd(a.done, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    l1loc = 0.0;
+  }
+  const uint32_t it = ++a.loop->iters;
+  const double L = __ldcg(a.l1) + l1loc;
+  a.loop->l1 = L;
+  a.loop->last = a.half;
+  *a.l1 = 0.0;
+  *a.done = 0;
+  if (!a.in_graph) return;  // the host reads the state and decides
+  const unsigned cont = (!(L < a.eps) && it < a.max_iters) ? 1u : 0u;
+  if (a.half == 0) cudaGraphSetConditional(a.h_if, cont);
+  cudaGraphSetConditional(a.h_while, cont);
 }
 
 // (s, c) += (s2, c2), compensated when kComp (TwoSum of the sums, errors added)
@@ -610,21 +692,20 @@ __device__ __forceinline__ uint32_t last_head_below(const uint32_t *flags, uint3
 // crosses chunk boundaries is carried by an inclusive segmented warp scan (a
 // lane holding a head starts a new segment) and the run open at a lane's
 // start is completed by the lane that holds its end.  Each run's total is
-// written over the staged value of its first slot, and a last pass finishes
-// the tile's vertices a lane each (consecutive vertices, coalesced).  One
-// fixed order per graph, so results are deterministic.
+// written over the staged value of its first slot, and a last pass finishes (or
+// writes the sums of) the tile's vertices, a lane each (consecutive vertices,
+// coalesced).  One fixed order per graph, so results are deterministic.
 template <bool kComp, typename T>
 __device__ __forceinline__ void pr_light_tile(const PrDesc &d, uint32_t len, T *buf, uint32_t *flags,
-                                              const uint64_t *__restrict__ off, const uint32_t *__restrict__ deg,
-                                              const T *__restrict__ p_curr, T *__restrict__ p_next,
-                                              T *__restrict__ pdiv_out, T damping, T added, double &l1loc) {
+                                              const PrIter<T> &a, double &l1loc) {
+  const uint64_t *__restrict__ off = a.off;
   const unsigned lane = lane_id();
   for (uint32_t w = lane; w < kPrFlagWords; w += 32) flags[w] = 0;
   __syncwarp();
   for (uint32_t x = d.v0 + lane; x < d.v1; x += 32) {
-    const uint64_t a = off[x], b = off[x + 1];
-    if (b > a) {
-      const uint32_t r0 = (uint32_t)(a - d.s0);
+    const uint64_t b = off[x], e = off[x + 1];
+    if (e > b) {
+      const uint32_t r0 = (uint32_t)(b - d.s0);
       atomicOr(flags + (r0 >> 5), 1u << (r0 & 31));
     }
   }
@@ -676,42 +757,38 @@ __device__ __forceinline__ void pr_light_tile(const PrDesc &d, uint32_t len, T *
     buf[last_head_below(flags, len)] = kComp ? ss + sc : ss;
   __syncwarp();
   for (uint32_t x = d.v0 + lane; x < d.v1; x += 32) {
-    const uint64_t a = off[x], b = off[x + 1];
-    pr_finish<kComp, T>(x, b > a ? buf[a - d.s0] : T(0), deg, p_curr, p_next, pdiv_out, damping, added, l1loc);
+    const uint64_t b = off[x], e = off[x + 1];
+    const T tot = e > b ? buf[b - d.s0] : T(0);
+    if constexpr (kPrInPlace<T>) pr_finish(a, x, tot, l1loc); else a.sum[x] = tot;
   }
   __syncwarp();
 }
 
 // One warp per unit, no block-wide barriers: the warp gathers p_div of the
 // unit's slots (16 independent loads per lane in flight) into its own stage in
-// shared memory, then reduces.  Light tile: runs of <= 32 one lane each, longer
-// runs (found by ballot) one warp each.  Heavy chunk: warp partial to part[];
-// with kDirectHeavy (FP64) each lane sums its gathered slots lane, lane+32, ...
-// in registers without the stage, in the same order: measured at RMAT 2^22,
-// 20 FP64 iterations 34.0 -> 28.8 ms, while FP32 runs 1% faster staged.
+// shared memory, then reduces.  Light tile: pr_light_tile.  Heavy chunk: warp
+// partial to part[]; with kDirectHeavy (FP64) each lane sums its gathered slots
+// lane, lane+32, ... in registers without the stage, in the same order:
+// measured at RMAT 2^22, 20 FP64 iterations 34.0 -> 28.8 ms, while FP32 runs 1%
+// faster staged.  FP64 takes 64 registers (4 CTAs an SM): 48 spill the gathers
+// in flight, 263 against 207 us an iteration at RMAT 2^20.
 template <bool kComp, typename T, bool kDirectHeavy>
-__global__ void __launch_bounds__(kPrBlock, 5) k_pr_units(const uint64_t *__restrict__ off,
-                                                       const uint32_t *__restrict__ slots,
-                                                       const uint32_t *__restrict__ deg,
-                                                       const PrDesc *__restrict__ desc,
-                                                       const uint64_t *__restrict__ counts,
-                                                       const T *__restrict__ pdiv_in, const T *__restrict__ p_curr,
-                                                       T *__restrict__ p_next, T *__restrict__ pdiv_out,
-                                                       T *__restrict__ part, T damping, T added, double *l1) {
+__global__ void __launch_bounds__(kPrBlock, sizeof(T) == 8 ? 4 : 5) k_pr_units(PrIter<T> a) {
   extern __shared__ __align__(16) unsigned char pr_smem[];
   __shared__ double sm[kPrBlock / 32 + 1];
-  const uint64_t nunits = counts[0] + counts[1];  // light tiles + heavy chunks
+  double l1loc = 0.0;
+  const uint64_t nunits = a.counts[0] + a.counts[1];  // light tiles + heavy chunks
+  const T *__restrict__ pdiv_in = a.pdiv_in;
   const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
   T *buf = reinterpret_cast<T *>(pr_smem) + (size_t)warp * kPrStage;
   uint32_t *flags = reinterpret_cast<uint32_t *>(reinterpret_cast<T *>(pr_smem) + (size_t)(kPrBlock / 32) * kPrStage) +
                     (size_t)warp * kPrFlagWords;
   const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  double l1loc = 0.0;
   for (uint64_t t = gw; t < nunits; t += nw) {
-    const PrDesc d = desc[t];
+    const PrDesc d = a.desc[t];
     const uint32_t len = (uint32_t)(d.s1 - d.s0);
-    const uint32_t *id = slots + d.s0;
+    const uint32_t *__restrict__ id = a.slots + d.s0;
     if (d.v1 == kNoVertex && kDirectHeavy) {
       T s = T(0), c = T(0);
       for (uint32_t i = lane; i < len; i += 32 * 16) {
@@ -726,14 +803,7 @@ __global__ void __launch_bounds__(kPrBlock, 5) k_pr_units(const uint64_t *__rest
           if (i + 32 * q < len) acc_add<kComp>(s, c, g[q]);
       }
       T tot = group_total<kComp, T, 32>(s, c);
-      if (lane == 0) {
-        if (d.pad) {
-          pr_finish<kComp, T>(d.v0, tot, deg, p_curr, p_next, pdiv_out, damping, added, l1loc);
-        } else {
-          part[2 * (uint64_t)d.chunk] = tot;
-          part[2 * (uint64_t)d.chunk + 1] = T(0);
-        }
-      }
+      if (lane == 0) a.part[d.chunk] = tot;
       continue;
     }
     for (uint32_t i = lane; i < len; i += 32 * 16) {
@@ -746,110 +816,104 @@ __global__ void __launch_bounds__(kPrBlock, 5) k_pr_units(const uint64_t *__rest
     }
     __syncwarp();
     if (d.v1 != kNoVertex) {
-      pr_light_tile<kComp, T>(d, len, buf, flags, off, deg, p_curr, p_next, pdiv_out, damping, added, l1loc);
+      pr_light_tile<kComp, T>(d, len, buf, flags, a, l1loc);
     } else {
       T s = T(0), c = T(0);
       for (uint32_t r = lane; r < len; r += 32) acc_add<kComp>(s, c, buf[r]);
       T tot = group_total<kComp, T, 32>(s, c);
       if (lane == 0) {
-        if (d.pad) {
-          pr_finish<kComp, T>(d.v0, tot, deg, p_curr, p_next, pdiv_out, damping, added, l1loc);
-        } else {
-          part[2 * (uint64_t)d.chunk] = tot;
-          part[2 * (uint64_t)d.chunk + 1] = T(0);
-        }
+        if (kPrInPlace<T> && d.pad) pr_finish(a, d.v0, tot, l1loc); else a.part[d.chunk] = tot;
       }
     }
     __syncwarp();
   }
-  l1loc = block_sum(l1loc, sm);
-  if (threadIdx.x == 0 && l1loc != 0.0) atomicAdd(l1, l1loc);
+  if constexpr (kPrInPlace<T>) {
+    l1loc = block_sum(l1loc, sm);
+    if (threadIdx.x == 0 && l1loc != 0.0) atomicAdd(a.l1, l1loc);
+  }
 }
 
-// A group of kCombineLanes lanes per heavy vertex (32 / kCombineLanes
-// vertices per warp; most heavy vertices have a few chunks): its chunk
-// partials, lane l of the group taking chunks l, l + G, ... in order, summed
-// by a fixed tree over the group; then the vertex is finished by the group's
-// first lane.  Measured at RMAT 2^22 (ms per iteration of units + combine):
-// groups of 32 / 8 / 4 lanes 0.563 / 0.543 / 0.549.
+// FP32: a group of kCombineLanes lanes per heavy vertex of several chunks (most
+// have a few): its chunk partials, lane l of the group taking chunks l, l + G,
+// ... in order, summed by a fixed tree over the group; then the vertex is
+// finished by the group's first lane.  Measured at RMAT 2^22 (ms per iteration
+// of units + combine): groups of 32 / 8 / 4 lanes 0.563 / 0.543 / 0.549.
+// FP64: the heavy vertices' sums, a lane each, for an addition costs a warp the
+// same whatever lanes take part: up to 8 partials by the same tree in a lane,
+// more by the warp.
 constexpr int kCombineLanes = 8;
 template <bool kComp, typename T>
-__global__ void __launch_bounds__(256) k_pr_combine(const uint32_t *__restrict__ heavy,
-                                                    const uint64_t *__restrict__ cbase, uint64_t nheavy,
-                                                    const T *__restrict__ part, const uint32_t *__restrict__ deg,
-                                                    const T *__restrict__ p_curr, T *__restrict__ p_next,
-                                                    T *__restrict__ pdiv_out, T damping, T added, double *l1) {
+__global__ void __launch_bounds__(256) k_pr_combine(PrIter<T> a) {
   __shared__ double sm[9];
-  constexpr int kPer = 32 / kCombineLanes;
-  const unsigned lane = lane_id(), gl = lane % kCombineLanes;
+  const unsigned lane = lane_id();
   const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  double l1loc = 0.0;
-  for (uint64_t base = gw * kPer; base < nheavy; base += nw * kPer) {
-    const uint64_t h = base + lane / kCombineLanes;
-    T s = T(0), c = T(0);
-    bool mine = false;  // a vertex of several chunks (one chunk: finished by its unit)
-    if (h < nheavy) {
-      const uint64_t c0 = cbase[h], c1 = cbase[h + 1];
-      mine = c1 - c0 > 1;
-      if (mine)
-        for (uint64_t k = c0 + gl; k < c1; k += kCombineLanes) {
-          acc_add<kComp>(s, c, part[2 * k]);
-          if (kComp) c += part[2 * k + 1];
-        }
+  if constexpr (kPrInPlace<T>) {
+    constexpr int kPer = 32 / kCombineLanes;
+    const unsigned gl = lane % kCombineLanes;
+    double l1loc = 0.0;
+    for (uint64_t base = gw * kPer; base < a.nheavy; base += nw * kPer) {
+      const uint64_t h = base + lane / kCombineLanes;
+      T s = T(0), c = T(0);
+      bool mine = false;  // a vertex of several chunks (one chunk: finished by its unit)
+      if (h < a.nheavy) {
+        const uint64_t c0 = a.cbase[h], c1 = a.cbase[h + 1];
+        mine = c1 - c0 > 1;
+        if (mine)
+          for (uint64_t k = c0 + gl; k < c1; k += kCombineLanes) acc_add<kComp>(s, c, a.part[k]);
+      }
+      const T tot = group_total<kComp, T, kCombineLanes>(s, c);
+      if (mine && gl == 0) pr_finish(a, a.heavy[h], tot, l1loc);
     }
-    const T tot = group_total<kComp, T, kCombineLanes>(s, c);
-    if (mine && gl == 0)
-      pr_finish<kComp, T>(heavy[h], tot, deg, p_curr, p_next, pdiv_out, damping, added, l1loc);
+    pr_end(a, l1loc, sm);
+  } else {
+    for (uint64_t base = gw * 32; base < a.nheavy; base += nw * 32) {
+      const uint64_t h = base + lane;
+      const uint64_t c0 = h < a.nheavy ? a.cbase[h] : 0, c1 = h < a.nheavy ? a.cbase[h + 1] : 0;
+      const bool wide = c1 - c0 > kCombineLanes;
+      T s[kCombineLanes], c[kCombineLanes];
+#pragma unroll
+      for (int k = 0; k < kCombineLanes; k++) {
+        s[k] = !wide && c0 + k < c1 ? a.part[c0 + k] : T(0);
+        c[k] = T(0);
+      }
+#pragma unroll
+      for (int o = kCombineLanes / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < o; k++) acc_merge<kComp>(s[k], c[k], s[k + o], c[k + o]);
+      T tot = kComp ? s[0] + c[0] : s[0];
+      for (unsigned m = __ballot_sync(kFull, wide); m; m &= m - 1) {
+        const int o = __ffs(m) - 1;
+        const uint64_t a0 = __shfl_sync(kFull, c0, o), a1 = __shfl_sync(kFull, c1, o);
+        T x = T(0), y = T(0);
+        for (uint64_t k = a0 + lane; k < a1; k += 32) acc_add<kComp>(x, y, a.part[k]);
+        const T t = group_total<kComp, T, 32>(x, y);
+        if ((int)lane == o) tot = t;
+      }
+      if (h < a.nheavy) a.sum[a.heavy[h]] = tot;
+    }
   }
-  l1loc = block_sum(l1loc, sm);
-  if (threadIdx.x == 0 && l1loc != 0.0) atomicAdd(l1, l1loc);
+}
+
+// FP64: the vertices from their sums, a thread each.
+template <typename T>
+__global__ void __launch_bounds__(256) k_pr_finish(PrIter<T> a) {
+  __shared__ double sm[9];
+  double l1loc = 0.0;
+  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < a.n; v += (uint64_t)gridDim.x * blockDim.x)
+    pr_finish(a, v, a.sum[v], l1loc);
+  pr_end(a, l1loc, sm);
 }
 
 template <typename T>
-__global__ void k_pr_init(const uint32_t *__restrict__ deg, uint64_t n, T *p_curr, T *pdiv, T one_over_n) {
+__global__ void k_pr_init(const uint32_t *__restrict__ deg, uint64_t n, T *p_curr, T *pdiv, T *rdeg, T one_over_n) {
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n;
        v += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t d = deg[v];
     p_curr[v] = one_over_n;
-    pdiv[v] = one_over_n / (T)deg[v];
+    pdiv[v] = one_over_n / (T)d;
+    if (rdeg && d) rdeg[v] = T(1) / (T)d;
   }
-}
-
-// State of the graph-driven iteration loop (device side).
-struct PrLoop {
-  double l1;
-  uint32_t iters;
-  int32_t last;  // -1: no iteration ran; 0: the last iterate is in pb; 1: in pa
-};
-
-// After an iteration: records its L1 norm, clears the accumulators, and
-// tells the loop whether another iteration runs (PageRank.h:176-190: stop
-// when L1 < eps or after max_iters).  half 0 ends the first iteration of a
-// loop body (pa -> pb) and sets both conditions; half 1 ends the second
-// (pb -> pa) and sets the loop's.
-__global__ void k_pr_check(double *d_l1, double eps, uint32_t max_iters, PrLoop *st, int half,
-                           cudaGraphConditionalHandle h_if, cudaGraphConditionalHandle h_while) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const uint32_t it = ++st->iters;
-  const double L = d_l1[0];
-  st->l1 = L;
-  st->last = half;
-  d_l1[0] = 0.0;
-  d_l1[1] = 0.0;
-  const unsigned cont = (!(L < eps) && it < max_iters) ? 1u : 0u;
-  if (half == 0) cudaGraphSetConditional(h_if, cont);
-  cudaGraphSetConditional(h_while, cont);
-}
-
-// k_pr_check for stream launches: records the iteration's L1 and clears the
-// accumulators; the host reads the state and decides.
-__global__ void k_pr_check_plain(double *d_l1, PrLoop *st, int half) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  ++st->iters;
-  st->l1 = d_l1[0];
-  st->last = half;
-  d_l1[0] = 0.0;
-  d_l1[1] = 0.0;
 }
 
 template <typename T>
@@ -899,7 +963,12 @@ static int pagerank_impl(byo_graph *g, double eps, uint32_t max_iters, double *d
   BYO_CU(ctx, cudaMemcpyAsync(counts + 1, tot, 8, cudaMemcpyDeviceToDevice, ctx->stream));
   h[3] = n;  // h[3] is not written again before the next synchronisation
   BYO_CU(ctx, cudaMemcpyAsync(tstart + ntiles, h + 3, 4, cudaMemcpyHostToDevice, ctx->stream));
-  launch(ctx, k_pr_init<T>, dim3(grid_for(ctx, n, 256)), dim3(256), 0, (const uint32_t *)g->d_deg, n, pa, da,
+  T *sum = nullptr, *rdeg = nullptr;
+  if (!kPrInPlace<T>) {
+    BYO_TRY(ws(g, WS_LP, n, &sum));
+    BYO_TRY(ws(g, WS_FRONT_LIST_A, n, &rdeg));
+  }
+  launch(ctx, k_pr_init<T>, dim3(grid_for(ctx, n, 256)), dim3(256), 0, (const uint32_t *)g->d_deg, n, pa, da, rdeg,
          (T)(1.0 / (double)n));
   const uint64_t max_chunks = g->nslots / kPrTile + nheavy + 1;
   // descriptors: compacted light tiles, then heavy chunks
@@ -911,10 +980,10 @@ static int pagerank_impl(byo_graph *g, double eps, uint32_t max_iters, double *d
     launch(ctx, k_pr_desc_chunks, dim3(grid_for(ctx, nheavy, 256)), dim3(256), 0, (const uint64_t *)g->d_off,
            (const uint32_t *)heavy, (const uint64_t *)cbase, nheavy, (const uint64_t *)counts, desc);
   T *part = nullptr;
-  BYO_TRY(ws(g, WS_TC_CNT, 2 * max_chunks + 2, &part));
+  BYO_TRY(ws(g, WS_TC_CNT, max_chunks + 2, &part));
   const T damping = (T)0.85;
   const T added = (T)((1 - 0.85) * (1 / (double)n));
-  const int grid_c = grid_for(ctx, nheavy * kCombineLanes, 256, 8);
+  const int grid_c = grid_for(ctx, kPrInPlace<T> ? nheavy * kCombineLanes : nheavy, 256, 8);
   const size_t units_smem = (size_t)(kPrBlock / 32) * pr_warp_smem<T>();
   BYO_CU(ctx, cudaFuncSetAttribute(k_pr_units<kComp, T, sizeof(T) == 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)units_smem));
@@ -924,14 +993,21 @@ static int pagerank_impl(byo_graph *g, double eps, uint32_t max_iters, double *d
   const int grid_u = grid_for(ctx, (ntiles + max_chunks) * 32, kPrBlock, units_per_sm > 0 ? units_per_sm : 1);
   // The iterations run as one CUDA graph: a WHILE node whose body holds two
   // iterations (pa -> pb, then under an IF node pb -> pa), each ending in
-  // k_pr_check, which sets the conditions from the L1 norm on the device.
+  // pr_end, which sets the conditions from the L1 norm on the device.
   // No host round trip happens between iterations.
   PrLoop *loop = reinterpret_cast<PrLoop *>((reinterpret_cast<uintptr_t>(db + n + 2) + 7) & ~(uintptr_t)7);
+  unsigned int *done = reinterpret_cast<unsigned int *>(d_l1 + 1);
   BYO_CU(ctx, cudaMemsetAsync(d_l1, 0, 16, ctx->stream));
   {
     PrLoop z{0.0, 0u, -1};
     BYO_CU(ctx, cudaMemcpyAsync(loop, &z, sizeof(PrLoop), cudaMemcpyHostToDevice, ctx->stream));
   }
+  PrIter<T> iter[2];
+  for (int h : {0, 1})
+    iter[h] = PrIter<T>{g->d_off, g->d_slots, g->d_deg, desc, counts, heavy, cbase, nheavy, n, h ? db : da,
+                        h ? pb : pa, rdeg, h ? pa : pb, h ? da : db, part, sum, damping, added, d_l1, done, loop, eps,
+                        max_iters, h, ctx->pr_graphs ? 1 : 0, 0, 0};
+  const int grid_f = grid_for(ctx, n, 256);
   uint32_t it = 0;
   double L1 = 0.0;
   const T *last = pa;
@@ -940,18 +1016,11 @@ static int pagerank_impl(byo_graph *g, double eps, uint32_t max_iters, double *d
     // each iteration (the same kernels in the same order: the same results)
     PrLoop *hs = nullptr;
     BYO_TRY(pinned(ctx, 4096, (void **)&hs));
-    const T *pdiv_in[2] = {da, db}, *pcur[2] = {pa, pb};
-    T *pnext[2] = {pb, pa}, *pdiv_out[2] = {db, da};
     for (int hh = 0;; hh ^= 1) {
-      launch_t(ctx, "pr_pull", k_pr_units<kComp, T, sizeof(T) == 8>, dim3(grid_u), dim3(kPrBlock), units_smem,
-               (const uint64_t *)g->d_off, (const uint32_t *)g->d_slots, (const uint32_t *)g->d_deg,
-               (const PrDesc *)desc, (const uint64_t *)counts, pdiv_in[hh], pcur[hh], pnext[hh], pdiv_out[hh], part,
-               damping, added, d_l1);
-      if (nheavy)
-        launch_t(ctx, "pr_pull", k_pr_combine<kComp, T>, dim3(grid_c), dim3(256), 0, (const uint32_t *)heavy,
-                 (const uint64_t *)cbase, nheavy, (const T *)part, (const uint32_t *)g->d_deg, pcur[hh], pnext[hh],
-                 pdiv_out[hh], damping, added, d_l1);
-      launch(ctx, k_pr_check_plain, dim3(1), dim3(32), 0, d_l1, loop, hh);
+      launch_t(ctx, "pr_pull", k_pr_units<kComp, T, sizeof(T) == 8>, dim3(grid_u), dim3(kPrBlock), units_smem, iter[hh]);
+      if (nheavy || kPrInPlace<T>)
+        launch_t(ctx, "pr_pull", k_pr_combine<kComp, T>, dim3(grid_c), dim3(256), 0, iter[hh]);
+      if (!kPrInPlace<T>) launch_t(ctx, "pr_pull", k_pr_finish<T>, dim3(grid_f), dim3(256), 0, iter[hh]);
       BYO_CU(ctx, cudaMemcpyAsync(hs, loop, sizeof(PrLoop), cudaMemcpyDeviceToHost, ctx->stream));
       BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
       if (hs->l1 < eps || hs->iters >= max_iters) break;
@@ -985,59 +1054,31 @@ static int pagerank_impl(byo_graph *g, double eps, uint32_t max_iters, double *d
     if (rc == BYO_OK &&
         (e = cudaGraphConditionalHandleCreate(&h_if, graph, 0, cudaGraphCondAssignDefault)) != cudaSuccess)
       fail("pagerank half condition", e);
-    // one iteration: units, combine, check; returns its last node
-    const uint64_t *off_ = g->d_off;
-    const uint32_t *slots_ = g->d_slots, *deg_ = g->d_deg, *heavy_ = heavy;
-    const uint64_t *cbase_ = cbase;
-    const PrDesc *desc_ = desc;
-    const uint64_t *counts_ = counts;
-    T *pa_ = pa, *pb_ = pb, *da_ = da, *db_ = db;
-    double *l1_ = d_l1;
-    PrLoop *loop_ = loop;
-    const double eps_ = eps;
-    const uint32_t maxit_ = max_iters;
-    T damping_ = damping, added_ = added;
-    uint64_t nheavy_ = nheavy;
-    int half0 = 0, half1 = 1;
-    const T *pdiv_in[2] = {da_, db_}, *pcur[2] = {pa_, pb_};
-    T *pnext[2] = {pb_, pa_}, *pdiv_out[2] = {db_, da_};
+    // one iteration: units, combine, FP64's finish; returns its last node
+    for (int h : {0, 1}) {
+      iter[h].h_if = h_if;
+      iter[h].h_while = h_while;
+    }
     auto add_iter = [&](cudaGraph_t gr, int h, cudaGraphNode_t dep, cudaGraphNode_t *lastn) {
-      if (rc != BYO_OK) return;
-      cudaKernelNodeParams kp = {};
-      cudaGraphNode_t nu = nullptr, nc = nullptr, nk = nullptr;
-      void *ua[] = {(void *)&off_, (void *)&slots_, (void *)&deg_, (void *)&desc_, (void *)&counts_,
-                    (void *)&pdiv_in[h], (void *)&pcur[h], (void *)&pnext[h], (void *)&pdiv_out[h], (void *)&part,
-                    (void *)&damping_, (void *)&added_, (void *)&l1_};
-      kp.func = (void *)k_pr_units<kComp, T, sizeof(T) == 8>;
-      kp.gridDim = dim3(grid_u);
-      kp.blockDim = dim3(kPrBlock);
-      kp.sharedMemBytes = (unsigned)units_smem;
-      kp.kernelParams = ua;
-      cudaError_t x = cudaGraphAddKernelNode(&nu, gr, dep ? &dep : nullptr, dep ? 1 : 0, &kp);
-      kp.sharedMemBytes = 0;
-      if (x != cudaSuccess) return fail("pagerank units node", x);
-      cudaGraphNode_t prev = nu;
-      if (nheavy_) {
-        void *ca[] = {(void *)&heavy_, (void *)&cbase_, (void *)&nheavy_, (void *)&part, (void *)&deg_,
-                      (void *)&pcur[h], (void *)&pnext[h], (void *)&pdiv_out[h], (void *)&damping_, (void *)&added_,
-                      (void *)&l1_};
-        kp.func = (void *)k_pr_combine<kComp, T>;
-        kp.gridDim = dim3(grid_c);
-        kp.blockDim = dim3(256);
-        kp.kernelParams = ca;
-        x = cudaGraphAddKernelNode(&nc, gr, &prev, 1, &kp);
-        if (x != cudaSuccess) return fail("pagerank combine node", x);
-        prev = nc;
-      }
-      void *ka[] = {(void *)&l1_, (void *)&eps_, (void *)&maxit_, (void *)&loop_, (void *)(h ? &half1 : &half0),
-                    (void *)&h_if, (void *)&h_while};
-      kp.func = (void *)k_pr_check;
-      kp.gridDim = dim3(1);
-      kp.blockDim = dim3(32);
-      kp.kernelParams = ka;
-      x = cudaGraphAddKernelNode(&nk, gr, &prev, 1, &kp);
-      if (x != cudaSuccess) return fail("pagerank check node", x);
-      *lastn = nk;
+      cudaGraphNode_t prev = dep;
+      auto add = [&](void *func, int grid, int block, size_t smem, const char *what) {
+        if (rc != BYO_OK) return;
+        void *args[] = {&iter[h]};
+        cudaKernelNodeParams kp = {};
+        kp.func = func;
+        kp.gridDim = dim3(grid);
+        kp.blockDim = dim3(block);
+        kp.sharedMemBytes = (unsigned)smem;
+        kp.kernelParams = args;
+        cudaGraphNode_t node = nullptr;
+        const cudaError_t x = cudaGraphAddKernelNode(&node, gr, prev ? &prev : nullptr, prev ? 1 : 0, &kp);
+        if (x != cudaSuccess) return fail(what, x);
+        prev = node;
+      };
+      add((void *)k_pr_units<kComp, T, sizeof(T) == 8>, grid_u, kPrBlock, units_smem, "pagerank units node");
+      if (nheavy || kPrInPlace<T>) add((void *)k_pr_combine<kComp, T>, grid_c, 256, 0, "pagerank combine node");
+      if (!kPrInPlace<T>) add((void *)k_pr_finish<T>, grid_f, 256, 0, "pagerank finish node");
+      *lastn = prev;
     };
     cudaGraphNode_t k0 = nullptr, k1 = nullptr;
     add_iter(body, 0, nullptr, &k0);
@@ -1066,7 +1107,7 @@ static int pagerank_impl(byo_graph *g, double eps, uint32_t max_iters, double *d
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     BYO_TRY(rc);
-    ctx->launches += (uint64_t)(nheavy ? 3 : 2) * hs.iters - 1;  // kernels the graph ran
+    ctx->launches += (uint64_t)(1 + (nheavy || kPrInPlace<T>) + !kPrInPlace<T>) * hs.iters - 1;  // kernels the graph ran
     it = hs.iters;
     L1 = hs.l1;
     last = hs.last == 0 ? pb : pa;
