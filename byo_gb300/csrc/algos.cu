@@ -4,8 +4,8 @@
 // Connectivity (SimpleUnionAsync semantics, Connectivity.h:32-136): union-find
 // that always hooks the larger root under the smaller, so every root is the
 // minimum id of its component.  Edges are processed Afforest-style
-// (Sutton, Ben-Nun & Barak, IPDPS 2018): link the first kSample neighbours of
-// every vertex, compress, pick the most frequent root among sampled vertices,
+// (Sutton, Ben-Nun & Barak, IPDPS 2018): join every vertex to its first
+// kSample neighbours, compress, pick the most frequent root among sampled vertices,
 // then link the remaining edges of vertices outside that component only.  The
 // final labels do not depend on the order of links.
 //
@@ -31,23 +31,33 @@ constexpr int kSample = 2;  // cc_run's two rounds
 
 __device__ __forceinline__ uint32_t ld_parent(const uint32_t *p, uint32_t v) { return __ldcg(p + v); }
 
-// Root of v, with path halving when kHalve; parents only ever point to
-// smaller ids.
-template <bool kHalve = true>
+// Root of v; parents only ever point to smaller ids.  With kShorten the entries
+// read on the way are pointed at ancestors: v's own at the root, and the others
+// by path halving from the kPlainHops-th step on, which a chain needs.  Halving
+// at every step, all vertices of a large tree store into the few entries below
+// its root, and stores and loads of one word take turns at the L2, about one a ns
+// (second round of a uniform graph of 1 M vertices, average degree 1.6: 0.4 to
+// 1.6 ms halving at every step, the whole labelling 0.4 ms now).
+constexpr int kPlainHops = 16;
+template <bool kShorten = true>
 __device__ __forceinline__ uint32_t cc_find(uint32_t *p, uint32_t v) {
   uint32_t cur = ld_parent(p, v);
   if (cur == v) return v;
   uint32_t prev = v, next;
+  int hops = 0;
   while (cur > (next = ld_parent(p, cur))) {
-    if (kHalve) p[prev] = next;
+    if (kShorten && ++hops > kPlainHops) p[prev] = next;
     prev = cur;
     cur = next;
   }
+  if (kShorten && hops) p[v] = cur;
   return cur;
 }
 
-// Hook the larger root under the smaller until both share a root.
+// Hook the larger root under the smaller until both share a root.  Equal parents
+// end it before the roots, which are the words all threads read, are touched.
 __device__ __forceinline__ void cc_link(uint32_t *p, uint32_t u, uint32_t v) {
+  if (ld_parent(p, u) == ld_parent(p, v)) return;
   uint32_t ru = cc_find(p, u), rv = cc_find(p, v);
   while (ru != rv) {
     uint32_t hi = ru > rv ? ru : rv, lo = ru > rv ? rv : ru;
@@ -57,12 +67,6 @@ __device__ __forceinline__ void cc_link(uint32_t *p, uint32_t u, uint32_t v) {
     ru = cc_find(p, old);
     rv = cc_find(p, lo);
   }
-}
-
-__global__ void k_cc_init(uint32_t *p, uint64_t n) {
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n;
-       v += (uint64_t)gridDim.x * blockDim.x)
-    p[v] = (uint32_t)v;
 }
 
 // The round-th neighbour of v (kSentinel: it has fewer).
@@ -87,91 +91,137 @@ __device__ __forceinline__ uint32_t cc_sampled(const uint64_t *__restrict__ off,
   return kSentinel;
 }
 
-// Whether the first round left so many trees that the second hooks them first
-// (see cc_run): more than n / 256.
-__device__ __forceinline__ bool cc_many(const unsigned long long *trees, uint64_t n) { return *trees * 256 > n; }
-
-// Sampling round r (Afforest): every vertex links to its r-th neighbour (one
-// thread per vertex); a compress between rounds keeps the trees flat for the
-// next round's finds.  After hooking passes the rounds before r are linked
-// again, for the unions that a pass lost.
-__global__ void k_cc_sample(const uint64_t *__restrict__ off, const uint32_t *__restrict__ slots,
-                            uint32_t *p, uint64_t n, int round, const unsigned long long *trees) {
-  const int first = trees && cc_many(trees, n) ? 0 : round;
+// The first sampling round: every vertex under its first neighbour where that
+// is smaller, by one store.  The edges to larger ones are left to k_cc_sample.
+__global__ void k_cc_first(const uint64_t *__restrict__ off, const uint32_t *__restrict__ slots, uint32_t *p,
+                           uint64_t n) {
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n;
        v += (uint64_t)gridDim.x * blockDim.x)
-    for (int r = first; r <= round; r++) {
-      const uint32_t x = cc_sampled(off, slots, v, r);
-      if (x != kSentinel) cc_link(p, (uint32_t)v, x);
-    }
+    p[v] = min((uint32_t)v, cc_sampled(off, slots, v, 0));  // kSentinel (no neighbour) is larger than v
 }
 
-// Hooking passes over the edges to the round-th neighbours, a compress after
-// each: the larger parent of an edge's ends goes under the smaller, by one
-// atomicMin and no search.  A parent that two edges lower keeps the lower one,
-// so a pass can lose a union of a sampled edge; the linking that follows makes
-// it again, so the passes only prepare, and a grid barrier that gave up would
-// end them early and nothing else.  Parents stay below their children
-// throughout.  One cooperative kernel: where the passes are not wanted it costs
-// one launch, not six.
-constexpr int kCcHookBlock = 1024, kCcHooks = 3;
-__global__ void __launch_bounds__(kCcHookBlock, 2) k_cc_hook(const uint64_t *__restrict__ off,
-                                                             const uint32_t *__restrict__ slots, uint32_t *p,
-                                                             uint64_t n, int round, const unsigned long long *trees,
-                                                             GridBar *bar) {
-  if (!cc_many(trees, n)) return;
-  const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, nthr = (uint64_t)gridDim.x * blockDim.x;
-  for (int pass = 0; pass < kCcHooks; pass++) {
-    for (uint64_t v = tid; v < n; v += nthr) {
-      const uint32_t x = cc_sampled(off, slots, v, round);
-      if (x == kSentinel) continue;
-      const uint32_t pv = ld_parent(p, (uint32_t)v), px = ld_parent(p, x);
-      const uint32_t hi = max(pv, px), lo = min(pv, px);
-      if (hi != lo && ld_parent(p, hi) > lo) atomicMin(p + hi, lo);
-    }
-    if (!grid_sync(bar, gridDim.x)) return;
-    for (uint64_t v = tid; v < n; v += nthr) __stcg(p + v, cc_find<false>(p, (uint32_t)v));
-    if (!grid_sync(bar, gridDim.x)) return;
+// What the first round left: the edges to a larger first neighbour, then every
+// vertex to its second.
+__global__ void k_cc_sample(const uint64_t *__restrict__ off, const uint32_t *__restrict__ slots,
+                            uint32_t *p, uint64_t n) {
+  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n;
+       v += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t x = cc_sampled(off, slots, v, 0);
+    if (x == kSentinel) continue;
+    if (x > v) cc_link(p, (uint32_t)v, x);
+    const uint32_t y = cc_sampled(off, slots, v, 1);
+    if (y != kSentinel) cc_link(p, (uint32_t)v, y);
   }
 }
 
-// Every vertex to its root.  The finds do not halve: a halving store into
-// p[w] by a thread passing through w could land after w's own thread wrote
-// its root there, and leave a stale ancestor behind the last pass.
+// v to its root, by pointer jumping.  Only v's thread writes p[v]: a store into
+// another vertex's entry could land after its own thread wrote its root there,
+// and leave a stale ancestor behind the last pass.  Every step is stored, for
+// the first round may leave chains as long as the graph (a path, a grid's
+// columns), and the threads on a chain halve it together.
+__device__ __forceinline__ uint32_t cc_compress(uint32_t *p, uint32_t v) {
+  uint32_t cur = ld_parent(p, v), next = ld_parent(p, cur);
+  while (next != cur) {
+    __stcg(p + v, next);
+    cur = next;
+    next = ld_parent(p, cur);
+  }
+  return cur;
+}
 __global__ void k_cc_compress(uint32_t *p, uint64_t n) {
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n;
        v += (uint64_t)gridDim.x * blockDim.x)
-    p[v] = cc_find<false>(p, (uint32_t)v);
-}
-// Counts the trees of vertices with edges beside it.
-__global__ void __launch_bounds__(256) k_cc_compress_count(uint32_t *p, const uint32_t *__restrict__ deg, uint64_t n,
-                                                           unsigned long long *trees) {
-  __shared__ unsigned int sm[9];
-  unsigned int mine = 0;
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n;
-       v += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t r = cc_find<false>(p, (uint32_t)v);
-    p[v] = r;
-    mine += r == (uint32_t)v && deg[v];
-  }
-  mine = block_sum(mine, sm);
-  if (threadIdx.x == 0 && mine) atomicAdd(trees, (unsigned long long)mine);
+    cc_compress(p, (uint32_t)v);
 }
 
-// The vertices whose remaining edges must be linked: more than kSample
-// neighbours (the first kSample are linked by the sampling rounds) and a root
-// other than the giant component's, a thread per vertex, appended to `list`.
+// The vertex that probe i of a fixed hash draws.
+__device__ __forceinline__ uint32_t cc_probe(uint64_t n, uint32_t i) {
+  uint64_t z = 0x5EEDull + (uint64_t)(i + 1) * 0x9E3779B97F4A7C15ull;
+  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+  z ^= z >> 31;
+  return (uint32_t)(((z & 0xFFFFFFFFull) * n) >> 32);
+}
+// The most frequent root among a warp's (ties: the smallest).
+__device__ __forceinline__ uint32_t cc_mode(uint32_t root) {
+  const uint32_t same = __popc(__match_any_sync(kFull, root));
+  const uint32_t most = __reduce_max_sync(kFull, same);
+  return __reduce_min_sync(kFull, same == most ? root : kSentinel);
+}
+
+// The compress between the rounds, then hooking passes over the edges to the
+// second neighbours where they pay (see cc_run), a compress after each: the
+// larger parent of an edge's ends goes under the smaller, by one atomicMin and no
+// search.  At the start of a pass every parent is a root, and only roots get a
+// new one, so what was joined before stays joined.  A root that two edges
+// lower keeps the lower one, so a pass can lose the other edge's union; the
+// linking that follows makes it again, so the passes only prepare, and a grid
+// barrier that gave up would end them early and nothing else.  Parents stay
+// below their children throughout.  One cooperative kernel: where the passes are
+// not wanted it costs a barrier.
+__device__ __forceinline__ void cc_hook(uint32_t *p, uint32_t v, uint32_t x) {
+  const uint32_t pv = ld_parent(p, v), px = ld_parent(p, x);
+  const uint32_t hi = max(pv, px), lo = min(pv, px);
+  if (hi != lo && ld_parent(p, hi) > lo) atomicMin(p + hi, lo);
+}
+// Three passes: two are 10% faster on skewed graphs and up to 1.7x slower on uniform
+// ones (1 M vertices of degree 2: 417 against 240 us), four are 3 to 10% slower.
+constexpr int kCcHookBlock = 1024, kCcHooks = 3;
+constexpr uint64_t kCcHookLeast = 1 << 15;
+__global__ void __launch_bounds__(kCcHookBlock, 2) k_cc_hook(const uint64_t *__restrict__ off,
+                                                             const uint32_t *__restrict__ slots,
+                                                             const uint32_t *__restrict__ deg, uint32_t *p, uint64_t n,
+                                                             unsigned long long *trees, GridBar *bar) {
+  __shared__ unsigned int sm[kCcHookBlock / 32 + 1];
+  __shared__ uint32_t cand;
+  const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, nthr = (uint64_t)gridDim.x * blockDim.x;
+  unsigned int mine = 0;
+  for (uint64_t v = tid; v < n; v += nthr) mine += cc_compress(p, (uint32_t)v) == (uint32_t)v && deg[v];
+  mine = block_sum(mine, sm);
+  if (threadIdx.x == 0 && mine) atomicAdd(trees, (unsigned long long)mine);
+  if (!grid_sync(bar, gridDim.x)) return;
+  if (__ldcg(trees) * 256 <= n) return;
+  const uint32_t root = ld_parent(p, cc_probe(n, threadIdx.x));
+  if (threadIdx.x < 32) {
+    const uint32_t c = cc_mode(root);
+    if (threadIdx.x == 0) cand = c;
+  }
+  __syncthreads();
+  if (__syncthreads_count(root == cand) * 5 >= kCcHookBlock) return;
+  if (!grid_sync(bar, gridDim.x)) return;  // every block has probed
+  for (int pass = 0; pass < kCcHooks; pass++) {
+    for (uint64_t v = tid; v < n; v += nthr) {
+      const uint32_t x = cc_sampled(off, slots, v, 0);
+      if (x == kSentinel) continue;
+      if (x > v) cc_hook(p, (uint32_t)v, x);
+      const uint32_t y = cc_sampled(off, slots, v, 1);
+      if (y != kSentinel) cc_hook(p, (uint32_t)v, y);
+    }
+    if (!grid_sync(bar, gridDim.x)) return;
+    for (uint64_t v = tid; v < n; v += nthr) cc_compress(p, (uint32_t)v);
+    if (!grid_sync(bar, gridDim.x)) return;
+  }
+}
+
+// Every vertex to its root, and the list of those whose remaining edges must be
+// linked: more than kSample neighbours (the first kSample are linked by the
+// sampling rounds) and a root other than the giant component's, the most
+// frequent one among 32 probes (links are over, so every block finds the same).
 // A vertex inside the giant component is skipped entirely: each of its
 // neighbours outside it will link the edge from its own side, and roots only
 // merge, so a vertex found inside stays inside.
 __global__ void __launch_bounds__(256) k_cc_outside(const uint32_t *__restrict__ deg, uint32_t *p, uint64_t n,
-                                                    const uint32_t *__restrict__ giant_root, uint32_t *list,
-                                                    unsigned long long *count) {
-  const uint32_t giant = *giant_root;
+                                                    uint32_t *list, unsigned long long *count) {
+  __shared__ uint32_t giant;
+  if (threadIdx.x < 32) {
+    const uint32_t c = cc_mode(cc_find<false>(p, cc_probe(n, threadIdx.x)));
+    if (threadIdx.x == 0) giant = c;
+  }
+  __syncthreads();
   for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < n;
        base += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t v = base + lane_id();
-    const bool keep = v < n && deg[v] > (uint32_t)kSample && cc_find(p, (uint32_t)v) != giant;
+    const bool keep = v < n && cc_compress(p, (uint32_t)v) != giant && deg[v] > (uint32_t)kSample;
     const uint64_t at = warp_append(keep, count);
     if (keep) list[at] = (uint32_t)v;
   }
@@ -202,86 +252,44 @@ __global__ void __launch_bounds__(256) k_cc_finish(const uint64_t *__restrict__ 
   }
 }
 
-// The most frequent root among kCcProbe vertices drawn by a fixed hash (the
-// giant component, skipped by k_cc_finish): one CTA sorts the roots in
-// shared memory and keeps the longest run (ties: the smallest root).
-constexpr uint32_t kCcProbe = 1024;
-__global__ void __launch_bounds__(kCcProbe) k_cc_giant(const uint32_t *__restrict__ p, uint64_t n, uint64_t seed,
-                                                       uint32_t *giant) {
-  __shared__ uint32_t s[kCcProbe], st[kCcProbe];
-  __shared__ unsigned long long best;
-  const uint32_t t = threadIdx.x;
-  uint64_t z = seed + (uint64_t)(t + 1) * 0x9E3779B97F4A7C15ull;
-  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-  z ^= z >> 31;
-  s[t] = __ldcg(p + (uint32_t)(((z & 0xFFFFFFFFull) * n) >> 32));
-  if (t == 0) best = 0;
-  __syncthreads();
-  for (uint32_t k = 2; k <= kCcProbe; k <<= 1)
-    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      const uint32_t x = t ^ j;
-      if (x > t) {
-        const uint32_t a = s[t], b = s[x];
-        if ((a > b) == ((t & k) == 0)) {
-          s[t] = b;
-          s[x] = a;
-        }
-      }
-      __syncthreads();
-    }
-  st[t] = (t == 0 || s[t] != s[t - 1]) ? t : 0;  // start of t's run after a max-scan
-  __syncthreads();
-  for (uint32_t d = 1; d < kCcProbe; d <<= 1) {
-    const uint32_t v = t >= d ? st[t - d] : 0;
-    __syncthreads();
-    if (v > st[t]) st[t] = v;
-    __syncthreads();
-  }
-  if (t == kCcProbe - 1 || s[t] != s[t + 1])
-    atomicMax(&best, ((unsigned long long)(t - st[t] + 1) << 32) | (0xFFFFFFFFu - s[t]));
-  __syncthreads();
-  if (t == 0) *giant = 0xFFFFFFFFu - (uint32_t)best;
-}
-
 int cc_run(byo_graph *g, uint32_t *d_label) {
   byo_ctx *ctx = g->ctx;
   const uint64_t n = g->n;
   if (n == 0) return BYO_OK;
   uint32_t *p = d_label;
-  launch(ctx, k_cc_init, dim3(grid_for(ctx, n, 256)), dim3(256), 0, p, n);
   const dim3 grid_v(grid_for(ctx, n, 256));
-  uint32_t *giant = nullptr, *list = nullptr;
-  // [0] giant root, [2..3] count of listed vertices, [4..5] trees, then the barrier
-  BYO_TRY(ws(g, WS_MISC, 6 + sizeof(GridBar) / 4, &giant));
+  uint32_t *words = nullptr, *list = nullptr;
+  // [0..1] count of listed vertices, [2..3] trees, then the barrier
+  BYO_TRY(ws(g, WS_MISC, 4 + sizeof(GridBar) / 4, &words));
   BYO_TRY(ws(g, WS_FRONT_LIST_A, n, &list));
-  unsigned long long *count = reinterpret_cast<unsigned long long *>(giant + 2), *trees = count + 1;
-  GridBar *bar = reinterpret_cast<GridBar *>(giant + 6);
-  BYO_CU(ctx, cudaMemsetAsync(count, 0, 16 + sizeof(GridBar), ctx->stream));
+  unsigned long long *count = reinterpret_cast<unsigned long long *>(words), *trees = count + 1;
+  GridBar *bar = reinterpret_cast<GridBar *>(words + 4);
+  BYO_CU(ctx, cudaMemsetAsync(words, 0, 16 + sizeof(GridBar), ctx->stream));
   const uint64_t *off = g->d_off;
-  const uint32_t *slots = g->d_slots;
-  launch(ctx, k_cc_sample, grid_v, dim3(256), 0, off, slots, p, n, 0, (const unsigned long long *)nullptr);
-  launch(ctx, k_cc_compress_count, grid_v, dim3(256), 0, p, (const uint32_t *)g->d_deg, n, trees);
-  // Where no hubs gather the trees (a uniform graph of average degree d keeps
-  // one for every d + 1 vertices), the second round's links chase trees that
-  // grow under them: 0.9 to 3.5 ms for 3 M vertices of average degree 6.
-  // Hooking passes leave little to link: 0.67 ms in all.  A skewed graph (RMAT,
-  // Chung-Lu) is linked at once; below 2^18 vertices the links are quick.
-  const unsigned long long *decide = nullptr;
-  if (n >= (1u << 18)) {
-    decide = trees;
-    int per_sm = 0, round = 1;
+  const uint32_t *slots = g->d_slots, *deg = g->d_deg;
+  launch(ctx, k_cc_first, grid_v, dim3(256), 0, off, slots, p, n);
+  // Where no tree of the first round holds much, the second round's links wait for
+  // one another on a few growing trees, and hooking passes first leave them little
+  // to join: uniform graphs of average degree 16, 40000 / 300007 / 4 M vertices,
+  // 186 / 829 / 1529 us without and 76 / 149 / 969 with them; RMAT with permuted
+  // ids, 2^17 / 2^22 vertices, 116 / 1881 and 79 / 501.  Where hubs gather the
+  // trees (k_cc_hook sees one of n / 5 vertices or more) they made it 1.3 to 2x slower, so
+  // there the kernel only compresses, 4 to 8 us slower than k_cc_compress, which
+  // smaller graphs keep (uniform, 10007: 68 us either way).  Nor do they pay below
+  // an average degree of 1.6, where the trees stay small: 300007 vertices, degree
+  // 1.2 / 1.5 / 1.7: 82 / 162 / 140 us without, 116 / 132 / 132 with.
+  if (n < kCcHookLeast || 5 * g->m < 8 * n) {
+    launch(ctx, k_cc_compress, grid_v, dim3(256), 0, p, n);
+  } else {
+    int per_sm = 0;
     BYO_CU(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cc_hook, kCcHookBlock, 0));
-    void *args[] = {(void *)&off, (void *)&slots, (void *)&p, (void *)&n, (void *)&round, (void *)&decide, (void *)&bar};
+    void *args[] = {(void *)&off, (void *)&slots, (void *)&deg, (void *)&p, (void *)&n, (void *)&trees, (void *)&bar};
     BYO_CU(ctx, cudaLaunchCooperativeKernel((const void *)k_cc_hook, dim3(per_sm * ctx->num_sms), dim3(kCcHookBlock),
                                             args, 0, ctx->stream));
     ctx->launches++;
   }
-  launch(ctx, k_cc_sample, grid_v, dim3(256), 0, off, slots, p, n, 1, decide);
-  launch(ctx, k_cc_compress, grid_v, dim3(256), 0, p, n);
-  launch(ctx, k_cc_giant, dim3(1), dim3(kCcProbe), 0, (const uint32_t *)p, n, (uint64_t)0x5EEDull, giant);
-  launch(ctx, k_cc_outside, dim3(grid_for(ctx, n, 256)), dim3(256), 0, (const uint32_t *)g->d_deg, p, n,
-         (const uint32_t *)giant, list, count);
+  launch(ctx, k_cc_sample, grid_v, dim3(256), 0, off, slots, p, n);
+  launch(ctx, k_cc_outside, dim3(grid_for(ctx, n, 256)), dim3(256), 0, deg, p, n, list, count);
   const double avg = (double)g->m / (double)n;
   const int GS = avg >= 24 ? 16 : avg >= 8 ? 8 : 4;
   const int grid = grid_for(ctx, n * GS, 256, 16);
