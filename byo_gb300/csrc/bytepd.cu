@@ -17,14 +17,14 @@
 // GB300 holds a 2^32-edge CSR in 16 GB, so the graph is decoded once into the
 // library's CSR / PMA at load time rather than traversed compressed.
 //
-// Decode: one warp per block.  The warp reads 32 bytes at a time, a ballot of
-// the bytes with bit 7 clear marks where integers end, each ending lane
-// assembles its integer from up to 5 bytes by shuffles, and a warp scan of the
-// differences gives the neighbour ids, written with consecutive stores; the
-// next window starts after the last complete integer.  Encode: every edge's
+// Decode: a group of lanes or a warp per block, an aligned word a lane.  A lane
+// assembles the integers that end in its word from it and the word before (an
+// integer takes at most 5 bytes), ballots count the ends before it, and a scan of
+// the lanes' sums of differences gives the neighbour ids.  Encode: every edge's
 // byte length is independent (its difference to the source or the previous
-// neighbour), so a scan over the lengths places every edge's bytes and every
-// block header, and a thread per edge writes them.
+// neighbour); a block's are summed, a scan over the blocks places every block and
+// header, and the lengths are scanned again to write the bytes: one word a block
+// is kept, where a byte and an 8-byte place an edge were.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -38,8 +38,10 @@ namespace byo {
 
 constexpr uint32_t kBpdDefaultBlock = 1000;
 
-__device__ __forceinline__ uint32_t bpd_u32(const unsigned char *p) {
-  return (uint32_t)p[0] | (uint32_t)p[1] << 8 | (uint32_t)p[2] << 16 | (uint32_t)p[3] << 24;
+// The word at byte offset p of an aligned buffer whose last word is whole.
+__device__ __forceinline__ uint32_t bpd_u32(const uint32_t *__restrict__ words, uint64_t p) {
+  const uint32_t lo = words[p >> 2], hi = words[(p + 3) >> 2];
+  return __funnelshift_r(lo, hi, 8 * (uint32_t)(p & 3));
 }
 __device__ __forceinline__ void bpd_put_u32(unsigned char *p, uint32_t x) {
   p[0] = (unsigned char)x;
@@ -47,16 +49,9 @@ __device__ __forceinline__ void bpd_put_u32(unsigned char *p, uint32_t x) {
   p[2] = (unsigned char)(x >> 16);
   p[3] = (unsigned char)(x >> 24);
 }
-__host__ __device__ __forceinline__ uint32_t bpd_blocks(uint64_t d, uint32_t P) {
-  return d ? (uint32_t)(1 + (d - 1) / P) : 0;
-}
-__device__ __forceinline__ uint32_t varint_bytes(uint64_t a) {  // 7 bits a byte; 0 takes none
-  uint32_t k = 0;
-  while (a) {
-    k++;
-    a >>= 7;
-  }
-  return k;
+__device__ __forceinline__ uint32_t bpd_blocks(uint32_t d, uint32_t P) { return d ? 1 + (d - 1) / P : 0; }
+__device__ __forceinline__ uint32_t varint_bytes(uint32_t a) {  // 7 bits a byte; 0 takes none
+  return (uint32_t)(38 - __clz(a)) / 7;
 }
 
 // ---------------------------------------------------------------- decode
@@ -76,104 +71,178 @@ __global__ void k_bpd_block_owner(const uint32_t *__restrict__ deg, uint64_t n, 
   }
 }
 
-// bad: 1 malformed run
-__global__ void __launch_bounds__(256) k_bpd_decode(const unsigned char *__restrict__ bytes,
+// A block's integers: those after the first, k - done of them at byte offsets
+// [p, pend), go to out[done ..]; run is the neighbour before them.
+struct BpdRun {
+  uint64_t p, pend, out;
+  uint32_t k, done, run;
+};
+
+// Decodes one run in each group of GS lanes, an aligned word a lane, the groups
+// of the warp in step.  Ids are sums modulo 2^32: every difference is below 2^32,
+// so a sum that wraps, or a zero, shows as an id not above the one before.
+template <int GS>
+__device__ __forceinline__ bool bpd_decode_runs(BpdRun x, const uint32_t *__restrict__ words, uint32_t *nbrs) {
+  const uint32_t gl = lane_id() % GS, shift = lane_id() & ~(uint32_t)(GS - 1);
+  const uint32_t gmask = GS == 32 ? kFull : ((1u << (GS & 31)) - 1), below = (1u << gl) - 1;
+  uint32_t last = 0, last2 = 0;  // the two words before the window; 0: four ends
+  bool wrong = false;
+  for (uint64_t at = (x.p & ~3ull) + 4 * gl; __any_sync(kFull, x.done < x.k); at += 4 * GS) {
+    if (x.done < x.k && at - 4 * gl >= x.pend) {  // an integer running past the block
+      wrong = true;
+      x.k = x.done;
+    }
+    uint32_t w = 0x80808080u, in = 0;  // in: bit 7 of the block's bytes
+    if (x.done < x.k && at < x.pend) {
+      w = words[at >> 2];
+      in = 0x80808080u;
+      if (at + 4 > x.pend) in >>= 8 * (uint32_t)(at + 4 - x.pend);
+      if (at < x.p) {  // bytes before the run count as ends
+        const uint32_t skip = 8 * (uint32_t)(x.p - at);
+        w = w >> skip << skip;
+        in = in >> skip << skip;
+      }
+    }
+    uint32_t q = __shfl_up_sync(kFull, w, 1, GS);
+    if (gl == 0) q = last;
+    uint32_t before = __shfl_up_sync(kFull, q, 1, GS);
+    if (gl == 0) before = last2;
+    last2 = __shfl_sync(kFull, w, GS - 2, GS);
+    last = __shfl_sync(kFull, w, GS - 1, GS);
+    const uint32_t ends = ~w & in, need = x.k - x.done;
+    uint32_t rank = 0, total = 0;  // ends in the group's lanes before, in all
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t m = __ballot_sync(kFull, (ends >> (8 * j + 7)) & 1u) >> shift & gmask;
+      rank += __popc(m & below);
+      total += __popc(m);
+    }
+    // the bytes that q leaves open: its last ones without an end
+    const uint32_t open = (uint32_t)__clz(~q & 0x80808080u) >> 3;  // 4 if there is none
+    const uint32_t raw = open ? q >> (32 - 8 * open) : 0;
+    uint32_t acc = (raw & 0x7fu) | (raw >> 1 & 0x3f80u) | (raw >> 2 & 0x1fc000u) | (raw >> 3 & 0xfe00000u);
+    uint32_t sh = 7 * open, sum = 0, upto[4];
+    bool over = open == 4 && (before >> 31);  // the first end here ends more than 5 bytes
+    const uint32_t mine = rank < need ? need - rank : 0;
+    uint32_t seen = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t c = w >> (8 * j);
+      over |= sh > 28 || (sh == 28 && (c & 0x70u));  // a sixth byte, or 2^32 and more
+      acc |= sh <= 28 ? (c & 0x7fu) << sh : 0;
+      sh += 7;
+      if ((ends >> (8 * j + 7)) & 1u) {
+        wrong |= over && seen < mine;
+        sum += acc;
+        seen++;
+      }
+      if (!(c & 0x80u)) {  // an end, or a byte before the run
+        acc = 0;
+        sh = 0;
+        over = false;
+      }
+      upto[j] = sum;
+    }
+    uint32_t inc = sum;
+#pragma unroll
+    for (int o = 1; o < GS; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, inc, o, GS);
+      if (gl >= (uint32_t)o) inc += y;
+    }
+    uint32_t prev = x.run + inc - sum;
+    const uint32_t base = prev;
+    uint32_t *to = nbrs + x.out + x.done + rank;
+    seen = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (((ends >> (8 * j + 7)) & 1u) && seen < mine) {
+        const uint32_t id = base + upto[j];
+        wrong |= id <= prev || id == kSentinel;
+        to[seen++] = id;
+        prev = id;
+      }
+    x.run += __shfl_sync(kFull, inc, GS - 1, GS);
+    x.done += min(total, need);
+  }
+  return wrong;
+}
+
+// bad: 1 malformed run.  A warp takes kBpdTake blocks a step, a lane group each:
+// the group reads the headers and the first integer, and runs of up to kBpdShort
+// bytes are decoded side by side, the others by the whole warp in turn.  Bound by
+// instructions (70% of issue slots): a warp per block had most lanes idle, for half
+// the vertices of RMAT 2^20 (2^24 draws) have five neighbours or fewer.  649 -> 350
+// us there, uniform 2^20 of degree 32 / 4 and Chung-Lu of degree 6 570 -> 426,
+// 213 -> 142, 175 -> 116 (against a warp per block with the same words a lane
+// for the first, 4 blocks a step for the others).  4 / 8 / 16 blocks a step: 354 /
+// 318 / 315 at 64 bytes; 64 / 96 / 128 bytes at 8 blocks: 318 / 350 / 368, and 561 /
+// 426 / 404 on the uniform graph of degree 32.
+constexpr int kBpdTake = 8;
+constexpr uint64_t kBpdShort = 96;
+__global__ void __launch_bounds__(256) k_bpd_decode(const uint32_t *__restrict__ words,
                                                     const uint64_t *__restrict__ bo,
                                                     const uint32_t *__restrict__ deg,
                                                     const uint64_t *__restrict__ off,
                                                     const uint64_t *__restrict__ bfirst,
                                                     const uint32_t *__restrict__ blk_vertex, uint64_t nblocks,
                                                     uint32_t P, uint32_t *nbrs, unsigned int *bad) {
-  const unsigned lane = lane_id();
+  constexpr int GS = 32 / kBpdTake;
   const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t g = gw; g < nblocks; g += nw) {
-    const uint32_t v = blk_vertex[g];
-    const uint64_t i = g - bfirst[v];
-    const uint64_t d = deg[v], vb = bo[v], vlen = bo[v + 1] - vb;
-    const uint32_t nbk = bpd_blocks(d, P);
-    const unsigned char *base = bytes + vb;
-    const uint64_t hdr = 4 + 4ull * (nbk - 1);
-    if (vlen < hdr + 4 || bpd_u32(base) != d) {
-      if (lane == 0) atomicOr(bad, 1u);
-      continue;
-    }
-    const uint64_t pb = i == 0 ? hdr : bpd_u32(base + 4 + 4 * (i - 1));
-    const uint64_t pe = i + 1 == nbk ? vlen : bpd_u32(base + 4 + 4 * i);
-    if (pb + 4 > pe || pe > vlen) {
-      if (lane == 0) atomicOr(bad, 1u);
-      continue;
-    }
-    if (i + 1 < nbk && pe + 4 > vlen) {
-      if (lane == 0) atomicOr(bad, 1u);
-      continue;
-    }
-    const uint64_t e0 = bpd_u32(base + pb), e1 = i + 1 == nbk ? d : bpd_u32(base + pe);
-    if (e0 > e1 || e1 > d) {
-      if (lane == 0) atomicOr(bad, 1u);
-      continue;
-    }
-    const uint32_t k = (uint32_t)(e1 - e0);
-    uint32_t *out = nbrs + off[v] + e0;
-    uint64_t p = vb + pb + 4;
-    const uint64_t pend = vb + pe;
-    uint32_t done = 0;
-    int64_t run = 0;  // the last neighbour written
-    while (done < k) {
-      const bool in = p + lane < pend;
-      const uint32_t b = in ? bytes[p + lane] : 0x80u;
-      unsigned T = __ballot_sync(kFull, in && !(b & 0x80u));
-      // only the integers this block still needs
-      const uint32_t need = k - done;
-      while ((uint32_t)__popc(T) > need) T &= ~(1u << (31 - __clz(T)));
-      if (!T) {  // an integer running past the block, or longer than 32 bytes
-        if (lane == 0) atomicOr(bad, 1u);
-        break;
+  const uint32_t group = lane_id() / GS;
+  bool wrong = false;
+  // blocks in strides: neighbouring ones are as heavy as each other
+  for (uint64_t g0 = gw; g0 < nblocks; g0 += kBpdTake * nw) {
+    const uint64_t g = g0 + group * nw;
+    BpdRun x{0, 0, 0, 0, 0, 0};
+    if (g < nblocks) {
+      const uint32_t v = blk_vertex[g], d = deg[v], i = (uint32_t)(g - bfirst[v]), nbk = bpd_blocks(d, P);
+      const uint64_t vb = bo[v], vlen = bo[v + 1] - vb, hdr = 4ull * nbk;
+      bool ok = vlen >= hdr + 4 && bpd_u32(words, vb) == d;
+      uint64_t pb = 0, pe = 0, e0 = 0, e1 = 0;
+      if (ok) {
+        pb = i == 0 ? hdr : bpd_u32(words, vb + 4ull * i);
+        pe = i + 1 == nbk ? vlen : bpd_u32(words, vb + 4 + 4ull * i);
+        ok = pb + 4 <= pe && pe <= vlen && (i + 1 == nbk || pe + 4 <= vlen);
       }
-      const bool mine = (T >> lane) & 1u;
-      const unsigned below = T & lanemask_lt();
-      const uint32_t start = below ? 32 - __clz(below) : 0;
-      const bool first = done == 0 && start == 0;  // the block's first neighbour
-      uint64_t val = 0;
-      bool neg = false, over = false;
-#pragma unroll
-      for (int j = 0; j < 5; j++) {
-        const uint32_t src_lane = start + j < 32 ? start + j : 31;
-        const uint32_t bj = __shfl_sync(kFull, b, src_lane);
-        if (mine && start + j <= lane) {
-          if (first) {
-            if (j == 0) {
-              val = bj & 0x3fu;
-              neg = (bj & 0x40u) != 0;
-            } else {
-              val |= (uint64_t)(bj & 0x7fu) << (6 + 7 * (j - 1));
-            }
-          } else {
-            val |= (uint64_t)(bj & 0x7fu) << (7 * j);
-          }
+      if (ok) {
+        e0 = bpd_u32(words, vb + pb);
+        e1 = i + 1 == nbk ? d : bpd_u32(words, vb + pe);
+        ok = e0 <= e1 && e1 <= d;
+      }
+      if (ok && e1 > e0) {  // the first neighbour: signed, from the source
+        x = BpdRun{vb + pb + 4, vb + pe, off[v] + e0, (uint32_t)(e1 - e0), 1, 0};
+        const unsigned char *bytes = reinterpret_cast<const unsigned char *>(words);
+        uint32_t c = x.p < x.pend ? bytes[x.p++] : 0x80u, sh = 6;
+        uint64_t far = c & 0x3fu;
+        const bool neg = c & 0x40u;
+        while ((c & 0x80u) && x.p < x.pend && sh < 34) {
+          c = bytes[x.p++];
+          far |= (uint64_t)(c & 0x7fu) << sh;
+          sh += 7;
         }
+        const int64_t id = neg ? (int64_t)v - (int64_t)far : (int64_t)v + (int64_t)far;
+        ok = !(c & 0x80u) && id >= 0 && id < (int64_t)kSentinel;
+        x.run = (uint32_t)id;
+        if (ok && lane_id() % GS == 0) nbrs[x.out] = x.run;
       }
-      if (mine && lane - start >= 5) over = true;
-      // differences to the previous neighbour; the first is taken from the source
-      int64_t delta = 0;
-      if (mine) delta = first ? (neg ? (int64_t)v - (int64_t)val : (int64_t)v + (int64_t)val) - run : (int64_t)val;
-      int64_t inc = delta;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int64_t y = __shfl_up_sync(kFull, inc, o);
-        if (lane >= (unsigned)o) inc += y;
+      if (!ok) {
+        wrong = true;
+        x.k = x.done = 0;
       }
-      const int64_t id = run + inc;
-      if (mine) {
-        if (over || id < 0 || id > 0xFFFFFFFEll || (!first && val == 0)) atomicOr(bad, 1u);
-        out[done + __popc(below)] = (uint32_t)id;
-      }
-      if (__any_sync(kFull, mine && over)) break;
-      run += __shfl_sync(kFull, inc, 31);
-      done += __popc(T);
-      p += 32 - __clz(T);
+    }
+    const bool wide = x.k > x.done && x.pend - x.p > kBpdShort;
+    BpdRun narrow = x;
+    if (wide) narrow.k = narrow.done;
+    wrong |= bpd_decode_runs<GS>(narrow, words, nbrs);
+    for (uint32_t m = __ballot_sync(kFull, wide && lane_id() % GS == 0); m; m &= m - 1) {
+      const int o = __ffs(m) - 1;
+      const BpdRun y{__shfl_sync(kFull, x.p, o),  __shfl_sync(kFull, x.pend, o), __shfl_sync(kFull, x.out, o),
+                     __shfl_sync(kFull, x.k, o), __shfl_sync(kFull, x.done, o), __shfl_sync(kFull, x.run, o)};
+      wrong |= bpd_decode_runs<32>(y, words, nbrs);
     }
   }
+  if (wrong) atomicOr(bad, 1u);
 }
 
 // The blocks of P edges of every vertex: bfirst[v] (its first block, n+1
@@ -225,8 +294,8 @@ int bytepd_decode(byo_ctx *ctx, uint64_t n, const uint64_t *d_bo, const uint32_t
   if (e0 != cudaSuccess) rc = set_error(ctx, BYO_ENOMEM, "cudaMalloc", e0);
   if (rc == BYO_OK) {
     cudaMemsetAsync(bad, 0, 4, ctx->stream);
-    launch_t(ctx, "bytepd_decode", k_bpd_decode, dim3(grid_for(ctx, nblocks * 32, 256, 8)), dim3(256), 0, d_bytes,
-             d_bo, d_deg, (const uint64_t *)d_off, (const uint64_t *)bfirst, (const uint32_t *)owner, nblocks, P,
+    launch_t(ctx, "bytepd_decode", k_bpd_decode, dim3(grid_for(ctx, nblocks * 32, 256, 8)), dim3(256), 0,
+             reinterpret_cast<const uint32_t *>(d_bytes), d_bo, d_deg, (const uint64_t *)d_off, (const uint64_t *)bfirst, (const uint32_t *)owner, nblocks, P,
              d_nbrs, bad);
     unsigned int hb = 0;
     cudaMemcpyAsync(&hb, bad, 4, cudaMemcpyDeviceToHost, ctx->stream);
@@ -242,88 +311,180 @@ int bytepd_decode(byo_ctx *ctx, uint64_t n, const uint64_t *d_bo, const uint32_t
 
 // ---------------------------------------------------------------- encode
 
-// bytes of each edge's integer, a warp per block of P edges (hubs spread over
-// many warps); bad |= 1 for a list that is not strictly increasing
-__global__ void k_bpd_len(const uint64_t *__restrict__ off, const uint32_t *__restrict__ nbrs, uint32_t P,
-                          const uint64_t *__restrict__ bfirst, const uint32_t *__restrict__ blk_vertex,
-                          uint64_t nblocks, unsigned char *len, unsigned int *bad) {
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t g = gw; g < nblocks; g += nw) {
-    const uint32_t v = blk_vertex[g];
-    const uint64_t b = off[v], e = off[v + 1];
-    const uint64_t x0 = b + (g - bfirst[v]) * P, x1 = x0 + P < e ? x0 + P : e;
-    for (uint64_t x = x0 + lane_id(); x < x1; x += 32) {
-      if (x > b && nbrs[x] <= nbrs[x - 1]) atomicOr(bad, 1u);
-      uint32_t l;
-      if (x == x0) {
-        const int64_t diff = (int64_t)nbrs[x] - (int64_t)v;
-        l = 1 + varint_bytes((uint64_t)(diff < 0 ? -diff : diff) >> 6);
-      } else {
-        l = varint_bytes(nbrs[x] - nbrs[x - 1]);
-      }
-      len[x] = (unsigned char)l;
+// The edges [x0, x1) of a block of v; started: v has edges before them.
+struct BpdBlock {
+  uint64_t x0, x1;
+  uint32_t v;
+  bool started;
+};
+
+// GS of a block's edges from x - lane up: a lane's bytes (0 past the block), and
+// what goes into them.  `before` is the neighbour before the GS, of the same list.
+struct BpdEdge {
+  uint32_t bytes, mag, nbr;  // mag: the difference, for a block's first edge its size
+  bool neg, rising;
+};
+template <int GS>
+__device__ __forceinline__ BpdEdge bpd_edge(const BpdBlock &k, const uint32_t *__restrict__ nbrs, uint64_t x,
+                                            uint32_t before) {
+  BpdEdge r;
+  r.nbr = x < k.x1 ? nbrs[x] : 0;
+  uint32_t prev = __shfl_up_sync(kFull, r.nbr, 1, GS);
+  if (lane_id() % GS == 0) prev = before;
+  r.rising = x >= k.x1 || r.nbr > prev || (x == k.x0 && !k.started);
+  r.neg = false;
+  r.mag = 0;
+  r.bytes = 0;
+  if (x < k.x1) {
+    if (x == k.x0) {
+      r.neg = r.nbr < k.v;
+      r.mag = r.neg ? k.v - r.nbr : r.nbr - k.v;
+      r.bytes = 1 + varint_bytes(r.mag >> 6);
+    } else {
+      r.mag = r.nbr - prev;
+      r.bytes = varint_bytes(r.mag);
     }
+  }
+  return r;
+}
+
+// A block in each group of GS lanes, the groups of the warp in step: its integers'
+// bytes (in the group's first lane), and whether its neighbours increase.
+template <int GS>
+__device__ __forceinline__ uint64_t bpd_size_runs(const BpdBlock &k, const uint32_t *__restrict__ nbrs, bool &rising) {
+  uint32_t before = k.started && k.x0 < k.x1 ? nbrs[k.x0 - 1] : 0;
+  uint64_t mine = 0;
+  for (uint64_t xb = k.x0; __any_sync(kFull, xb < k.x1); xb += GS) {
+    const BpdEdge r = bpd_edge<GS>(k, nbrs, xb + lane_id() % GS, before);
+    before = __shfl_sync(kFull, r.nbr, GS - 1, GS);
+    mine += r.bytes;
+    rising = rising && r.rising;
+  }
+#pragma unroll
+  for (int o = GS / 2; o > 0; o >>= 1) mine += __shfl_down_sync(kFull, mine, o, GS);
+  return mine;
+}
+// The same for writing: the integers of a block go to bytes[at ..].
+template <int GS>
+__device__ __forceinline__ void bpd_write_runs(const BpdBlock &k, const uint32_t *__restrict__ nbrs, uint64_t at,
+                                               unsigned char *bytes) {
+  const uint32_t gl = lane_id() % GS;
+  unsigned char *to = bytes + at;
+  uint32_t before = 0;
+  for (uint64_t xb = k.x0; __any_sync(kFull, xb < k.x1); xb += GS) {
+    const BpdEdge r = bpd_edge<GS>(k, nbrs, xb + gl, before);
+    before = __shfl_sync(kFull, r.nbr, GS - 1, GS);
+    uint32_t inc = r.bytes;
+#pragma unroll
+    for (int o = 1; o < GS; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, inc, o, GS);
+      if (gl >= (uint32_t)o) inc += y;
+    }
+    unsigned char *w = to + (inc - r.bytes);
+    uint32_t a = r.mag, left = r.bytes;
+    if (xb + gl == k.x0 && left) {
+      *w++ = (unsigned char)((a & 0x3f) | (r.neg ? 0x40 : 0) | (left > 1 ? 0x80 : 0));
+      a >>= 6;
+      left--;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 5; j++)
+      if (j < left) w[j] = (unsigned char)((a >> (7 * j) & 0x7f) | (j + 1 < left ? 0x80 : 0));
+    to += __shfl_sync(kFull, inc, GS - 1, GS);
   }
 }
 
-struct InLen {
-  const unsigned char *len;
-  __device__ uint64_t operator()(uint64_t i) const { return len[i]; }
-};
-// bytes of vertex v: headers plus its edges' bytes (epos is their prefix)
+// Blocks of up to kBpdFew edges are encoded side by side, kBpdTake to a warp, as
+// k_bpd_decode's short runs are; the others by the whole warp in turn.  RMAT 2^20
+// (2^24 draws): sizes 213 -> 179 us, writing 344 -> 296; the uniform graph of degree 32
+// 250 -> 127 and 406 -> 359.
+constexpr uint64_t kBpdFew = 48;
+__device__ __forceinline__ BpdBlock bpd_block_from(const BpdBlock &k, int o) {
+  return BpdBlock{__shfl_sync(kFull, k.x0, o), __shfl_sync(kFull, k.x1, o), __shfl_sync(kFull, k.v, o),
+                  __shfl_sync(kFull, (int)k.started, o) != 0};
+}
+
+// Bytes of each block's integers; bad |= 1 for a list that is not strictly
+// increasing.
+__global__ void __launch_bounds__(256) k_bpd_size(const uint64_t *__restrict__ off, const uint32_t *__restrict__ nbrs,
+                                                  uint32_t P, const uint64_t *__restrict__ bfirst,
+                                                  const uint32_t *__restrict__ blk_vertex, uint64_t nblocks,
+                                                  uint64_t *size, unsigned int *bad) {
+  constexpr int GS = 32 / kBpdTake;
+  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  bool rising = true;
+  for (uint64_t g0 = gw; g0 < nblocks; g0 += kBpdTake * nw) {
+    const uint64_t g = g0 + lane_id() / GS * nw;
+    BpdBlock k{0, 0, 0, false};
+    if (g < nblocks) {
+      k.v = blk_vertex[g];
+      const uint64_t b = off[k.v], e = off[k.v + 1];
+      k.x0 = b + (g - bfirst[k.v]) * P;
+      k.x1 = k.x0 + P < e ? k.x0 + P : e;
+      k.started = k.x0 > b;
+    }
+    const bool wide = k.x1 - k.x0 > kBpdFew;
+    BpdBlock few = k;
+    if (wide) few.x1 = few.x0;
+    const uint64_t bytes = bpd_size_runs<GS>(few, nbrs, rising);
+    if (lane_id() % GS == 0 && g < nblocks && !wide) size[g] = bytes;
+    for (uint32_t m = __ballot_sync(kFull, wide && lane_id() % GS == 0); m; m &= m - 1) {
+      const int o = __ffs(m) - 1;
+      const uint64_t all = bpd_size_runs<32>(bpd_block_from(k, o), nbrs, rising);
+      if (lane_id() == 0) size[g0 + o / GS * nw] = all;
+    }
+  }
+  if (!rising) atomicOr(bad, 1u);
+}
+
+// bytes of vertex v: headers plus its blocks' bytes (bpos is their prefix)
 struct InVertexBytes {
-  const uint64_t *off, *epos;
+  const uint64_t *off, *bfirst, *bpos;
   uint32_t P;
   __device__ uint64_t operator()(uint64_t v) const {
     const uint64_t d = off[v + 1] - off[v];
     if (!d) return 0;
-    const uint32_t nb = bpd_blocks(d, P);
-    return 4 + 4ull * (nb - 1) + 4ull * nb + (epos[off[v + 1]] - epos[off[v]]);
+    const uint32_t nb = bpd_blocks((uint32_t)d, P);
+    return 4 + 4ull * (nb - 1) + 4ull * nb + (bpos[bfirst[v + 1]] - bpos[bfirst[v]]);
   }
 };
 
-// A warp per block of P edges writes its header (and, for block 0, the
-// vertex's degree) and its edges' bytes.
-__global__ void k_bpd_write(const uint64_t *__restrict__ off, const uint32_t *__restrict__ nbrs, uint32_t P,
-                            const uint64_t *__restrict__ bfirst, const uint32_t *__restrict__ blk_vertex,
-                            uint64_t nblocks, const uint64_t *__restrict__ epos, const uint64_t *__restrict__ bo,
-                            unsigned char *bytes) {
+// Every block's header (and, for block 0, the vertex's degree) and its edges'
+// bytes, placed by a scan of their lengths.
+__global__ void __launch_bounds__(256) k_bpd_write(const uint64_t *__restrict__ off, const uint32_t *__restrict__ nbrs,
+                                                   uint32_t P, const uint64_t *__restrict__ bfirst,
+                                                   const uint32_t *__restrict__ blk_vertex, uint64_t nblocks,
+                                                   const uint64_t *__restrict__ bpos, const uint64_t *__restrict__ bo,
+                                                   unsigned char *bytes) {
+  constexpr int GS = 32 / kBpdTake;
   const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t g = gw; g < nblocks; g += nw) {
-    const uint32_t v = blk_vertex[g];
-    const uint64_t b = off[v], e = off[v + 1], d = e - b, blk = g - bfirst[v];
-    const uint32_t nb = bpd_blocks(d, P);
-    unsigned char *base = bytes + bo[v];
-    const uint64_t hdr = 4 + 4ull * (nb - 1);
-    const uint64_t x0 = b + blk * P, x1 = x0 + P < e ? x0 + P : e;
-    const uint64_t q0 = hdr + 4 * (blk + 1) + (epos[x0] - epos[b]);  // the block's first edge byte
-    if (lane_id() == 0) {
-      if (blk == 0) bpd_put_u32(base, (uint32_t)d);
-      else bpd_put_u32(base + 4 + 4 * (blk - 1), (uint32_t)(q0 - 4));
-      bpd_put_u32(base + q0 - 4, (uint32_t)(blk * P));
+  for (uint64_t g0 = gw; g0 < nblocks; g0 += kBpdTake * nw) {
+    const uint64_t g = g0 + lane_id() / GS * nw;
+    BpdBlock k{0, 0, 0, false};
+    uint64_t at = 0;  // the block's first edge byte
+    if (g < nblocks) {
+      k.v = blk_vertex[g];
+      const uint64_t b = off[k.v], e = off[k.v + 1], blk = g - bfirst[k.v];
+      const uint32_t nb = bpd_blocks((uint32_t)(e - b), P);
+      const uint64_t base = bo[k.v], q0 = 4ull * nb + 4 * (blk + 1) + (bpos[g] - bpos[g - blk]);
+      k.x0 = b + blk * P;
+      k.x1 = k.x0 + P < e ? k.x0 + P : e;
+      at = base + q0;
+      if (lane_id() % GS == 0) {
+        if (blk == 0) bpd_put_u32(bytes + base, (uint32_t)(e - b));
+        else bpd_put_u32(bytes + base + 4 * blk, (uint32_t)(q0 - 4));
+        bpd_put_u32(bytes + at - 4, (uint32_t)(blk * P));
+      }
     }
-    for (uint64_t x = x0 + lane_id(); x < x1; x += 32) {
-      unsigned char *w = base + q0 + (epos[x] - epos[x0]);
-      uint64_t a;
-      if (x == x0) {
-        const int64_t diff = (int64_t)nbrs[x] - (int64_t)v;
-        a = (uint64_t)(diff < 0 ? -diff : diff);
-        unsigned char c = (unsigned char)(a & 0x3f);
-        if (diff < 0) c |= 0x40;
-        a >>= 6;
-        if (a) c |= 0x80;
-        *w++ = c;
-      } else {
-        a = nbrs[x] - nbrs[x - 1];
-      }
-      while (a) {
-        unsigned char y = (unsigned char)(a & 0x7f);
-        a >>= 7;
-        if (a) y |= 0x80;
-        *w++ = y;
-      }
+    const bool wide = k.x1 - k.x0 > kBpdFew;
+    BpdBlock few = k;
+    if (wide) few.x1 = few.x0;
+    bpd_write_runs<GS>(few, nbrs, at, bytes);
+    for (uint32_t m = __ballot_sync(kFull, wide && lane_id() % GS == 0); m; m &= m - 1) {
+      const int o = __ffs(m) - 1;
+      bpd_write_runs<32>(bpd_block_from(k, o), nbrs, __shfl_sync(kFull, at, o), bytes);
     }
   }
 }
@@ -335,17 +496,14 @@ int bytepd_encode(byo_graph *g, uint32_t P, uint64_t **d_bo_out, unsigned char *
   byo_ctx *ctx = g->ctx;
   byo_graph *t = nullptr;
   BYO_TRY(traversal_view(g, &t));
-  const uint64_t n = t->n, m = t->nslots;
+  const uint64_t n = t->n;
   *d_bo_out = nullptr;
   *d_bytes_out = nullptr;
-  unsigned char *len = nullptr;
-  uint64_t *epos = nullptr, *bo = nullptr;
+  uint64_t *size = nullptr, *bo = nullptr;
   unsigned char *bytes = nullptr;
   unsigned int *bad = nullptr;
   int rc = BYO_OK;
-  cudaError_t e = cudaMalloc(&len, m ? m : 1);
-  if (e == cudaSuccess) e = cudaMalloc(&epos, (m + 1) * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&bo, (n + 1) * 8);
+  cudaError_t e = cudaMalloc(&bo, (n + 1) * 8);
   if (e == cudaSuccess) e = cudaMalloc(&bad, 4);
   if (e != cudaSuccess) rc = set_error(ctx, BYO_ENOMEM, "cudaMalloc", e);
   uint64_t *h = nullptr;
@@ -354,15 +512,18 @@ int bytepd_encode(byo_graph *g, uint32_t P, uint64_t **d_bo_out, unsigned char *
   uint32_t *owner = nullptr;
   uint64_t nblocks = 0;
   if (rc == BYO_OK) rc = block_list(ctx, n, t->d_deg, P, &bfirst, &owner, &nblocks);
+  if (rc == BYO_OK && (e = cudaMalloc(&size, (2 * nblocks + 1) * 8)) != cudaSuccess)
+    rc = set_error(ctx, BYO_ENOMEM, "cudaMalloc", e);
+  uint64_t *bpos = size + nblocks;
   if (rc == BYO_OK) {
     cudaMemsetAsync(bad, 0, 4, ctx->stream);
-    launch(ctx, k_bpd_len, dim3(grid_for(ctx, nblocks * 32, 256, 8)), dim3(256), 0, (const uint64_t *)t->d_off,
-           (const uint32_t *)t->d_slots, P, (const uint64_t *)bfirst, (const uint32_t *)owner, nblocks, len, bad);
+    launch(ctx, k_bpd_size, dim3(grid_for(ctx, nblocks * 32, 256, 8)), dim3(256), 0, (const uint64_t *)t->d_off,
+           (const uint32_t *)t->d_slots, P, (const uint64_t *)bfirst, (const uint32_t *)owner, nblocks, size, bad);
     const uint64_t *tot = nullptr;
-    rc = scan_apply(ctx, m, InLen{len}, OutPrefix{epos}, &tot);
+    rc = scan_apply(ctx, nblocks, InU64{size}, OutPrefix{bpos}, &tot);
     if (rc == BYO_OK) {
-      cudaMemcpyAsync(epos + m, tot, 8, cudaMemcpyDeviceToDevice, ctx->stream);
-      rc = scan_apply(ctx, n, InVertexBytes{t->d_off, epos, P}, OutPrefix{bo}, &tot);
+      cudaMemcpyAsync(bpos + nblocks, tot, 8, cudaMemcpyDeviceToDevice, ctx->stream);
+      rc = scan_apply(ctx, n, InVertexBytes{t->d_off, bfirst, bpos, P}, OutPrefix{bo}, &tot);
     }
     if (rc == BYO_OK) {
       cudaMemcpyAsync(bo + n, tot, 8, cudaMemcpyDeviceToDevice, ctx->stream);
@@ -379,13 +540,12 @@ int bytepd_encode(byo_graph *g, uint32_t P, uint64_t **d_bo_out, unsigned char *
   if (rc == BYO_OK) {
     launch_t(ctx, "bytepd_encode", k_bpd_write, dim3(grid_for(ctx, nblocks * 32, 256, 8)), dim3(256), 0,
              (const uint64_t *)t->d_off, (const uint32_t *)t->d_slots, P, (const uint64_t *)bfirst,
-             (const uint32_t *)owner, nblocks, (const uint64_t *)epos, (const uint64_t *)bo, bytes);
+             (const uint32_t *)owner, nblocks, (const uint64_t *)bpos, (const uint64_t *)bo, bytes);
     rc = check_launch(ctx, "bytepd_encode");
   }
   if (bfirst) cudaFree(bfirst);
   if (owner) cudaFree(owner);
-  if (len) cudaFree(len);
-  if (epos) cudaFree(epos);
+  if (size) cudaFree(size);
   if (bad) cudaFree(bad);
   if (rc != BYO_OK) {
     if (bo) cudaFree(bo);
@@ -417,7 +577,7 @@ int graph_from_bytepd_host(byo_ctx *ctx, uint64_t n, const uint64_t *h_bo, const
   int rc = BYO_OK;
   cudaError_t e = cudaMalloc(&d_bo, (n + 1) * 8);
   if (e == cudaSuccess) e = cudaMalloc(&d_deg, (n ? n : 1) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&d_bytes, nbytes ? nbytes : 1);
+  if (e == cudaSuccess) e = cudaMalloc(&d_bytes, (nbytes / 4 + 1) * 4);  // whole words: k_bpd_decode
   if (e == cudaSuccess) e = cudaMalloc(&d_off, (n + 1) * 8);
   if (e == cudaSuccess) e = cudaMalloc(&d_nbrs, (m + 16) * 4);
   if (e != cudaSuccess) rc = set_error(ctx, BYO_ENOMEM, "cudaMalloc", e);
