@@ -15,7 +15,7 @@ def _keys(kind, count, n, rng):
     return (rng.integers(0, high, count).astype(np.uint64) << np.uint64(32)) | rng.integers(0, high, count).astype(np.uint64)
 
 
-@pytest.mark.parametrize("container", ["pma", "pcsr"])
+@pytest.mark.parametrize("container", ["pma", "pcsr", "vos"])
 @pytest.mark.parametrize("kind", ["random", "repeated", "equal", "falling"])
 @pytest.mark.parametrize("count", [1, 2, 31, 32, 33, 255, 257, 1024, 1025, 2047, 2049, 4095, 4096, 4097])
 def test_insert_and_remove(ctx, container, kind, count):
