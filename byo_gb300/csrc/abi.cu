@@ -622,7 +622,7 @@ int byo_pagerank(byo_graph *g, double eps, uint32_t max_iters, int precision, do
                  double *l1) {
   if (!g || !h_p) return BYO_EINVAL;
   double *d = nullptr;
-  BYO_TRY(ws(g, WS_TC_CNT, 2 * g->n + 2, (uint32_t **)&d));
+  BYO_TRY(host_out_buffer(g, g->n, &d));
   byo_graph *t = nullptr;
   BYO_TRY(traversal_view(g, &t));
   BYO_TRY(pagerank_run(t, eps, max_iters, precision, d, iters, l1));
