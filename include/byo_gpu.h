@@ -313,7 +313,9 @@ int byo_pagerank_delta_device(byo_graph *g, double eps, double local_eps, uint32
                               uint32_t *rounds, double *l1);
 
 /* Triangle counting, degree ordering
- * (benchmarks/TriangleCounting/ShunTangwongsan15/Triangle.h:167-204). */
+ * (benchmarks/TriangleCounting/ShunTangwongsan15/Triangle.h:167-204): the sum
+ * over the stored edges u -> v to a higher (degree, id) of the common such
+ * neighbours of u and v, also where edges are stored at one end only. */
 int byo_triangle_count(byo_graph *g, uint64_t *count);
 
 /* A stream of update batches (Batch_insert_runner's loop,
