@@ -49,6 +49,8 @@ constexpr uint32_t kTcMapBytes = 112 * 1024, kTcMidBytes = 28 * 1024;
 constexpr uint32_t kTcByteRanks = kTcMapBytes, kTcMidRanks = 8 * kTcMidBytes;
 constexpr uint32_t kTcHashMax = 256;           // longest N+ in a warp's hash set
 constexpr uint32_t kTcHash = 4 * kTcHashMax;   // its table's entries: load <= 1/4
+constexpr uint32_t kTcHashFew = 16;            // longest N+ in half a warp's
+constexpr uint32_t kTcHashSplit = 1 << 16;     // ranks from which they have a launch of their own
 constexpr uint32_t kTcChunk = 4096;            // u's of one map work unit
 
 // Which kernel counts v: a warp with a hash set when N+ is short and N- too
@@ -129,13 +131,34 @@ __global__ void __launch_bounds__(256) k_tc_rows(TcRows a, uint32_t v0) {
   const unsigned lane = lane_id();
   const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  // the next row's place is loaded during this one, and the vertex after that
+  auto vertex = [&](uint64_t t) { return t < a.n2 ? a.sorted[a.n - 1 - t] : 0; };
+  uint64_t key = vertex(v0 + gw), key1 = vertex(v0 + gw + nw);
+  uint64_t b = a.off[(uint32_t)key], e = a.off[(uint32_t)key + 1];
   unsigned long long mark = 0;
   for (uint64_t t = v0 + gw; t < a.n2; t += nw) {
     const uint32_t v = (uint32_t)t;
-    const uint64_t key = a.sorted[a.n - 1 - t];
-    const uint32_t y = (uint32_t)key;
-    const uint64_t b = a.off[y], e = a.off[y + 1], base = a.roff[t], end = base + tc_round4(key >> 32) + 4;
+    const uint64_t key2 = vertex(t + 2 * nw), b1 = a.off[(uint32_t)key1], e1 = a.off[(uint32_t)key1 + 1];
+    const uint64_t base = a.roff[t], end = base + tc_round4(key >> 32) + 4;
     uint32_t c = 0, ic = 0;
+    if (e - b <= 32) {
+      uint32_t x = b + lane < e ? a.slots[b + lane] : kSentinel;
+      x = x != kSentinel ? __ldg(a.rank + x) : kSentinel;
+      const bool out = x < v, in = x > v && x < a.n2;
+      const unsigned mo = __ballot_sync(kFull, out), mi = __ballot_sync(kFull, in);
+      const uint64_t m = tc_mark(a.seed, out ? v : x, out ? x : v);
+      if (out) {
+        st[__popc(mo & lanemask_lt())] = x;
+        mark += m;
+      }
+      if (in) {
+        a.nbr[end - 1 - __popc(mi & lanemask_lt())] = x;
+        mark -= m;
+      }
+      c = __popc(mo);
+      ic = __popc(mi);
+      b = e;
+    }
     for (uint64_t j0 = b; j0 < e; j0 += 128) {
       uint32_t x[4];
 #pragma unroll
@@ -158,12 +181,14 @@ __global__ void __launch_bounds__(256) k_tc_rows(TcRows a, uint32_t v0) {
     if (c <= 32) {
       uint32_t r = lane < c ? st[lane] : kSentinel;
 #pragma unroll
-      for (int size = 2; size <= 32; size <<= 1)
+      for (int size = 2; size <= 32; size <<= 1) {
+        if (size > 8 && c <= size / 2) break;  // (the lanes past c hold kSentinel)
 #pragma unroll
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
           const uint32_t o = __shfl_xor_sync(kFull, r, stride);
           r = (((lane & size) == 0) == ((lane & stride) == 0)) ? min(r, o) : max(r, o);
         }
+      }
       if (lane < tc_round4(c)) a.nbr[base + lane] = r;
     } else {
       const uint32_t P = 1u << (32 - __clz((int)(c - 1)));
@@ -189,6 +214,10 @@ __global__ void __launch_bounds__(256) k_tc_rows(TcRows a, uint32_t v0) {
       a.icnt[t] = ic;
     }
     __syncwarp();
+    key = key1;
+    key1 = key2;
+    b = b1;
+    e = e1;
   }
   mark = block_sum(mark, sm);
   if (threadIdx.x == 0 && mark) atomicAdd(a.differ, mark);
@@ -311,18 +340,18 @@ __global__ void __launch_bounds__(256) k_tc_units(const uint64_t *__restrict__ r
   }
 }
 
-// Lookups of N+(u) below v, 8 lanes to a list, 4 entries a lane: left at the
+// Lookups of N+(u) below v, G lanes to a list, 4 entries a lane: left at the
 // first entry >= v when the list is sorted (len <= sorted_cap).  in_set gives
 // 1 for an entry of N+(v) and 0 for any other (kSentinel too).  Called by whole
-// groups of 8.
-template <class Set>
+// groups of G.
+template <int G, class Set>
 __device__ __forceinline__ uint32_t tc_lookup(const uint32_t *__restrict__ nbr, uint64_t row, uint32_t v,
                                               uint32_t sorted_cap, const Set &in_set) {
-  const unsigned gm = 0xFFu << (lane_id() & 24);
+  const unsigned gm = ((1u << G) - 1) << (lane_id() & ~(G - 1));
   const uint32_t len = (uint32_t)row & 0xFFFFFF;
   const uint4 *list = reinterpret_cast<const uint4 *>(nbr + (row >> 24));
   uint32_t cnt = 0;
-  for (uint32_t k = 4 * (lane_id() & 7);; k += 32) {
+  for (uint32_t k = 4 * (lane_id() & (G - 1));; k += 4 * G) {
     uint4 x = make_uint4(kSentinel, kSentinel, kSentinel, kSentinel);
     if (k < len) x = __ldg(list + (k >> 2));
     cnt += in_set(x.x) + in_set(x.y) + in_set(x.z) + in_set(x.w);
@@ -334,7 +363,7 @@ __device__ __forceinline__ uint32_t tc_lookup(const uint32_t *__restrict__ nbr, 
 
 // Lookups of the lists of u = ulist[i], ulist[i + kStep], ... below i1, the next
 // list's place loaded while one is looked up.
-template <uint32_t kStep, class Set>
+template <int G, uint32_t kStep, class Set>
 __device__ __forceinline__ uint64_t tc_lookups(const uint32_t *__restrict__ nbr, const uint64_t *__restrict__ row,
                                                const uint32_t *__restrict__ ulist, uint32_t i, uint32_t i1, uint32_t v,
                                                uint32_t sorted_cap, const Set &set) {
@@ -343,7 +372,7 @@ __device__ __forceinline__ uint64_t tc_lookups(const uint32_t *__restrict__ nbr,
   while (i < i1) {
     i += kStep;
     const uint64_t nxt = i < i1 ? row[ulist[i]] : 0;
-    cnt += tc_lookup(nbr, cur, v, sorted_cap, set);
+    cnt += tc_lookup<G>(nbr, cur, v, sorted_cap, set);
     cur = nxt;
   }
   return cnt;
@@ -419,7 +448,7 @@ __global__ void __launch_bounds__(kBlock, 2048 / kBlock) k_tc_map(const uint32_t
         have = v <= room ? v : kSentinel;
         __syncthreads();
       }
-      cnt += tc_lookups<kBlock / 8>(nbr, row, ulist, i0 + (threadIdx.x >> 3), i1, v, sorted_cap, set);
+      cnt += tc_lookups<8, kBlock / 8>(nbr, row, ulist, i0 + (threadIdx.x >> 3), i1, v, sorted_cap, set);
       __syncthreads();
     }
   }
@@ -443,36 +472,49 @@ struct TcHash {
   }
 };
 
-// A warp per hashed v (tc_class): N+(v) in an open-addressing hash set of the
-// next power of two >= 4 |N+(v)| entries (a miss, most lookups, ends after ~1.2
-// probes), four u's at a time.
+// L lanes to each hashed v (tc_class): N+(v) in an open-addressing hash set of
+// the next power of two >= 4 |N+(v)| entries (a miss, most lookups, ends after ~1.2
+// probes).  Up to 16 entries half a warp, 8 u's at a time with two lanes to a list
+// (the lists of the u's are then as short); more a warp, 4 u's at a time.  Bound by
+// instructions and the chain row -> lists -> rows of the u's -> their lists: uniform
+// 10^6 vertices of degree 16 492 us with the halves, 665 by warps alone.  Below
+// kTcHashSplit ranks a second launch costs what it saves (Chung-Lu 10^4 240 us a count
+// with it, 226 without; uniform 10^5 346 with, 360 without).
+template <int L>
 __global__ void __launch_bounds__(256) k_tc_hash(const uint32_t *__restrict__ nbr, const uint64_t *__restrict__ row,
                                                  const uint64_t *__restrict__ in, const uint32_t *__restrict__ icnt,
-                                                 uint32_t n2, uint32_t sorted_cap, unsigned long long *total) {
-  __shared__ uint32_t tabs[8][kTcHash];
+                                                 uint32_t n2, uint32_t few, uint32_t sorted_cap,
+                                                 unsigned long long *total) {
+  constexpr uint32_t kTable = L == 32 ? kTcHash : 4 * kTcHashFew;
+  constexpr int G = L == 32 ? 8 : 2;
+  __shared__ uint32_t tabs[256 / L][kTable];
   __shared__ unsigned long long sm[9];
-  const unsigned lane = lane_id();
-  uint32_t *tab = tabs[threadIdx.x >> 5];
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const unsigned lane = threadIdx.x % L, mask = L == 32 ? kFull : ((1u << (L & 31)) - 1) << (lane_id() & ~(L - 1));
+  uint32_t *tab = tabs[threadIdx.x / L];
+  const uint64_t g0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / L;
+  const uint64_t ng = ((uint64_t)gridDim.x * blockDim.x) / L;
   uint64_t cnt = 0;
-  for (uint64_t t = gw; t < n2; t += nw) {
-    const uint64_t own = row[t];
-    const uint32_t nout = (uint32_t)own & 0xFFFFFF, ni = icnt[t];
-    if (tc_class((uint32_t)t, nout, ni) != kTcHashed) continue;
-    const uint32_t lg = max(6, 32 - __clz((int)(4 * nout - 1))), size = 1u << lg;
-    for (uint32_t i = lane; i < size; i += 32) tab[i] = kSentinel;
-    __syncwarp();
-    for (uint32_t i = lane; i < nout; i += 32) {
-      const uint32_t x = nbr[(own >> 24) + i];
-      uint32_t h = (x * 0x9E3779B1u) >> (32 - lg);
-      while (atomicCAS(tab + h, kSentinel, x) != kSentinel) h = (h + 1) & (size - 1);
+  uint64_t own = g0 < n2 ? row[g0] : 0;  // loaded ahead: most v's are passed over
+  uint32_t ni = g0 < n2 ? icnt[g0] : 0;
+  for (uint64_t t = g0; t < n2; t += ng) {
+    const uint64_t own1 = t + ng < n2 ? row[t + ng] : 0;
+    const uint32_t ni1 = t + ng < n2 ? icnt[t + ng] : 0, nout = (uint32_t)own & 0xFFFFFF;
+    if (tc_class((uint32_t)t, nout, ni) == kTcHashed && (nout <= few) == (L < 32)) {
+      const uint32_t lg = max(6, 32 - __clz((int)(4 * nout - 1))), size = 1u << lg;
+      for (uint32_t i = lane; i < size; i += L) tab[i] = kSentinel;
+      __syncwarp(mask);
+      for (uint32_t i = lane; i < nout; i += L) {
+        const uint32_t x = nbr[(own >> 24) + i];
+        uint32_t h = (x * 0x9E3779B1u) >> (32 - lg);
+        while (atomicCAS(tab + h, kSentinel, x) != kSentinel) h = (h + 1) & (size - 1);
+      }
+      __syncwarp(mask);
+      const TcHash set{tab, size - 1, 32 - lg, (uint32_t)t};
+      cnt += tc_lookups<G, L / G>(nbr, row, nbr + in[t], lane / G, ni, (uint32_t)t, sorted_cap, set);
+      __syncwarp(mask);
     }
-    __syncwarp();
-    const TcHash set{tab, size - 1, 32 - lg, (uint32_t)t};
-    const uint32_t *ulist = nbr + in[t];
-    cnt += tc_lookups<4>(nbr, row, ulist, lane >> 3, ni, (uint32_t)t, sorted_cap, set);
-    __syncwarp();
+    own = own1;
+    ni = ni1;
   }
   const unsigned long long tot = block_sum((unsigned long long)cnt, sm);
   if (threadIdx.x == 0 && tot) atomicAdd(total, tot);
@@ -545,8 +587,12 @@ int tc_run(byo_graph *g, uint64_t *count) {
     BYO_TRY(count_class(kTcByte, k_tc_map<TcBytes, 1024>, 1024, kTcMapBytes));
     BYO_TRY(count_class(kTcMid, k_tc_map<TcBits, 256>, 256, kTcMidBytes));
     if (n2 > kTcMidRanks) BYO_TRY(count_class(kTcFar, k_tc_map<TcBits, 1024>, 1024, kTcMapBytes));
-    launch_t(ctx, "tc_intersect", k_tc_hash, dim3(grid_for(ctx, (uint64_t)n2 * 32, 256)), dim3(256), 0,
-             (const uint32_t *)nbr, (const uint64_t *)row, (const uint64_t *)in, (const uint32_t *)icnt, n2, cap, d);
+    const uint32_t few = n2 < kTcHashSplit ? 0 : kTcHashFew;
+    launch_t(ctx, "tc_intersect", k_tc_hash<32>, dim3(grid_for(ctx, (uint64_t)n2 * 32, 256)), dim3(256), 0,
+             (const uint32_t *)nbr, (const uint64_t *)row, (const uint64_t *)in, (const uint32_t *)icnt, n2, few, cap, d);
+    if (few)
+      launch_t(ctx, "tc_intersect", k_tc_hash<16>, dim3(grid_for(ctx, (uint64_t)n2 * 16, 256)), dim3(256), 0,
+               (const uint32_t *)nbr, (const uint64_t *)row, (const uint64_t *)in, (const uint32_t *)icnt, n2, few, cap, d);
     BYO_CU(ctx, cudaMemcpyAsync(h, d, 80, cudaMemcpyDeviceToHost, ctx->stream));
     BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
     return BYO_OK;
