@@ -564,6 +564,12 @@ byo_tuning effective_tuning(const byo_graph *g) {
   return t;
 }
 
+// Shared memory of k_pull: what it has besides the staged words (its lists; the
+// compiler's figure), the most words (check_tuning), and the bytes of words up to
+// which two CTAs share an SM's 228 KB.
+constexpr int kPullStatic = 25408, kPullMaxStage = 49152;
+constexpr int kPullPairBytes = (228 * 1024) / 2 - 1024 - kPullStatic;
+
 int check_tuning(byo_ctx *ctx, const byo_tuning *t) {
   const char *bad = nullptr;
   if (t->push_group && t->push_group != 4 && t->push_group != 8 && t->push_group != 16 && t->push_group != 32)
@@ -578,7 +584,7 @@ int check_tuning(byo_ctx *ctx, const byo_tuning *t) {
     bad = "ms_heavy_deg must be <= 65536";
   else if (t->ms_hub_deg && (t->ms_hub_deg < 32 || t->ms_hub_deg > (1u << 20)))
     bad = "ms_hub_deg must be in [32, 2^20]";
-  else if (t->pull_stage_words && (t->pull_stage_words < 256 || t->pull_stage_words > 49152))
+  else if (t->pull_stage_words && (t->pull_stage_words < 256 || t->pull_stage_words > kPullMaxStage))
     bad = "pull_stage_words must be in [256, 49152]";
   else if (t->tc_stage && (t->tc_stage < 512 || t->tc_stage > 49152))
     bad = "tc_stage must be in [512, 49152]";
@@ -647,16 +653,6 @@ int ensure_bits(byo_graph *g, Frontier &f) {
   return check_launch(ctx, "ensure_bits");
 }
 
-static int pull_smem_ok(int bytes) {
-  static int configured = 0;  // (24 KB more are static)
-  if (configured < bytes) {
-    if (cudaFuncSetAttribute(k_pull, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
-      return 0;
-    configured = bytes;
-  }
-  return 1;
-}
-
 int edge_map_round(byo_graph *g, TravState &st, Frontier &in, Frontier &out, int mode,
                    const EngineTuning &tune, bool run_policy) {
   byo_ctx *ctx = g->ctx;
@@ -674,16 +670,14 @@ int edge_map_round(byo_graph *g, TravState &st, Frontier &in, Frontier &out, int
   const uint64_t lvl = (uint64_t)st.round << 32;
   if (mode == MODE_PULL) {
     BYO_TRY(ensure_bits(g, in));
-    int stage = tune.pull_stage_words;
-    int smem = stage * 4;
-    if (!pull_smem_ok(smem)) {
-      if (stage > 12 * 1024) stage = 12 * 1024;
-      smem = stage * 4;
-    }
+    const int stage = tune.pull_stage_words, smem = stage * 4;
+    // the attribute is the device's, and other contexts set it too: always the
+    // same value, and no record of having set it
+    BYO_CU(ctx, cudaFuncSetAttribute(k_pull, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kPullMaxStage));
     const uint64_t W = (g->n + 31) / 32;
     int block = 1024;
     int grid = (int)((W + 31) / 32);
-    int maxg = ctx->num_sms * (smem > 100 * 1024 ? 1 : 2);
+    int maxg = ctx->num_sms * (smem > kPullPairBytes ? 1 : 2);
     if (grid > maxg) grid = maxg;
     if (grid < 1) grid = 1;
     launch_t(ctx, "bfs_pull", k_pull, dim3(grid), dim3(block), (size_t)smem, (const uint64_t *)g->d_off,
