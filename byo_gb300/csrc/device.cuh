@@ -85,8 +85,9 @@ __device__ __forceinline__ uint64_t warp_append(bool pred, unsigned long long *c
 // to the list 64 or more at a time, with one add to its counter.  An add of
 // every warp to one address takes the L2 ~1 ns each, however few items it is for.
 constexpr uint32_t kWarpListCap = 96;
+template <uint32_t kCap = kWarpListCap>
 struct WarpList {
-  uint32_t *buf;  // [kWarpListCap], the warp's own
+  uint32_t *buf;  // [kCap], the warp's own
   uint32_t count = 0;
   __device__ __forceinline__ void flush(uint32_t *list, unsigned long long *counter) {
     if (!count) return;
@@ -103,7 +104,7 @@ struct WarpList {
     if (has) buf[count + __popc(m & lanemask_lt())] = x;
     count += __popc(m);
     __syncwarp();
-    if (count > kWarpListCap - 32) flush(list, counter);
+    if (count > kCap - 32) flush(list, counter);
   }
 };
 

@@ -48,7 +48,7 @@ __device__ __forceinline__ void hist_flush(unsigned long long *sh, RoundStats *s
 __device__ __forceinline__ void emit_next(bool emit, uint32_t v, uint32_t *out_list,
                                           uint32_t *out_bits, RoundStats *st,
                                           const uint32_t *__restrict__ deg, uint64_t &dsum,
-                                          WarpList &wl, unsigned long long *sh) {
+                                          WarpList<> &wl, unsigned long long *sh) {
   wl.add(emit, v, out_list, &st->count);
   uint32_t d = 0;
   if (emit) {
@@ -59,42 +59,47 @@ __device__ __forceinline__ void emit_next(bool emit, uint32_t v, uint32_t *out_l
   hist_warp_add(sh, emit, d);
 }
 
-// The end of a list that a block's warps append to: what they still hold, by one
-// add a block.  Warps that see a word or two each come here with all they found,
-// and an add a warp was a quarter of a pull round at 2^18 vertices (three rounds:
-// 47 -> 36 us) and 8% of a BFS on a uniform graph of 2 M (337 -> 308).
-// Block-collective; s is the list's own.
-__device__ __forceinline__ void block_flush(WarpList &wl, uint32_t *list, unsigned long long *counter,
-                                            unsigned long long *s /* [32] */) {
-  const uint32_t w = threadIdx.x >> 5, lane = lane_id(), nw = blockDim.x >> 5;
-  if (lane == 0) s[w] = wl.count;
-  __syncthreads();
-  if (w == 0) {
-    const uint32_t c = lane < nw ? (uint32_t)s[lane] : 0, upto = warp_inclusive_scan(c);
-    const uint32_t total = __shfl_sync(kFull, upto, 31);
-    unsigned long long base = 0;
-    if (lane == 0 && total) base = atomicAdd(counter, (unsigned long long)total);
-    base = __shfl_sync(kFull, base, 0);
-    if (lane < nw) s[lane] = base + upto - c;
-  }
-  __syncthreads();
-  for (uint32_t i = lane; i < wl.count; i += 32) list[s[w] + i] = wl.buf[i];
-  wl.count = 0;
+// Where the parts of a block's warps go in a list that they append to: s[w] holds
+// the counts, then the places, by one add to the list's counter.  By one warp.
+__device__ __forceinline__ void list_places(unsigned long long *s /* [32] */, uint32_t nw, unsigned long long *counter) {
+  const uint32_t lane = lane_id(), c = lane < nw ? (uint32_t)s[lane] : 0, upto = warp_inclusive_scan(c);
+  const uint32_t total = __shfl_sync(kFull, upto, 31);
+  unsigned long long base = 0;
+  if (lane == 0 && total) base = atomicAdd(counter, (unsigned long long)total);
+  base = __shfl_sync(kFull, base, 0);
+  if (lane < nw) s[lane] = base + upto - c;
 }
 
-// A visiting kernel's end: its part of the next frontier and of the round's
-// statistics.  Block-collective.
-__device__ __forceinline__ void round_flush(WarpList &wl, uint32_t *out_list, RoundStats *st, uint64_t dsum,
-                                            unsigned long long *sh) {
-  __shared__ unsigned long long s_at[32], s_sum[32];
+// A visiting kernel's end: what its warps still hold of the next frontier (and of
+// a second list, the pull's deferred vertices), by one add a block, and its part of
+// the round's statistics, a warp each, so that the adds are waited for together.
+// Warps that see a word or two each come here with all they found, and an add a
+// warp was a quarter of a pull round at 2^18 vertices (three rounds: 47 -> 36 us) and
+// 8% of a BFS on a uniform graph of 2 M (337 -> 308).  Block-collective, 4 warps or more.
+template <uint32_t kCap>
+__device__ __forceinline__ void round_flush(WarpList<kCap> &wl, uint32_t *out_list, RoundStats *st, uint64_t dsum,
+                                            unsigned long long *sh, WarpList<kCap> *wd = nullptr,
+                                            uint32_t *defer = nullptr) {
+  __shared__ unsigned long long s_at[32], s_defer[32], s_sum[32];
+  const uint32_t w = threadIdx.x >> 5, lane = lane_id(), nw = blockDim.x >> 5;
   dsum = warp_sum(dsum);
-  if (lane_id() == 0) s_sum[threadIdx.x >> 5] = dsum;
-  block_flush(wl, out_list, &st->count, s_at);
-  if (threadIdx.x < 32) {
-    dsum = warp_sum(threadIdx.x < blockDim.x >> 5 ? s_sum[threadIdx.x] : 0ull);
-    if (threadIdx.x == 0 && dsum) atomicAdd(&st->outdeg, (unsigned long long)dsum);
+  if (lane == 0) {
+    s_at[w] = wl.count;
+    if (wd) s_defer[w] = wd->count;
+    s_sum[w] = dsum;
   }
-  if (threadIdx.x < 8 && sh[threadIdx.x]) atomicAdd(&st->hist[threadIdx.x], sh[threadIdx.x]);
+  __syncthreads();
+  if (w == 0) list_places(s_at, nw, &st->count);
+  if (w == 1 && wd) list_places(s_defer, nw, &st->ndefer);
+  if (w == 2) {
+    dsum = warp_sum(lane < nw ? s_sum[lane] : 0ull);
+    if (lane == 0 && dsum) atomicAdd(&st->outdeg, (unsigned long long)dsum);
+  }
+  if (w == 3 && lane < 8 && sh[lane]) atomicAdd(&st->hist[lane], sh[lane]);
+  __syncthreads();
+  for (uint32_t i = lane; i < wl.count; i += 32) out_list[s_at[w] + i] = wl.buf[i];
+  if (wd)
+    for (uint32_t i = lane; i < wd->count; i += 32) defer[s_defer[w] + i] = wd->buf[i];
 }
 
 // Visits edge u->v for BFS_F: cond(v) = not visited before this round;
@@ -113,7 +118,7 @@ template <int R>
 __device__ __forceinline__ void visit_emit(const uint32_t (&u)[R], const uint32_t (&v)[R], uint64_t lvl, uint64_t *lp,
                                            const uint32_t *__restrict__ visited, uint32_t *out_list,
                                            uint32_t *out_bits, RoundStats *st, const uint32_t *__restrict__ deg,
-                                           uint64_t &dsum, WarpList &wl, unsigned long long *sh) {
+                                           uint64_t &dsum, WarpList<> &wl, unsigned long long *sh) {
   bool open[R];
 #pragma unroll
   for (int q = 0; q < R; q++) open[q] = v[q] != kSentinel && !test_bit_cg(visited, v[q]);
@@ -141,7 +146,7 @@ __global__ void __launch_bounds__(256) k_push(const uint64_t *__restrict__ off,
   __shared__ unsigned long long s_hist[8];
   hist_init(s_hist);
   __shared__ uint32_t s_list[8][kWarpListCap];
-  WarpList wl{s_list[threadIdx.x >> 5]};
+  WarpList<> wl{s_list[threadIdx.x >> 5]};
   constexpr int PER_WARP = 32 / GS;
   const unsigned lane = lane_id(), g = lane / GS, gl = lane % GS;
   const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -195,7 +200,7 @@ __global__ void __launch_bounds__(256) k_push_dense_fwd(const uint64_t *__restri
   __shared__ unsigned long long s_hist[8];
   hist_init(s_hist);
   __shared__ uint32_t s_list[8][kWarpListCap];
-  WarpList wl{s_list[threadIdx.x >> 5]};
+  WarpList<> wl{s_list[threadIdx.x >> 5]};
   const unsigned lane = lane_id();
   const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -233,7 +238,7 @@ __global__ void __launch_bounds__(256) k_push_hubs(const uint64_t *__restrict__ 
   __shared__ unsigned long long s_hist[8];
   hist_init(s_hist);
   __shared__ uint32_t s_list[8][kWarpListCap];
-  WarpList wl{s_list[threadIdx.x >> 5]};
+  WarpList<> wl{s_list[threadIdx.x >> 5]};
   const uint64_t nd = *(volatile unsigned long long *)&st->ndefer, nh = nd < hub_cap ? nd : hub_cap;
   uint64_t dsum = 0;
   for (uint64_t h = blockIdx.x; h < nh; h += gridDim.x) {
@@ -289,7 +294,7 @@ __global__ void __launch_bounds__(256) k_push_blocked(const uint64_t *__restrict
   __shared__ unsigned long long s_hist[8];
   hist_init(s_hist);
   __shared__ uint32_t s_list[8][kWarpListCap];
-  WarpList wl{s_list[threadIdx.x >> 5]};
+  WarpList<> wl{s_list[threadIdx.x >> 5]};
   __shared__ uint64_t s_slot[kBlockedStage];  // slot of a rank: rank + s_slot
   __shared__ uint32_t s_pre[kBlockedStage], s_u[kBlockedStage];
   __shared__ uint64_t s_lo, s_hi;
@@ -362,7 +367,12 @@ __device__ __forceinline__ bool in_frontier(const uint32_t *s_bits, int stage_wo
 
 // A thread per unvisited vertex.  Found and deferred vertices go out through
 // WarpLists: an add to the two counters from every warp held the first dense
-// round at RMAT 2^22 up by a third (138 us, 96 now).
+// round at RMAT 2^22 up by a third (138 us, 96 now).  The lists take what L1 has
+// for the ids and bits of a round that finds few: BFS by pulls alone on a uniform
+// graph of 10^6 vertices and degree 16 594 us with room for 96 entries, words and
+// slots counted in 64 bits (which spills) and an add after the other at the end;
+// 584 without those two; 560 with room for 64 as well (without lists 557).
+constexpr uint32_t kPullListCap = 64;
 __global__ void __launch_bounds__(1024, 2) k_pull(const uint64_t *__restrict__ off,
                                                const uint32_t *__restrict__ slots,
                                                const uint32_t *__restrict__ deg,
@@ -373,33 +383,31 @@ __global__ void __launch_bounds__(1024, 2) k_pull(const uint64_t *__restrict__ o
                                                int cap, int stage_words) {
   extern __shared__ uint32_t s_bits[];
   __shared__ unsigned long long s_hist[8];
-  __shared__ uint32_t s_list[2][32][kWarpListCap];
-  __shared__ unsigned long long s_defer[32];
-  WarpList wl{s_list[0][threadIdx.x >> 5]}, wdefer{s_list[1][threadIdx.x >> 5]};
+  __shared__ uint32_t s_list[2][32][kPullListCap];
+  WarpList<kPullListCap> wl{s_list[0][threadIdx.x >> 5]}, wdefer{s_list[1][threadIdx.x >> 5]};
   for (int i = threadIdx.x; i < stage_words; i += blockDim.x) s_bits[i] = Fbits[i];
   if (threadIdx.x < 8) s_hist[threadIdx.x] = 0;
   __syncthreads();
-  const uint64_t W = (n + 31) >> 5;
+  const uint32_t W = (uint32_t)((n + 31) >> 5);
   const unsigned lane = lane_id();
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint32_t nw = gridDim.x * (blockDim.x >> 5);
   uint64_t dsum = 0;
-  for (uint64_t w = gw; w < W; w += nw) {
+  for (uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < W; w += nw) {
     const uint32_t vword = visited[w];
     if (vword == kFull) continue;
-    const uint64_t v = w * 32 + lane;
-    bool active = v < n && !((vword >> lane) & 1u);
+    const uint32_t v = w * 32 + lane;
     bool found = false, deferred = false;
     uint32_t parent = 0;
-    if (active) {
-      const uint64_t b = off[v], e = off[v + 1];
-      const uint64_t lim = (e - b > (uint64_t)cap) ? b + cap : e;
+    if (v < n && !((vword >> lane) & 1u)) {
+      const uint64_t b = off[v], len = off[v + 1] - b;
+      const uint32_t *const ids = slots + b;
+      const uint32_t lim = (uint32_t)min(len, (uint64_t)cap);
       // eight neighbours at a time: their ids, then their frontier bits, are
       // loaded together; the first hit in slot order is the parent
-      for (uint64_t j0 = b; j0 < lim && !found; j0 += 8) {
+      for (uint32_t j0 = 0; j0 < lim && !found; j0 += 8) {
         uint32_t u[8];
 #pragma unroll
-        for (int q = 0; q < 8; q++) u[q] = j0 + q < lim ? slots[j0 + q] : kSentinel;
+        for (int q = 0; q < 8; q++) u[q] = j0 + q < lim ? ids[j0 + q] : kSentinel;
         bool h[8];
 #pragma unroll
         for (int q = 0; q < 8; q++) h[q] = u[q] != kSentinel && in_frontier(s_bits, stage_words, Fbits, u[q]);
@@ -410,25 +418,24 @@ __global__ void __launch_bounds__(1024, 2) k_pull(const uint64_t *__restrict__ o
             parent = u[q];
           }
       }
-      deferred = !found && lim < e;
+      deferred = !found && len > lim;
     }
     if (found) lp[v] = lvl | parent;
     const unsigned fb = __ballot_sync(kFull, found);
     if (lane == 0 && fb) {
       out_bits[w] = fb;
-      visited[w] = vword | fb;
+      visited[w] |= fb;
     }
-    wl.add(found, (uint32_t)v, out_list, &st->count);
+    wl.add(found, v, out_list, &st->count);
     uint32_t d = 0;
     if (found) {
       d = deg[v];
       dsum += d;
     }
     hist_warp_add(s_hist, found, d);
-    wdefer.add(deferred, (uint32_t)v, defer, &st->ndefer);
+    wdefer.add(deferred, v, defer, &st->ndefer);
   }
-  block_flush(wdefer, defer, &st->ndefer, s_defer);
-  round_flush(wl, out_list, st, dsum, s_hist);
+  round_flush(wl, out_list, st, dsum, s_hist, &wdefer, defer);
 }
 
 // Warp per deferred vertex: 32 neighbours per step, ballot, lowest lane wins.
@@ -567,7 +574,7 @@ byo_tuning effective_tuning(const byo_graph *g) {
 // Shared memory of k_pull: what it has besides the staged words (its lists; the
 // compiler's figure), the most words (check_tuning), and the bytes of words up to
 // which two CTAs share an SM's 228 KB.
-constexpr int kPullStatic = 25408, kPullMaxStage = 49152;
+constexpr int kPullStatic = 17216, kPullMaxStage = 49152;
 constexpr int kPullPairBytes = (228 * 1024) / 2 - 1024 - kPullStatic;
 
 int check_tuning(byo_ctx *ctx, const byo_tuning *t) {
