@@ -20,8 +20,10 @@
 //     per vertex) to those in the frontier, leaving at the first !cond.  A
 //     lane takes a vertex of <= kDenseShort slots; longer runs go to a warp
 //     that loads and tests 32 neighbours at a time and applies the updates in
-//     order.  PR_F and PR_Delta_F have kernels of their own (k_em_sum_lanes,
-//     k_em_sum_warps, k_em_sum_ctas), whose sums are bit-identical to a sequential scan.
+//     order.  PR_F and PR_Delta_F have kernels of their own, whose sums are
+//     bit-identical to a sequential scan: a round on its own a lane, a warp or a CTA
+//     a vertex (k_em_sum_direct, k_em_sum_warps, k_em_sum_ctas), rounds of one
+//     plan lanes by class (k_em_sum_lanes).
 //   dense forward (edgeMapDenseForward, gbbs/edge_map_data.h:180-247): the
 //     frontier's members push with updateAtomic, as the sparse round does.
 // The output is a list and a bitmap kept together (the engine's Frontier).
@@ -231,21 +233,32 @@ __global__ void __launch_bounds__(256) k_em_pull_long(const uint64_t *__restrict
 // run of the first ones, a warp one of the next to last and a CTA one of the
 // last.  A warp's FP64 addition takes the pipe 19 cycles however many lanes
 // add, so 32 runs of one length cost a warp what a single one would.
-constexpr uint32_t kSumLaneMax = 128;
+constexpr uint32_t kSumLaneMax = 128, kSumWarpMax = 4096, kSumShort = 32;
 constexpr int kSumLanes = 11, kSumWarp = kSumLanes, kSumCta = kSumLanes + 1, kSumClasses = kSumLanes + 2;
 __device__ __forceinline__ int sum_class(uint64_t len) {  // 1..2, 3..4, ..8, ..12, ..16, 24, 32, .. kSumLaneMax
   if (len <= 8) return len <= 2 ? 0 : len <= 4 ? 1 : 2;
-  if (len > kSumLaneMax) return len <= 4096 ? kSumWarp : kSumCta;
+  if (len > kSumLaneMax) return len <= kSumWarpMax ? kSumWarp : kSumCta;
   const int lg = 31 - __clz((int)len - 1);  // 8 < len: len - 1 in [2^lg, 2^(lg+1))
   return 3 + 2 * (lg - 3) + (int)(((len - 1) >> (lg - 1)) & 1);
 }
 struct SumPlan {
   uint32_t *list;             // the classes' vertices, one class after the other
   unsigned long long *count;  // [kSumClasses] vertices, [kSumClasses] cursors, [1] next warp run
+  // of a round on its own: the warps' runs only, and the CTAs' from the end of n;
+  // listed already, or by k_em_sum_direct
+  bool direct, listed;
+  __device__ const uint32_t *runs(int c, uint64_t n) const {
+    if (direct) return c == kSumCta ? list + (n - count[c]) : list;
+    uint64_t start = 0;
+    for (int k = 0; k < c; k++) start += count[k];
+    return list + start;
+  }
 };
+constexpr int kSumCounts = 2 * kSumClasses + 1;
 
 // What one neighbour adds: a value computed once per vertex (PR_F: n divisions
-// instead of one an edge; FP64 division is slow here), or read in place.
+// instead of one an edge; FP64 division is slow here), or read in place, or
+// (kDivide, small views) divided there.
 struct SumArgs {
   const uint64_t *off;
   const uint32_t *slots;
@@ -259,7 +272,11 @@ struct SumArgs {
   uint32_t *out_list, *out_bits;
   unsigned long long *cnt;  // members out, their degrees
   SumPlan plan;
-  __device__ double value(uint32_t u) const { return __ldg(val + (uint64_t)u * stride + at); }
+  template <bool kDivide = false>
+  __device__ double value(uint32_t u) const {
+    const double x = __ldg(val + (uint64_t)u * stride + at);
+    return kDivide ? __ddiv_rn(x, (double)deg[u]) : x;
+  }
   __device__ bool member(uint32_t u) const { return u != kSentinel && (!fb || test_bit(fb, u)); }
 };
 
@@ -308,7 +325,8 @@ __global__ void k_em_values(PrF f, uint64_t n, double *val) {
     val[v] = f.value((uint32_t)v);
 }
 
-// A lane per run: 32 runs of one class, kWin terms of each at a time gathered
+// A planned round, which is one of every vertex without output.  A lane per run:
+// 32 runs of one class, kWin terms of each at a time gathered
 // by the whole warp (the runs' ids in pieces of kWin) and staged, then added
 // by the runs' lanes.  Bound by a warp's own chain (64 cycles an FP64 addition,
 // two gathers a window), so longer runs than kSumLaneMax are composed by a warp
@@ -317,7 +335,7 @@ __global__ void k_em_values(PrF f, uint64_t n, double *val) {
 // of up to 64 slots with a division for every term took 270.
 template <int kWin>
 __device__ __forceinline__ void sum_lane_runs(const SumArgs &a, const uint32_t *list, uint64_t runs, uint64_t group,
-                                              double *stage, uint64_t &outdeg) {
+                                              double *stage) {
   const unsigned lane = lane_id();
   const uint64_t i = group * 32 + lane;
   uint32_t v = 0;
@@ -329,7 +347,7 @@ __device__ __forceinline__ void sum_lane_runs(const SumArgs &a, const uint32_t *
     len = (uint32_t)(a.off[v + 1] - b);
   }
   double acc = len ? a.sum[v] : 0.0;
-  bool any = false, zero = false;
+  bool any = false;
   for (uint32_t w0 = 0; __ballot_sync(kFull, w0 < len); w0 += kWin) {
     uint32_t u[kWin];
 #pragma unroll
@@ -343,7 +361,7 @@ __device__ __forceinline__ void sum_lane_runs(const SumArgs &a, const uint32_t *
     uint32_t has = 0;
 #pragma unroll
     for (int q = 0; q < kWin; q++) {
-      const bool in = a.member(u[q]);
+      const bool in = u[q] != kSentinel;
       if (in) stage[(q * (32 / kWin) + lane / kWin) * (kWin + 1) + lane % kWin] = a.value(u[q]);
       const unsigned m = __ballot_sync(kFull, in);
       if ((int)(lane / (32 / kWin)) == q) has = m >> (lane % (32 / kWin) * kWin);
@@ -353,14 +371,10 @@ __device__ __forceinline__ void sum_lane_runs(const SumArgs &a, const uint32_t *
     any |= has != 0;
 #pragma unroll
     for (int k = 0; k < kWin; k++)
-      if ((has >> k) & 1u) {
-        zero |= seq_zero(acc);
-        acc = __dadd_rn(acc, stage[lane * (kWin + 1) + k]);
-      }
+      if ((has >> k) & 1u) acc = __dadd_rn(acc, stage[lane * (kWin + 1) + k]);
     __syncwarp();
   }
   if (any) a.sum[v] = acc;
-  emit_out(a.output && (a.zero_marks ? zero : any), v, a.out_list, a.out_bits, a.deg, a.cnt, outdeg);
 }
 
 __global__ void __launch_bounds__(256) k_em_sum_lanes(SumArgs a) {
@@ -382,7 +396,6 @@ __global__ void __launch_bounds__(256) k_em_sum_lanes(SumArgs a) {
   const uint64_t gw = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   double *st = stage[threadIdx.x >> 5];
-  uint64_t outdeg = 0;
   int c = kSumLanes - 1;  // the longest runs first
   for (uint64_t t = gw; t < first[kSumLanes]; t += nw) {
     const uint64_t g = first[kSumLanes] - 1 - t;
@@ -390,11 +403,147 @@ __global__ void __launch_bounds__(256) k_em_sum_lanes(SumArgs a) {
     const uint32_t *list = a.plan.list + vert[c];
     const uint64_t runs = vert[c + 1] - vert[c];
     if (c <= 1)
-      sum_lane_runs<4>(a, list, runs, g - first[c], st, outdeg);
+      sum_lane_runs<4>(a, list, runs, g - first[c], st);
     else if (c == 2)
-      sum_lane_runs<8>(a, list, runs, g - first[c], st, outdeg);
+      sum_lane_runs<8>(a, list, runs, g - first[c], st);
     else
-      sum_lane_runs<16>(a, list, runs, g - first[c], st, outdeg);
+      sum_lane_runs<16>(a, list, runs, g - first[c], st);
+  }
+}
+
+// One run by a warp, 256 neighbours a step; stage: seq_at<8>(256) values, mask: 8 words.
+template <bool kDivide>
+__device__ __forceinline__ SeqSum sum_warp_run(const SumArgs &a, uint32_t v, uint64_t b, uint64_t e, double *stage,
+                                               uint32_t *mask) {
+  const unsigned lane = lane_id();
+  SeqSum s{a.sum[v], false, false};
+  for (uint64_t j0 = b; j0 < e; j0 += 256) {
+    uint32_t u[8];
+#pragma unroll
+    for (int r = 0; r < 8; r++) u[r] = j0 + r * 32 + lane < e ? a.slots[j0 + r * 32 + lane] : kSentinel;
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+      const bool has = a.member(u[r]);
+      const unsigned word = __ballot_sync(kFull, has);
+      stage[seq_at<8>(r * 32 + lane)] = has ? a.value<kDivide>(u[r]) : 0.0;
+      if (lane == 0) mask[r] = word;
+    }
+    __syncwarp();
+    double x[8];
+#pragma unroll
+    for (int r = 0; r < 8; r++) x[r] = stage[seq_at<8>(8 * lane + r)];
+    seq_warp(s, x, reinterpret_cast<const unsigned char *>(mask)[lane]);
+    __syncwarp();
+  }
+  if (lane == 0 && s.any) a.sum[v] = s.acc;
+  return s;
+}
+
+// A round on its own: planning it costs two passes and the launches of three
+// streams, 12 us of a 40 us call on small graphs, and on uniform graphs there is
+// little to tell apart (10^6 vertices of degree 16, a fiftieth of them in the
+// frontier: 326 us a call by a plan, 237 so).  A lane per vertex of up to kSumShort
+// slots, 8 of them in flight; the longer runs are listed for the kernels below.  At
+// 16 / 24 / 32 / 64 slots: that graph 524 / 252 / 237 / 236 us a call, Chung-Lu of 10^5
+// vertices 93 / 93 / 93 / 98, RMAT 2^20 / 2^24 draws 521 / 515 / 517 / 540.
+// On a view with gaps (kGaps) a short list may have a leaf's gap in it: up to
+// kGapRun slots its warp takes it at once.
+constexpr uint32_t kGapRun = 512;
+template <bool kGaps>
+__device__ __forceinline__ bool sum_gap(const SumArgs &a, uint64_t v, uint64_t len) {
+  return kGaps && len > kSumShort && len <= kGapRun && a.deg[v] <= kSumShort;
+}
+
+// The long runs listed by a pass of its own: from kSumBeside slots on, so that
+// their kernels run beside the lanes (a call 517 -> 506 us on RMAT 2^20 / 2^24 draws,
+// 389 -> 334 on Chung-Lu of 10^6 vertices and degree 16).
+template <bool kGaps>
+__global__ void __launch_bounds__(1024) k_sum_long(SumArgs a) {
+  __shared__ unsigned int cnt[2];
+  __shared__ unsigned long long at[2];
+  for (uint64_t base = blockIdx.x * 4096ull; base < a.n; base += gridDim.x * 4096ull) {
+    if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
+    __syncthreads();
+    int c[4];
+    unsigned int slot[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const uint64_t v = base + q * 1024 + threadIdx.x, len = v < a.n ? a.off[v + 1] - a.off[v] : 0;
+      c[q] = len > kSumWarpMax ? 1 : len > kSumShort && !sum_gap<kGaps>(a, v, len) ? 0 : -1;
+      slot[q] = c[q] >= 0 ? atomicAdd(cnt + c[q], 1u) : 0;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 && cnt[threadIdx.x])
+      at[threadIdx.x] = atomicAdd(a.plan.count + kSumWarp + threadIdx.x, (unsigned long long)cnt[threadIdx.x]);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (c[q] >= 0) {
+        const uint64_t i = at[c[q]] + slot[q];
+        a.plan.list[c[q] ? a.n - 1 - i : i] = (uint32_t)(base + q * 1024 + threadIdx.x);
+      }
+    __syncthreads();
+  }
+}
+
+template <bool kDivide, bool kGaps>
+__global__ void __launch_bounds__(256, kDivide || kGaps ? 4 : 5) k_em_sum_direct(SumArgs a) {
+  __shared__ double stages[kGaps ? 8 : 1][kGaps ? seq_at<8>(256) : 1];
+  __shared__ uint32_t masks[8][8];
+  const uint64_t W = (a.n + 31) / 32;
+  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  uint64_t outdeg = 0;
+  for (uint64_t w = gw; w < W; w += nw) {
+    const uint64_t v = w * 32 + lane_id();
+    const uint64_t b = v < a.n ? a.off[v] : 0, len = v < a.n ? a.off[v + 1] - b : 0;
+    bool any = false, zero = false;
+    if (len && len <= kSumShort) {
+      const uint32_t *const ids = a.slots + b;
+      double acc = 0.0;
+      for (uint32_t j = 0; j < len; j += 8) {
+        uint32_t u[8];
+        double x[8];
+        unsigned in = 0;
+#pragma unroll
+        for (int q = 0; q < 8; q++) u[q] = j + q < len ? ids[j + q] : kSentinel;
+#pragma unroll
+        for (int q = 0; q < 8; q++) in |= a.member(u[q]) ? 1u << q : 0u;
+        if (!in) continue;
+#pragma unroll
+        for (int q = 0; q < 8; q++) x[q] = (in >> q) & 1u ? a.value<kDivide>(u[q]) : 0.0;
+        if (!any) acc = a.sum[v];
+        any = true;
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+          if ((in >> q) & 1u) {
+            zero |= seq_zero(acc);
+            acc = __dadd_rn(acc, x[q]);
+          }
+      }
+      if (any) a.sum[v] = acc;
+    }
+    const bool gap = sum_gap<kGaps>(a, v, len);
+    if constexpr (kGaps) {
+      for (unsigned m = __ballot_sync(kFull, gap); m; m &= m - 1) {
+        const int k = __ffs(m) - 1;
+        const uint64_t from = __shfl_sync(kFull, b, k);
+        const SeqSum s = sum_warp_run<kDivide>(a, (uint32_t)(w * 32 + k), from, from + __shfl_sync(kFull, len, k),
+                                               stages[threadIdx.x >> 5], masks[threadIdx.x >> 5]);
+        if ((int)lane_id() == k) {
+          any = s.any;
+          zero = s.zero;
+        }
+      }
+    }
+    if (!a.plan.listed) {
+      const bool cta = len > kSumWarpMax, warp = len > kSumShort && !gap && !cta;
+      const uint64_t at = warp_append(warp, a.plan.count + kSumWarp);
+      if (warp) a.plan.list[at] = (uint32_t)v;
+      const uint64_t back = warp_append(cta, a.plan.count + kSumCta);
+      if (cta) a.plan.list[a.n - 1 - back] = (uint32_t)v;
+    }
+    emit_out(a.output && (a.zero_marks ? zero : any), (uint32_t)v, a.out_list, a.out_bits, a.deg, a.cnt, outdeg);
   }
   outdeg = warp_sum(outdeg);
   if (lane_id() == 0 && outdeg) atomicAdd(a.cnt + 1, (unsigned long long)outdeg);
@@ -405,15 +554,14 @@ __global__ void __launch_bounds__(256) k_em_sum_lanes(SumArgs a) {
 // neighbours: 172 us a round; one lane adding a warp's values in turn took 20 ms.
 // 64 registers instead of 128 spill the loads in flight: 364 us.
 constexpr int kSumBlock = 512, kSumTerms = 8;
+template <bool kDivide>
 __global__ void __launch_bounds__(kSumBlock, 1) k_em_sum_ctas(SumArgs a) {
   __shared__ double stage[seq_at<kSumTerms>(kSumTerms * kSumBlock)];
   __shared__ uint32_t mask[kSumTerms * kSumBlock / 32];
   __shared__ uint64_t sums[2][32];
   __shared__ SeqSum shared;
   const SeqBlockMem mem{stage, mask, sums, &shared};
-  uint64_t start = 0;
-  for (int c = 0; c < kSumCta; c++) start += a.plan.count[c];
-  const uint32_t *runs = a.plan.list + start;
+  const uint32_t *runs = a.plan.runs(kSumCta, a.n);
   const uint64_t ncta = a.plan.count[kSumCta];
   uint64_t outdeg = 0;
   unsigned turn = 0;
@@ -439,7 +587,7 @@ __global__ void __launch_bounds__(kSumBlock, 1) k_em_sum_ctas(SumArgs a) {
       for (int r = 0; r < kSumTerms; r++) {
         const bool has = a.member(u[r]);
         in |= (has ? 1u : 0u) << r;
-        x[r] = has ? a.value(u[r]) : 0.0;
+        x[r] = has ? a.value<kDivide>(u[r]) : 0.0;
       }
     };
     constexpr uint64_t kStep = kSumTerms * kSumBlock;
@@ -464,18 +612,16 @@ __global__ void __launch_bounds__(kSumBlock, 1) k_em_sum_ctas(SumArgs a) {
   if (threadIdx.x == 0 && outdeg) atomicAdd(a.cnt + 1, (unsigned long long)outdeg);
 }
 
-// Runs of kSumLaneMax to 4096 slots, a warp each, 256 neighbours a step: 108 us a
-// round on the same graph (with the lanes' and the CTAs' runs side by side).
+// Runs of kSumLaneMax to 4096 slots, a warp each: 108 us a round on the same graph
+// (with the lanes' and the CTAs' runs side by side).
+template <bool kDivide>
 __global__ void __launch_bounds__(256) k_em_sum_warps(SumArgs a) {
   __shared__ double stages[8][seq_at<8>(256)];
   __shared__ uint32_t masks[8][8];
   const unsigned lane = lane_id();
-  double *stage = stages[threadIdx.x >> 5];
-  uint32_t *mask = masks[threadIdx.x >> 5];
-  uint64_t start = 0;
-  for (int c = 0; c < kSumWarp; c++) start += a.plan.count[c];
-  const uint32_t *runs = a.plan.list + start;
+  const uint32_t *runs = a.plan.runs(kSumWarp, a.n);
   const uint64_t nwarp = a.plan.count[kSumWarp];
+  if (!nwarp) return;
   uint64_t outdeg = 0;
   for (;;) {
     unsigned long long i = 0;
@@ -483,27 +629,7 @@ __global__ void __launch_bounds__(256) k_em_sum_warps(SumArgs a) {
     i = __shfl_sync(kFull, i, 0);
     if (i >= nwarp) break;
     const uint32_t v = runs[i];
-    const uint64_t b = a.off[v], e = a.off[v + 1];
-    SeqSum s{a.sum[v], false, false};
-    for (uint64_t j0 = b; j0 < e; j0 += 256) {
-      uint32_t u[8];
-#pragma unroll
-      for (int r = 0; r < 8; r++) u[r] = j0 + r * 32 + lane < e ? a.slots[j0 + r * 32 + lane] : kSentinel;
-#pragma unroll
-      for (int r = 0; r < 8; r++) {
-        const bool has = a.member(u[r]);
-        const unsigned word = __ballot_sync(kFull, has);
-        stage[seq_at<8>(r * 32 + lane)] = has ? a.value(u[r]) : 0.0;
-        if (lane == 0) mask[r] = word;
-      }
-      __syncwarp();
-      double x[8];
-#pragma unroll
-      for (int r = 0; r < 8; r++) x[r] = stage[seq_at<8>(8 * lane + r)];
-      seq_warp(s, x, reinterpret_cast<const unsigned char *>(mask)[lane]);
-      __syncwarp();
-    }
-    if (lane == 0 && s.any) a.sum[v] = s.acc;
+    const SeqSum s = sum_warp_run<kDivide>(a, v, a.off[v], a.off[v + 1], stages[threadIdx.x >> 5], masks[threadIdx.x >> 5]);
     emit_out(lane == 0 && a.output && (a.zero_marks ? s.zero : s.any), v, a.out_list, a.out_bits, a.deg, a.cnt, outdeg);
   }
   outdeg = warp_sum(outdeg);
@@ -665,25 +791,34 @@ __global__ void k_fill_f64(double *a, uint64_t n, double x) {
 int sum_plan(byo_graph *g, SumPlan *p) {
   byo_ctx *ctx = g->ctx;
   BYO_TRY(ws(g, WS_DEFER, g->n + 1, &p->list));
-  BYO_TRY(ws(g, WS_BUCKETS, 2 * kSumClasses + 1, &p->count));
-  BYO_CU(ctx, cudaMemsetAsync(p->count, 0, (2 * kSumClasses + 1) * 8, ctx->stream));
+  BYO_TRY(ws(g, WS_BUCKETS, kSumCounts, &p->count));
+  BYO_CU(ctx, cudaMemsetAsync(p->count, 0, kSumCounts * 8, ctx->stream));
+  p->direct = p->listed = false;
   const dim3 grid(grid_for(ctx, (g->n + 3) / 4, 1024, 2));
   launch(ctx, k_sum_plan<false>, grid, dim3(1024), 0, (const uint64_t *)g->d_off, g->n, *p);
   launch(ctx, k_sum_plan<true>, grid, dim3(1024), 0, (const uint64_t *)g->d_off, g->n, *p);
   return check_launch(ctx, "edge_map plan");
 }
 
-// A dense round of a functor that sums (PR_F, PR_Delta_F).
-int sum_round(byo_graph *g, SumArgs a, Frontier &in, Frontier &out, bool output, unsigned long long *cnt,
-              const SumPlan *plan) {
+// A round of edgeMap: its counts on the device ([0..1] the members out and their
+// edges, [2] k_em_pull's long runs, from kEmCounts on those of a SumPlan).
+constexpr uint64_t kSumBeside = 1 << 22;
+constexpr int kEmCounts = 8, kEmWords = kEmCounts + kSumCounts;
+struct EmRound {
+  const SumPlan *plan;
+  unsigned long long *cnt;
+};
+
+// A dense round of a functor that sums (PR_F, PR_Delta_F): by a plan, or on its
+// own.
+template <bool kDivide>
+int sum_round(byo_graph *g, SumArgs a, Frontier &in, Frontier &out, bool output, EmRound &r) {
   byo_ctx *ctx = g->ctx;
   a.fb = nullptr;
   if (!in.all) {  // (a list may hold an id twice, so its size does not tell)
     BYO_TRY(ensure_bits(g, in));
     a.fb = in.bits;
   }
-  if (plan) a.plan = *plan; else BYO_TRY(sum_plan(g, &a.plan));
-  BYO_CU(ctx, cudaMemsetAsync(a.plan.count + 2 * kSumClasses, 0, 8, ctx->stream));
   a.off = g->d_off;
   a.slots = g->d_slots;
   a.deg = g->d_deg;
@@ -691,13 +826,44 @@ int sum_round(byo_graph *g, SumArgs a, Frontier &in, Frontier &out, bool output,
   a.output = output ? 1 : 0;
   a.out_list = out.list;
   a.out_bits = out.bits;
-  a.cnt = cnt;
+  a.cnt = r.cnt;
+  if (!r.plan) {
+    a.plan.count = r.cnt + kEmCounts;
+    a.plan.direct = true;
+    BYO_TRY(ws(g, WS_DEFER, g->n + 1, &a.plan.list));
+    const bool gaps = g->nslots != g->m;
+    // the longest run there can be
+    const uint64_t longest = gaps ? g->nslots : std::min(g->n, g->m);
+    const dim3 lanes(grid_for(ctx, (g->n + 31) / 32 * 32, 256)), ctas(ctx->num_sms),
+        warps(grid_for(ctx, g->nslots / kSumShort * 32, 256, 4));
+    const auto direct = gaps ? k_em_sum_direct<kDivide, true> : k_em_sum_direct<kDivide, false>;
+    if (g->nslots <= kSumBeside) {
+      launch(ctx, direct, lanes, dim3(256), 0, a);
+      if (longest > kSumShort) launch(ctx, k_em_sum_warps<kDivide>, warps, dim3(256), 0, a);
+      if (longest > kSumWarpMax) launch(ctx, k_em_sum_ctas<kDivide>, ctas, dim3(kSumBlock), 0, a);
+      return check_launch(ctx, "edge_map");
+    }
+    a.plan.listed = true;
+    launch(ctx, gaps ? k_sum_long<true> : k_sum_long<false>, dim3(grid_for(ctx, (g->n + 3) / 4, 1024, 2)), dim3(1024), 0,
+           a);
+    BYO_TRY(side_fork(ctx, 0));
+    BYO_TRY(side_fork(ctx, 1));
+    k_em_sum_ctas<kDivide><<<ctas, kSumBlock, 0, ctx->side[0]>>>(a);
+    k_em_sum_warps<kDivide><<<warps, 256, 0, ctx->side[1]>>>(a);
+    ctx->launches += 2;
+    launch(ctx, direct, lanes, dim3(256), 0, a);
+    BYO_TRY(side_join(ctx, 0));
+    BYO_TRY(side_join(ctx, 1));
+    return check_launch(ctx, "edge_map");
+  }
+  a.plan = *r.plan;
+  BYO_CU(ctx, cudaMemsetAsync(a.plan.count + 2 * kSumClasses, 0, 8, ctx->stream));
   // the three take vertices of their own: side by side, the longest runs' few
   // CTAs leave room for the rest
   BYO_TRY(side_fork(ctx, 0));
   BYO_TRY(side_fork(ctx, 1));
-  k_em_sum_ctas<<<ctx->num_sms, kSumBlock, 0, ctx->side[0]>>>(a);
-  k_em_sum_warps<<<grid_for(ctx, g->nslots / kSumLaneMax * 32, 256), 256, 0, ctx->side[1]>>>(a);
+  k_em_sum_ctas<kDivide><<<ctx->num_sms, kSumBlock, 0, ctx->side[0]>>>(a);
+  k_em_sum_warps<kDivide><<<grid_for(ctx, g->nslots / kSumLaneMax * 32, 256), 256, 0, ctx->side[1]>>>(a);
   ctx->launches += 2;
   launch(ctx, k_em_sum_lanes, dim3(grid_for(ctx, g->n, 256)), dim3(256), 0, a);
   BYO_TRY(side_join(ctx, 0));
@@ -705,32 +871,38 @@ int sum_round(byo_graph *g, SumArgs a, Frontier &in, Frontier &out, bool output,
   return check_launch(ctx, "edge_map");
 }
 
-int pull_round(byo_graph *g, const PrF &f, Frontier &in, Frontier &out, bool output, unsigned long long *cnt,
-               const SumPlan *plan) {
+// Slots up to which the divisions are made one an edge: one a vertex is a launch
+// of its own (2.5 us), but a warp's 32 terms take a division's time if one needs it.
+constexpr uint64_t kDivideSlots = 1 << 16;
+
+int pull_round(byo_graph *g, const PrF &f, Frontier &in, Frontier &out, bool output, EmRound &r) {
   SumArgs a{};
+  a.stride = 1;
+  a.sum = f.pn;
+  if (!r.plan && g->nslots <= kDivideSlots) {
+    a.val = f.pc;
+    return sum_round<true>(g, a, in, out, output, r);
+  }
   double *val = nullptr;
   BYO_TRY(ws(g, WS_PR_D, g->n + 1, &val));
   launch(g->ctx, k_em_values, dim3(grid_for(g->ctx, g->n, 256)), dim3(256), 0, f, g->n, val);
   a.val = val;
-  a.stride = 1;
-  a.sum = f.pn;
-  return sum_round(g, a, in, out, output, cnt, plan);
+  return sum_round<false>(g, a, in, out, output, r);
 }
 
-int pull_round(byo_graph *g, const PrDeltaF &f, Frontier &in, Frontier &out, bool output, unsigned long long *cnt,
-               const SumPlan *plan) {
+int pull_round(byo_graph *g, const PrDeltaF &f, Frontier &in, Frontier &out, bool output, EmRound &r) {
   SumArgs a{};
   a.val = f.delta;
   a.stride = 2;
   a.at = 1;
   a.sum = f.ngh;
   a.zero_marks = 1;
-  return sum_round(g, a, in, out, output, cnt, plan);
+  return sum_round<false>(g, a, in, out, output, r);
 }
 
-int pull_round(byo_graph *g, const LabelF &f, Frontier &in, Frontier &out, bool output, unsigned long long *cnt,
-               const SumPlan *) {
+int pull_round(byo_graph *g, const LabelF &f, Frontier &in, Frontier &out, bool output, EmRound &r) {
   byo_ctx *ctx = g->ctx;
+  unsigned long long *const cnt = r.cnt;
   BYO_TRY(ensure_bits(g, in));
   uint32_t *defer = nullptr;
   BYO_TRY(ws(g, WS_DEFER, g->n + 1, &defer));
@@ -745,18 +917,17 @@ int pull_round(byo_graph *g, const LabelF &f, Frontier &in, Frontier &out, bool 
 }
 
 template <class F>
-int run_round(byo_graph *g, const F &f, Frontier &in, Frontier &out, int mode, bool output,
-              unsigned long long *cnt, const SumPlan *plan) {
+int run_round(byo_graph *g, const F &f, Frontier &in, Frontier &out, int mode, bool output, EmRound &r) {
   byo_ctx *ctx = g->ctx;
   const int block = 256;
   if (mode == MODE_PULL) {
-    BYO_TRY(pull_round(g, f, in, out, output, cnt, plan));
+    BYO_TRY(pull_round(g, f, in, out, output, r));
   } else {  // sparse, blocked and dense forward: updateAtomic from the members
     BYO_TRY(ensure_list(g, in));
     if (in.size)
       launch(ctx, k_em_push<F>, dim3(grid_for(ctx, in.size * 32, block)), dim3(block), 0,
              (const uint64_t *)g->d_off, (const uint32_t *)g->d_slots, (const uint32_t *)g->d_deg, f,
-             (const uint32_t *)in.list, in.size, output ? 1 : 0, out.list, out.bits, cnt);
+             (const uint32_t *)in.list, in.size, output ? 1 : 0, out.list, out.bits, r.cnt);
   }
   return check_launch(ctx, "edge_map");
 }
@@ -796,18 +967,18 @@ int frontier_from_bits(byo_graph *g, const uint32_t *d_bits, Frontier &f) {
 static int edge_map_planned(byo_graph *g, const FunctorArgs &fa, Frontier &in, Frontier &out, int mode, bool output,
                             const SumPlan *plan) {
   byo_ctx *ctx = g->ctx;
-  unsigned long long *cnt = nullptr;
-  BYO_TRY(ws(g, WS_STATS, 8, (uint64_t **)&cnt));
-  BYO_CU(ctx, cudaMemsetAsync(cnt, 0, 64, ctx->stream));
+  EmRound r{plan, nullptr};
+  BYO_TRY(ws(g, WS_STATS, kEmWords, (uint64_t **)&r.cnt));
+  BYO_CU(ctx, cudaMemsetAsync(r.cnt, 0, kEmWords * 8, ctx->stream));
   switch (fa.kind) {
-    case BYO_F_BFS_LABEL: BYO_TRY(run_round(g, LabelF{fa.parents, fa.src}, in, out, mode, output, cnt, plan)); break;
-    case BYO_F_PR: BYO_TRY(run_round(g, PrF{fa.p_curr, fa.p_next, g->d_deg}, in, out, mode, output, cnt, plan)); break;
-    case BYO_F_PR_DELTA: BYO_TRY(run_round(g, PrDeltaF{fa.delta, fa.ngh}, in, out, mode, output, cnt, plan)); break;
+    case BYO_F_BFS_LABEL: BYO_TRY(run_round(g, LabelF{fa.parents, fa.src}, in, out, mode, output, r)); break;
+    case BYO_F_PR: BYO_TRY(run_round(g, PrF{fa.p_curr, fa.p_next, g->d_deg}, in, out, mode, output, r)); break;
+    case BYO_F_PR_DELTA: BYO_TRY(run_round(g, PrDeltaF{fa.delta, fa.ngh}, in, out, mode, output, r)); break;
     default: return set_error(ctx, BYO_EINVAL, "edge_map: unknown functor kind");
   }
   unsigned long long h[2] = {0, 0};
   if (output) {  // no output: the host waits for nothing
-    BYO_CU(ctx, cudaMemcpyAsync(h, cnt, 16, cudaMemcpyDeviceToHost, ctx->stream));
+    BYO_CU(ctx, cudaMemcpyAsync(h, r.cnt, 16, cudaMemcpyDeviceToHost, ctx->stream));
     BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
   }
   out.size = h[0];
