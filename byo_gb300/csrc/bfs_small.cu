@@ -11,7 +11,8 @@
 // which rounds it ran.  It leaves as soon as the next frontier is empty,
 // grows past `limit` edges or (gate_hub) holds a vertex of degree >= 4^5, and
 // hands the host the frontier in the engine's form (list + bitmap, its size,
-// out-degree and degree sketch), so the round loop continues from there.
+// out-degree and degree sketch), so the round loop continues from there.  It
+// counts slots as edges: a BFS runs on a view without gaps (traversal_view).
 //
 // A round is bound by the chain of dependent L2 accesses, so the chain is
 // kept short: a frontier entry carries its slot range, fetched when the vertex

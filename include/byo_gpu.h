@@ -206,7 +206,13 @@ int byo_gen_uniform_keys_device(byo_ctx *ctx, uint64_t seed, uint64_t n, uint64_
                                 uint64_t *d_keys);
 
 /* ------------------------------------------------------------------ traversal
- * Direction policy for edgeMap rounds (the choice never changes a result). */
+ * Direction policy for edgeMap rounds (the choice never changes a result where
+ * every edge is stored at both ends; a pull reads the edges of the vertex reached).
+ * Under M20, LEARNED and PUSH consecutive rounds on small frontiers run in one
+ * launch, always as pushes: under M20 and PUSH frontiers of up to 65536 vertices and
+ * edges together, whatever the rule would choose for them (a push costs least
+ * there), under LEARNED up to min(65536, max(4096, m / 1280)) without a vertex of
+ * degree 1024 or more. */
 enum byo_policy {
   BYO_POLICY_M20 = 0,          /* GBBS rule, edge_map_data.h:254-307 (sparse = push) */
   BYO_POLICY_LEARNED = 1,      /* MLP over frontier statistics, falls back to M20 */
@@ -494,7 +500,9 @@ int byo_vertex_map(byo_vertex_subset *vs, const byo_vertex_op *op);
 int byo_vertex_filter(byo_vertex_subset *vs, const byo_vertex_op *op, byo_vertex_subset **out);
 
 /* ------------------------------------------------------------------ statistics
- * Per-round log of the last traversal (the learned policy's training data). */
+ * Per-round log of the last traversal (the learned policy's training data).
+ * Rounds that ran in one launch (see byo_policy) are logged as pushes, with
+ * unvisited, ms and features zero. */
 typedef struct byo_round_log {
   uint32_t round;
   uint32_t mode;          /* 0 push, 1 pull, 2 blocked */
