@@ -134,8 +134,10 @@ __device__ __forceinline__ void visit_emit(const uint32_t (&u)[R], const uint32_
 // round of a 2^22-vertex RMAT graph's largest hubs up for 1.3 ms; 0.11 in chunks.
 constexpr uint32_t kHubChunk = 2048;
 
+// Eight CTAs an SM: at 40 registers, six, a BFS by pushes alone on RMAT 2^22 / 2^26
+// draws took 2300 us instead of 2000.
 template <int GS>
-__global__ void __launch_bounds__(256) k_push(const uint64_t *__restrict__ off,
+__global__ void __launch_bounds__(256, 8) k_push(const uint64_t *__restrict__ off,
                                               const uint32_t *__restrict__ slots,
                                               const uint32_t *__restrict__ deg,
                                               const uint32_t *__restrict__ F, uint64_t fsize,
