@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(256) k_em_pull_long(const uint64_t *__restrict
 // run of the first ones, a warp one of the next to last and a CTA one of the
 // last.  A warp's FP64 addition takes the pipe 19 cycles however many lanes
 // add, so 32 runs of one length cost a warp what a single one would.
-constexpr uint32_t kSumLaneMax = 128, kSumWarpMax = 4096, kSumShort = 32;
+constexpr uint32_t kSumLaneMax = 128, kSumWarpMax = 4096;
 constexpr int kSumLanes = 11, kSumWarp = kSumLanes, kSumCta = kSumLanes + 1, kSumClasses = kSumLanes + 2;
 __device__ __forceinline__ int sum_class(uint64_t len) {  // 1..2, 3..4, ..8, ..12, ..16, 24, 32, .. kSumLaneMax
   if (len <= 8) return len <= 2 ? 0 : len <= 4 ? 1 : 2;
@@ -439,19 +439,44 @@ __device__ __forceinline__ SeqSum sum_warp_run(const SumArgs &a, uint32_t v, uin
   return s;
 }
 
+// The listed runs of the warps, each warp the next one.
+template <bool kDivide>
+__device__ __forceinline__ void sum_warp_runs(const SumArgs &a, double *stage, uint32_t *mask) {
+  const unsigned lane = lane_id();
+  const uint32_t *runs = a.plan.runs(kSumWarp, a.n);
+  const uint64_t nwarp = a.plan.count[kSumWarp];
+  if (!nwarp) return;
+  uint64_t outdeg = 0;
+  for (;;) {
+    unsigned long long i = 0;
+    if (lane == 0) i = atomicAdd(a.plan.count + 2 * kSumClasses, 1ull);
+    i = __shfl_sync(kFull, i, 0);
+    if (i >= nwarp) break;
+    const uint32_t v = runs[i];
+    const SeqSum s = sum_warp_run<kDivide>(a, v, a.off[v], a.off[v + 1], stage, mask);
+    emit_out(lane == 0 && a.output && (a.zero_marks ? s.zero : s.any), v, a.out_list, a.out_bits, a.deg, a.cnt, outdeg);
+  }
+  outdeg = warp_sum(outdeg);
+  if (lane == 0 && outdeg) atomicAdd(a.cnt + 1, (unsigned long long)outdeg);
+}
+
 // A round on its own: planning it costs two passes and the launches of three
 // streams, 12 us of a 40 us call on small graphs, and on uniform graphs there is
 // little to tell apart (10^6 vertices of degree 16, a fiftieth of them in the
 // frontier: 326 us a call by a plan, 237 so).  A lane per vertex of up to kSumShort
-// slots, 8 of them in flight; the longer runs are listed for the kernels below.  At
-// 16 / 24 / 32 / 64 slots: that graph 524 / 252 / 237 / 236 us a call, Chung-Lu of 10^5
-// vertices 93 / 93 / 93 / 98, RMAT 2^20 / 2^24 draws 521 / 515 / 517 / 540.
-// On a view with gaps (kGaps) a short list may have a leaf's gap in it: up to
-// kGapRun slots its warp takes it at once.
-constexpr uint32_t kGapRun = 512;
+// neighbours, 8 of its slots in flight; the longer runs are listed for the kernels
+// below.  At 16 / 24 / 32 / 64 neighbours: that graph 524 / 252 / 237 / 236 us a call,
+// Chung-Lu of 10^5 vertices 93 / 93 / 93 / 98, RMAT 2^20 / 2^24 draws 521 / 515 / 517 / 540.
+// On a view with gaps (kGaps) so few neighbours may lie in a run of any length: a
+// lane takes it up to twice as many slots (a vector of runs has no more), its warp
+// at once up to kGapRun (a leaf's gap).
+constexpr uint32_t kSumShort = 32, kGapRun = 512;
+enum { kRunLane, kRunGap, kRunWarp, kRunCta };
 template <bool kGaps>
-__device__ __forceinline__ bool sum_gap(const SumArgs &a, uint64_t v, uint64_t len) {
-  return kGaps && len > kSumShort && len <= kGapRun && a.deg[v] <= kSumShort;
+__device__ __forceinline__ int sum_run(const SumArgs &a, uint64_t v, uint64_t len) {
+  if (len <= kSumShort) return kRunLane;
+  if (kGaps && len <= kGapRun && a.deg[v] <= kSumShort) return len <= 2 * kSumShort ? kRunLane : kRunGap;
+  return len <= kSumWarpMax ? kRunWarp : kRunCta;
 }
 
 // The long runs listed by a pass of its own: from kSumBeside slots on, so that
@@ -469,7 +494,8 @@ __global__ void __launch_bounds__(1024) k_sum_long(SumArgs a) {
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const uint64_t v = base + q * 1024 + threadIdx.x, len = v < a.n ? a.off[v + 1] - a.off[v] : 0;
-      c[q] = len > kSumWarpMax ? 1 : len > kSumShort && !sum_gap<kGaps>(a, v, len) ? 0 : -1;
+      const int run = sum_run<kGaps>(a, v, len);
+      c[q] = run == kRunCta ? 1 : run == kRunWarp ? 0 : -1;
       slot[q] = c[q] >= 0 ? atomicAdd(cnt + c[q], 1u) : 0;
     }
     __syncthreads();
@@ -498,7 +524,8 @@ __global__ void __launch_bounds__(256, kDivide || kGaps ? 4 : 5) k_em_sum_direct
     const uint64_t v = w * 32 + lane_id();
     const uint64_t b = v < a.n ? a.off[v] : 0, len = v < a.n ? a.off[v + 1] - b : 0;
     bool any = false, zero = false;
-    if (len && len <= kSumShort) {
+    const int run = sum_run<kGaps>(a, v, len);
+    if (len && run == kRunLane) {
       const uint32_t *const ids = a.slots + b;
       double acc = 0.0;
       for (uint32_t j = 0; j < len; j += 8) {
@@ -523,9 +550,8 @@ __global__ void __launch_bounds__(256, kDivide || kGaps ? 4 : 5) k_em_sum_direct
       }
       if (any) a.sum[v] = acc;
     }
-    const bool gap = sum_gap<kGaps>(a, v, len);
     if constexpr (kGaps) {
-      for (unsigned m = __ballot_sync(kFull, gap); m; m &= m - 1) {
+      for (unsigned m = __ballot_sync(kFull, run == kRunGap); m; m &= m - 1) {
         const int k = __ffs(m) - 1;
         const uint64_t from = __shfl_sync(kFull, b, k);
         const SeqSum s = sum_warp_run<kDivide>(a, (uint32_t)(w * 32 + k), from, from + __shfl_sync(kFull, len, k),
@@ -537,11 +563,10 @@ __global__ void __launch_bounds__(256, kDivide || kGaps ? 4 : 5) k_em_sum_direct
       }
     }
     if (!a.plan.listed) {
-      const bool cta = len > kSumWarpMax, warp = len > kSumShort && !gap && !cta;
-      const uint64_t at = warp_append(warp, a.plan.count + kSumWarp);
-      if (warp) a.plan.list[at] = (uint32_t)v;
-      const uint64_t back = warp_append(cta, a.plan.count + kSumCta);
-      if (cta) a.plan.list[a.n - 1 - back] = (uint32_t)v;
+      const uint64_t at = warp_append(run == kRunWarp, a.plan.count + kSumWarp);
+      if (run == kRunWarp) a.plan.list[at] = (uint32_t)v;
+      const uint64_t back = warp_append(run == kRunCta, a.plan.count + kSumCta);
+      if (run == kRunCta) a.plan.list[a.n - 1 - back] = (uint32_t)v;
     }
     emit_out(a.output && (a.zero_marks ? zero : any), (uint32_t)v, a.out_list, a.out_bits, a.deg, a.cnt, outdeg);
   }
@@ -552,9 +577,11 @@ __global__ void __launch_bounds__(256, kDivide || kGaps ? 4 : 5) k_em_sum_direct
 // Runs above 4096 slots, a CTA each (seqsum.cuh), 4096 neighbours a step: bound by
 // the largest hub's steps (1.4 us each).  Chung-Lu n = 10^6, whose hub has 500 K
 // neighbours: 172 us a round; one lane adding a warp's values in turn took 20 ms.
-// 64 registers instead of 128 spill the loads in flight: 364 us.
+// 64 registers instead of 128 spill the loads in flight: 364 us.  kRest: then the
+// warps' runs too, on views where the launch saved is more than what fewer warps
+// an SM (128 registers) cost: uniform 10^5 vertices of degree 8 56 -> 50 us a call.
 constexpr int kSumBlock = 512, kSumTerms = 8;
-template <bool kDivide>
+template <bool kDivide, bool kRest>
 __global__ void __launch_bounds__(kSumBlock, 1) k_em_sum_ctas(SumArgs a) {
   __shared__ double stage[seq_at<kSumTerms>(kSumTerms * kSumBlock)];
   __shared__ uint32_t mask[kSumTerms * kSumBlock / 32];
@@ -610,6 +637,12 @@ __global__ void __launch_bounds__(kSumBlock, 1) k_em_sum_ctas(SumArgs a) {
     }
   }
   if (threadIdx.x == 0 && outdeg) atomicAdd(a.cnt + 1, (unsigned long long)outdeg);
+  if constexpr (kRest) {
+    constexpr int kPart = seq_at<8>(256);
+    static_assert(kPart * kSumBlock / 32 == seq_at<kSumTerms>(kSumTerms * kSumBlock), "a warp's part of the stage");
+    __syncthreads();
+    sum_warp_runs<kDivide>(a, stage + (threadIdx.x >> 5) * kPart, mask + (threadIdx.x >> 5) * 8);
+  }
 }
 
 // Runs of kSumLaneMax to 4096 slots, a warp each: 108 us a round on the same graph
@@ -618,22 +651,7 @@ template <bool kDivide>
 __global__ void __launch_bounds__(256) k_em_sum_warps(SumArgs a) {
   __shared__ double stages[8][seq_at<8>(256)];
   __shared__ uint32_t masks[8][8];
-  const unsigned lane = lane_id();
-  const uint32_t *runs = a.plan.runs(kSumWarp, a.n);
-  const uint64_t nwarp = a.plan.count[kSumWarp];
-  if (!nwarp) return;
-  uint64_t outdeg = 0;
-  for (;;) {
-    unsigned long long i = 0;
-    if (lane == 0) i = atomicAdd(a.plan.count + 2 * kSumClasses, 1ull);
-    i = __shfl_sync(kFull, i, 0);
-    if (i >= nwarp) break;
-    const uint32_t v = runs[i];
-    const SeqSum s = sum_warp_run<kDivide>(a, v, a.off[v], a.off[v + 1], stages[threadIdx.x >> 5], masks[threadIdx.x >> 5]);
-    emit_out(lane == 0 && a.output && (a.zero_marks ? s.zero : s.any), v, a.out_list, a.out_bits, a.deg, a.cnt, outdeg);
-  }
-  outdeg = warp_sum(outdeg);
-  if (lane == 0 && outdeg) atomicAdd(a.cnt + 1, (unsigned long long)outdeg);
+  sum_warp_runs<kDivide>(a, stages[threadIdx.x >> 5], masks[threadIdx.x >> 5]);
 }
 
 // ---------------------------------------------------------------- frontier forms
@@ -839,8 +857,7 @@ int sum_round(byo_graph *g, SumArgs a, Frontier &in, Frontier &out, bool output,
     const auto direct = gaps ? k_em_sum_direct<kDivide, true> : k_em_sum_direct<kDivide, false>;
     if (g->nslots <= kSumBeside) {
       launch(ctx, direct, lanes, dim3(256), 0, a);
-      if (longest > kSumShort) launch(ctx, k_em_sum_warps<kDivide>, warps, dim3(256), 0, a);
-      if (longest > kSumWarpMax) launch(ctx, k_em_sum_ctas<kDivide>, ctas, dim3(kSumBlock), 0, a);
+      if (longest > kSumShort) launch(ctx, k_em_sum_ctas<kDivide, true>, ctas, dim3(kSumBlock), 0, a);
       return check_launch(ctx, "edge_map");
     }
     a.plan.listed = true;
@@ -848,7 +865,7 @@ int sum_round(byo_graph *g, SumArgs a, Frontier &in, Frontier &out, bool output,
            a);
     BYO_TRY(side_fork(ctx, 0));
     BYO_TRY(side_fork(ctx, 1));
-    k_em_sum_ctas<kDivide><<<ctas, kSumBlock, 0, ctx->side[0]>>>(a);
+    k_em_sum_ctas<kDivide, false><<<ctas, kSumBlock, 0, ctx->side[0]>>>(a);
     k_em_sum_warps<kDivide><<<warps, 256, 0, ctx->side[1]>>>(a);
     ctx->launches += 2;
     launch(ctx, direct, lanes, dim3(256), 0, a);
@@ -862,7 +879,7 @@ int sum_round(byo_graph *g, SumArgs a, Frontier &in, Frontier &out, bool output,
   // CTAs leave room for the rest
   BYO_TRY(side_fork(ctx, 0));
   BYO_TRY(side_fork(ctx, 1));
-  k_em_sum_ctas<kDivide><<<ctx->num_sms, kSumBlock, 0, ctx->side[0]>>>(a);
+  k_em_sum_ctas<kDivide, false><<<ctx->num_sms, kSumBlock, 0, ctx->side[0]>>>(a);
   k_em_sum_warps<kDivide><<<grid_for(ctx, g->nslots / kSumLaneMax * 32, 256), 256, 0, ctx->side[1]>>>(a);
   ctx->launches += 2;
   launch(ctx, k_em_sum_lanes, dim3(grid_for(ctx, g->n, 256)), dim3(256), 0, a);
