@@ -579,7 +579,8 @@ __global__ void __launch_bounds__(256, kDivide || kGaps ? 4 : 5) k_em_sum_direct
 // neighbours: 172 us a round; one lane adding a warp's values in turn took 20 ms.
 // 64 registers instead of 128 spill the loads in flight: 364 us.  kRest: then the
 // warps' runs too, on views where the launch saved is more than what fewer warps
-// an SM (128 registers) cost: uniform 10^5 vertices of degree 8 56 -> 50 us a call.
+// an SM (128 registers) cost: uniform 10^5 vertices of degree 8 50 -> 46 us a call, RMAT
+// 2^18 235 -> 212.
 constexpr int kSumBlock = 512, kSumTerms = 8;
 template <bool kDivide, bool kRest>
 __global__ void __launch_bounds__(kSumBlock, 1) k_em_sum_ctas(SumArgs a) {
