@@ -1800,6 +1800,10 @@ __device__ __forceinline__ void stream_sort(const StreamArgs &a, uint64_t bi, ui
 //   1. the long offset ranges of batch bi-1 (its merge is done), and the
 //      segments of batch bi (its keys were sorted during phase 2 of bi-1);
 //   2. the merge of batch bi by CTAs 1.., while CTA 0 sorts batch bi+1.
+// kQueries: ops may be queries.  Their traversal beside it takes registers from the
+// merge (64 a thread: 256 bytes spilled, none without): 400 batches of 10 to 2000
+// pairs, RMAT 2^24, 16.2 ms with it in the kernel, 14.7 without.
+template <bool kQueries>
 __global__ void __launch_bounds__(kStreamThreads) k_pma_stream(StreamArgs a) {
   extern __shared__ unsigned long long stream_smem[];
   uint64_t *As = reinterpret_cast<uint64_t *>(stream_smem);  // [kStreamWarps][kLeaf]
@@ -1816,7 +1820,7 @@ __global__ void __launch_bounds__(kStreamThreads) k_pma_stream(StreamArgs a) {
   for (uint64_t bi = a.first;; bi++) {
     const int cur = (int)(bi & 1), prv = cur ^ 1;
     const bool has = bi < a.nbatch;
-    const bool query = has && a.ops[bi] == kOpQuery;
+    const bool query = kQueries && has && a.ops[bi] == kOpQuery;
     const bool valid = has && (query || (c->bounds[cur][0] < a.n && c->bounds[cur][1] < a.n));
     // phase 1
     if (bi > a.first) {
@@ -1845,7 +1849,7 @@ __global__ void __launch_bounds__(kStreamThreads) k_pma_stream(StreamArgs a) {
       return;
     }
     const bool next_update = bi + 1 < a.nbatch && a.ops[bi + 1] != kOpQuery;
-    if (query) {
+    if constexpr (kQueries) if (query) {
       // a 64-source BFS over the current contents
       const MsArgs &qa = a.qargs[a.qnum[bi]];
       MsCtl *qc = qa.ctl;
@@ -1955,9 +1959,10 @@ int pma_update_stream(byo_graph *g, const uint64_t *d_keys, const uint64_t *d_bo
   BYO_TRY(ensure(ctx, p->misc, 128 + sizeof(StreamCtl) + 8 * nbatch));
   c = reinterpret_cast<StreamCtl *>((char *)p->misc.p + 128);
   d_changed = reinterpret_cast<long long *>(c + 1);
-  BYO_CU(ctx, cudaFuncSetAttribute(k_pma_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmem));
+  const auto stream_kernel = nq ? k_pma_stream<true> : k_pma_stream<false>;
+  BYO_CU(ctx, cudaFuncSetAttribute(stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmem));
   int per_sm = 0;
-  BYO_CU(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pma_stream, kStreamThreads, kStreamSmem));
+  BYO_CU(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stream_kernel, kStreamThreads, kStreamSmem));
   if (per_sm < 1) return set_error(ctx, BYO_EDEVICE, "update stream: persistent kernel cannot be resident");
   StreamCtl *hc = nullptr;
   BYO_TRY(pinned(ctx, std::max<size_t>(sizeof(StreamCtl), 4096), (void **)&hc));
@@ -2033,7 +2038,7 @@ int pma_update_stream(byo_graph *g, const uint64_t *d_keys, const uint64_t *d_bo
     a.qnum = d_qnum;
     a.op_ns = d_op_ns;
     void *args[] = {(void *)&a};
-    BYO_CU(ctx, cudaLaunchCooperativeKernel((const void *)k_pma_stream, dim3(ctx->num_sms * per_sm),
+    BYO_CU(ctx, cudaLaunchCooperativeKernel((const void *)stream_kernel, dim3(ctx->num_sms * per_sm),
                                             dim3(kStreamThreads), args, kStreamSmem, ctx->stream));
     ctx->launches++;
     BYO_CU(ctx, cudaMemcpyAsync(hc, c, sizeof(StreamCtl), cudaMemcpyDeviceToHost, ctx->stream));
