@@ -31,41 +31,45 @@ constexpr int kSample = 2;  // cc_run's two rounds
 
 __device__ __forceinline__ uint32_t ld_parent(const uint32_t *p, uint32_t v) { return __ldcg(p + v); }
 
-// Root of v; parents only ever point to smaller ids.  With kShorten the entries
-// read on the way are pointed at ancestors: v's own at the root, and the others
-// by path halving from the kPlainHops-th step on, which a chain needs.  Halving
-// at every step, all vertices of a large tree store into the few entries below
-// its root, and stores and loads of one word take turns at the L2, about one a ns
-// (second round of a uniform graph of 1 M vertices, average degree 1.6: 0.4 to
-// 1.6 ms halving at every step, the whole labelling 0.4 ms now).
+// Root of v, whose parent is `cur`; parents only ever point to smaller ids.  With
+// kShorten the entries read on the way are pointed at ancestors: v's own at the
+// root, and the others by path halving from the kPlainHops-th step on, which a
+// chain needs.  Halving at every step, all vertices of a large tree store into the
+// few entries below its root, and stores and loads of one word take turns at the L2,
+// about one a ns (second round of a uniform graph of 1 M vertices, average degree 1.6:
+// 0.4 to 1.6 ms halving at every step, the whole labelling 0.4 ms now).  kFar: where
+// the parents are far larger than the L2 a step waits for memory instead, and
+// halving at every step, with no other store, is the faster (see cc_run).
 constexpr int kPlainHops = 16;
-template <bool kShorten = true>
-__device__ __forceinline__ uint32_t cc_find(uint32_t *p, uint32_t v) {
-  uint32_t cur = ld_parent(p, v);
+template <bool kShorten = true, bool kFar = false>
+__device__ __forceinline__ uint32_t cc_find(uint32_t *p, uint32_t v, uint32_t cur) {
   if (cur == v) return v;
   uint32_t prev = v, next;
   int hops = 0;
   while (cur > (next = ld_parent(p, cur))) {
-    if (kShorten && ++hops > kPlainHops) p[prev] = next;
+    if (kShorten && (++hops > kPlainHops || kFar)) p[prev] = next;
     prev = cur;
     cur = next;
   }
-  if (kShorten && hops) p[v] = cur;
+  if (kShorten && !kFar && hops) p[v] = cur;
   return cur;
 }
 
 // Hook the larger root under the smaller until both share a root.  Equal parents
-// end it before the roots, which are the words all threads read, are touched.
-__device__ __forceinline__ void cc_link(uint32_t *p, uint32_t u, uint32_t v) {
-  if (ld_parent(p, u) == ld_parent(p, v)) return;
-  uint32_t ru = cc_find(p, u), rv = cc_find(p, v);
+// end it before the roots, which are the words all threads read, are touched
+// (`equal`: worth looking).
+template <bool kFar = false>
+__device__ __forceinline__ void cc_link(uint32_t *p, uint32_t u, uint32_t v, bool equal = true) {
+  const uint32_t pu = ld_parent(p, u), pv = ld_parent(p, v);
+  if (equal && pu == pv) return;
+  uint32_t ru = cc_find<true, kFar>(p, u, pu), rv = cc_find<true, kFar>(p, v, pv);
   while (ru != rv) {
     uint32_t hi = ru > rv ? ru : rv, lo = ru > rv ? rv : ru;
     uint32_t old = atomicCAS(p + hi, hi, lo);
     if (old == hi) return;
     // hi got a parent meanwhile: continue from the new roots
-    ru = cc_find(p, old);
-    rv = cc_find(p, lo);
+    ru = cc_find<true, kFar>(p, old, ld_parent(p, old));
+    rv = cc_find<true, kFar>(p, lo, ld_parent(p, lo));
   }
 }
 
@@ -102,15 +106,18 @@ __global__ void k_cc_first(const uint64_t *__restrict__ off, const uint32_t *__r
 
 // What the first round left: the edges to a larger first neighbour, then every
 // vertex to its second.
+// (kFar: *few, whether few of the parents are equal.)
+template <bool kFar>
 __global__ void k_cc_sample(const uint64_t *__restrict__ off, const uint32_t *__restrict__ slots,
-                            uint32_t *p, uint64_t n) {
+                            uint32_t *p, uint64_t n, const unsigned long long *few) {
+  const bool equal = !kFar || !*few;
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n;
        v += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t x = cc_sampled(off, slots, v, 0);
     if (x == kSentinel) continue;
-    if (x > v) cc_link(p, (uint32_t)v, x);
+    if (x > v) cc_link<kFar>(p, (uint32_t)v, x, equal);
     const uint32_t y = cc_sampled(off, slots, v, 1);
-    if (y != kSentinel) cc_link(p, (uint32_t)v, y);
+    if (y != kSentinel) cc_link<kFar>(p, (uint32_t)v, y, equal);
   }
 }
 
@@ -168,10 +175,12 @@ __device__ __forceinline__ void cc_hook(uint32_t *p, uint32_t v, uint32_t x) {
 // ones (1 M vertices of degree 2: 417 against 240 us), four are 3 to 10% slower.
 constexpr int kCcHookBlock = 1024, kCcHooks = 3;
 constexpr uint64_t kCcHookLeast = 1 << 15;
+constexpr uint64_t kCcFar = 1 << 24;  // 64 MB of parents
 __global__ void __launch_bounds__(kCcHookBlock, 2) k_cc_hook(const uint64_t *__restrict__ off,
                                                              const uint32_t *__restrict__ slots,
                                                              const uint32_t *__restrict__ deg, uint32_t *p, uint64_t n,
-                                                             unsigned long long *trees, GridBar *bar) {
+                                                             unsigned long long *trees, unsigned long long *few,
+                                                             int passes, GridBar *bar) {
   __shared__ unsigned int sm[kCcHookBlock / 32 + 1];
   __shared__ uint32_t cand;
   const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, nthr = (uint64_t)gridDim.x * blockDim.x;
@@ -181,15 +190,17 @@ __global__ void __launch_bounds__(kCcHookBlock, 2) k_cc_hook(const uint64_t *__r
   if (threadIdx.x == 0 && mine) atomicAdd(trees, (unsigned long long)mine);
   if (!grid_sync(bar, gridDim.x)) return;
   if (__ldcg(trees) * 256 <= n) return;
-  const uint32_t root = ld_parent(p, cc_probe(n, threadIdx.x));
+  const uint32_t probe = cc_probe(n, threadIdx.x), root = ld_parent(p, probe);
   if (threadIdx.x < 32) {
     const uint32_t c = cc_mode(root);
     if (threadIdx.x == 0) cand = c;
   }
   __syncthreads();
-  if (__syncthreads_count(root == cand) * 5 >= kCcHookBlock) return;
-  if (!grid_sync(bar, gridDim.x)) return;  // every block has probed
-  for (int pass = 0; pass < kCcHooks; pass++) {
+  const int joined = __syncthreads_count(deg[probe] != 0);
+  if (__syncthreads_count(root == cand) * 5 >= joined) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *few = 1;
+  if (!passes || !grid_sync(bar, gridDim.x)) return;  // every block has probed
+  for (int pass = 0; pass < passes; pass++) {
     for (uint64_t v = tid; v < n; v += nthr) {
       const uint32_t x = cc_sampled(off, slots, v, 0);
       if (x == kSentinel) continue;
@@ -214,7 +225,7 @@ __global__ void __launch_bounds__(256) k_cc_outside(const uint32_t *__restrict__
                                                     uint32_t *list, unsigned long long *count) {
   __shared__ uint32_t giant;
   if (threadIdx.x < 32) {
-    const uint32_t c = cc_mode(cc_find<false>(p, cc_probe(n, threadIdx.x)));
+    const uint32_t v = cc_probe(n, threadIdx.x), c = cc_mode(cc_find<false>(p, v, ld_parent(p, v)));
     if (threadIdx.x == 0) giant = c;
   }
   __syncthreads();
@@ -259,12 +270,13 @@ int cc_run(byo_graph *g, uint32_t *d_label) {
   uint32_t *p = d_label;
   const dim3 grid_v(grid_for(ctx, n, 256));
   uint32_t *words = nullptr, *list = nullptr;
-  // [0..1] count of listed vertices, [2..3] trees, then the barrier
-  BYO_TRY(ws(g, WS_MISC, 4 + sizeof(GridBar) / 4, &words));
+  // [0..1] count of listed vertices, [2..3] trees, [4..5] whether no tree holds
+  // much, then the barrier
+  BYO_TRY(ws(g, WS_MISC, 6 + sizeof(GridBar) / 4, &words));
   BYO_TRY(ws(g, WS_FRONT_LIST_A, n, &list));
-  unsigned long long *count = reinterpret_cast<unsigned long long *>(words), *trees = count + 1;
-  GridBar *bar = reinterpret_cast<GridBar *>(words + 4);
-  BYO_CU(ctx, cudaMemsetAsync(words, 0, 16 + sizeof(GridBar), ctx->stream));
+  unsigned long long *count = reinterpret_cast<unsigned long long *>(words), *trees = count + 1, *few = count + 2;
+  GridBar *bar = reinterpret_cast<GridBar *>(words + 6);
+  BYO_CU(ctx, cudaMemsetAsync(words, 0, 24 + sizeof(GridBar), ctx->stream));
   const uint64_t *off = g->d_off;
   const uint32_t *slots = g->d_slots, *deg = g->d_deg;
   launch(ctx, k_cc_first, grid_v, dim3(256), 0, off, slots, p, n);
@@ -273,22 +285,34 @@ int cc_run(byo_graph *g, uint32_t *d_label) {
   // to join: uniform graphs of average degree 16, 40000 / 300007 / 4 M vertices,
   // 186 / 829 / 1529 us without and 76 / 149 / 969 with them; RMAT with permuted
   // ids, 2^17 / 2^22 vertices, 116 / 1881 and 79 / 501.  Where hubs gather the
-  // trees (k_cc_hook sees one of n / 5 vertices or more) they made it 1.3 to 2x slower, so
+  // trees (k_cc_hook sees one of a fifth of the vertices with neighbours or more; of
+  // all vertices, RMAT 2^22 with 2^22 draws, half of them alone, took 311 us instead of
+  // 222) they made it 1.3 to 2x slower, so
   // there the kernel only compresses, 4 to 8 us slower than k_cc_compress, which
   // smaller graphs keep (uniform, 10007: 68 us either way).  Nor do they pay below
   // an average degree of 1.6, where the trees stay small: 300007 vertices, degree
   // 1.2 / 1.5 / 1.7: 82 / 162 / 140 us without, 116 / 132 / 132 with.
+  // Nor on uniform graphs whose parents are far larger than the L2, for each pass
+  // gathers two of them a vertex from memory, and the links, halving at every step,
+  // few: 2^24 / 2^25 / 2^26 vertices of degree 16 3.7 / 6.7 / 13.5 ms with the passes and
+  // 2.8 / 3.6 / 6.8 without; of degree 12 2.9 / 5.4 / 10.8 and 4.7 / 3.6 / 8.0, of degree 8
+  // 2.2 / 4.2 / 9.1 and 5.0 / 4.0 / 10.8.  There the kernel tells whether the links look
+  // for equal parents first: uniform 2^26 of degree 16 7.9 ms with and 6.8 without,
+  // RMAT 2^26 of degree 32 4.0 and 4.8.
+  const bool far = n >= kCcFar && g->m >= (n < 2 * kCcFar ? 15 : 11) * n;
   if (n < kCcHookLeast || 5 * g->m < 8 * n) {
     launch(ctx, k_cc_compress, grid_v, dim3(256), 0, p, n);
   } else {
-    int per_sm = 0;
+    int per_sm = 0, passes = far ? 0 : kCcHooks;
     BYO_CU(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cc_hook, kCcHookBlock, 0));
-    void *args[] = {(void *)&off, (void *)&slots, (void *)&deg, (void *)&p, (void *)&n, (void *)&trees, (void *)&bar};
+    void *args[] = {(void *)&off,   (void *)&slots, (void *)&deg,    (void *)&p,  (void *)&n,
+                    (void *)&trees, (void *)&few,   (void *)&passes, (void *)&bar};
     BYO_CU(ctx, cudaLaunchCooperativeKernel((const void *)k_cc_hook, dim3(per_sm * ctx->num_sms), dim3(kCcHookBlock),
                                             args, 0, ctx->stream));
     ctx->launches++;
   }
-  launch(ctx, k_cc_sample, grid_v, dim3(256), 0, off, slots, p, n);
+  launch(ctx, far ? k_cc_sample<true> : k_cc_sample<false>, grid_v, dim3(256), 0, off, slots, p, n,
+         (const unsigned long long *)few);
   launch(ctx, k_cc_outside, dim3(grid_for(ctx, n, 256)), dim3(256), 0, deg, p, n, list, count);
   const double avg = (double)g->m / (double)n;
   const int GS = avg >= 24 ? 16 : avg >= 8 ? 8 : 4;
