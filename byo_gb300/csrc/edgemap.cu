@@ -244,9 +244,8 @@ __device__ __forceinline__ int sum_class(uint64_t len) {  // 1..2, 3..4, ..8, ..
 struct SumPlan {
   uint32_t *list;             // the classes' vertices, one class after the other
   unsigned long long *count;  // [kSumClasses] vertices, [kSumClasses] cursors, [1] next warp run
-  // of a round on its own: the warps' runs only, and the CTAs' from the end of n;
-  // listed already, or by k_em_sum_direct
-  bool direct, listed;
+  // of a round on its own: the warps' runs only, and the CTAs' from the end of n
+  bool direct;
   __device__ const uint32_t *runs(int c, uint64_t n) const {
     if (direct) return c == kSumCta ? list + (n - count[c]) : list;
     uint64_t start = 0;
@@ -325,17 +324,16 @@ __global__ void k_em_values(PrF f, uint64_t n, double *val) {
     val[v] = f.value((uint32_t)v);
 }
 
-// A planned round, which is one of every vertex without output.  A lane per run:
-// 32 runs of one class, kWin terms of each at a time gathered
+// A lane per run: 32 runs of one class, kWin terms of each at a time gathered
 // by the whole warp (the runs' ids in pieces of kWin) and staged, then added
 // by the runs' lanes.  Bound by a warp's own chain (64 cycles an FP64 addition,
 // two gathers a window), so longer runs than kSumLaneMax are composed by a warp
 // instead: with lanes up to 512 slots, one warp's 32 windows took 285 us.
 // Chung-Lu n = 10^6, 16 M edges: 90 us a round; a lane that walked its own run
 // of up to 64 slots with a division for every term took 270.
-template <int kWin>
+template <int kWin, bool kMarks>
 __device__ __forceinline__ void sum_lane_runs(const SumArgs &a, const uint32_t *list, uint64_t runs, uint64_t group,
-                                              double *stage) {
+                                              double *stage, uint64_t &outdeg) {
   const unsigned lane = lane_id();
   const uint64_t i = group * 32 + lane;
   uint32_t v = 0;
@@ -347,7 +345,7 @@ __device__ __forceinline__ void sum_lane_runs(const SumArgs &a, const uint32_t *
     len = (uint32_t)(a.off[v + 1] - b);
   }
   double acc = len ? a.sum[v] : 0.0;
-  bool any = false;
+  bool any = false, zero = false;
   for (uint32_t w0 = 0; __ballot_sync(kFull, w0 < len); w0 += kWin) {
     uint32_t u[kWin];
 #pragma unroll
@@ -361,7 +359,7 @@ __device__ __forceinline__ void sum_lane_runs(const SumArgs &a, const uint32_t *
     uint32_t has = 0;
 #pragma unroll
     for (int q = 0; q < kWin; q++) {
-      const bool in = u[q] != kSentinel;
+      const bool in = kMarks ? a.member(u[q]) : u[q] != kSentinel;
       if (in) stage[(q * (32 / kWin) + lane / kWin) * (kWin + 1) + lane % kWin] = a.value(u[q]);
       const unsigned m = __ballot_sync(kFull, in);
       if ((int)(lane / (32 / kWin)) == q) has = m >> (lane % (32 / kWin) * kWin);
@@ -371,12 +369,18 @@ __device__ __forceinline__ void sum_lane_runs(const SumArgs &a, const uint32_t *
     any |= has != 0;
 #pragma unroll
     for (int k = 0; k < kWin; k++)
-      if ((has >> k) & 1u) acc = __dadd_rn(acc, stage[lane * (kWin + 1) + k]);
+      if ((has >> k) & 1u) {
+        if (kMarks) zero |= seq_zero(acc);
+        acc = __dadd_rn(acc, stage[lane * (kWin + 1) + k]);
+      }
     __syncwarp();
   }
   if (any) a.sum[v] = acc;
+  if (kMarks) emit_out(a.output && (a.zero_marks ? zero : any), v, a.out_list, a.out_bits, a.deg, a.cnt, outdeg);
 }
 
+// kMarks: a frontier, or members out (not in PageRank's rounds).
+template <bool kMarks>
 __global__ void __launch_bounds__(256) k_em_sum_lanes(SumArgs a) {
   __shared__ double stage[8][32 * 17];
   __shared__ uint64_t first[kSumLanes + 1], vert[kSumLanes + 1];  // groups and vertices before each class
@@ -396,6 +400,7 @@ __global__ void __launch_bounds__(256) k_em_sum_lanes(SumArgs a) {
   const uint64_t gw = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   double *st = stage[threadIdx.x >> 5];
+  uint64_t outdeg = 0;
   int c = kSumLanes - 1;  // the longest runs first
   for (uint64_t t = gw; t < first[kSumLanes]; t += nw) {
     const uint64_t g = first[kSumLanes] - 1 - t;
@@ -403,12 +408,15 @@ __global__ void __launch_bounds__(256) k_em_sum_lanes(SumArgs a) {
     const uint32_t *list = a.plan.list + vert[c];
     const uint64_t runs = vert[c + 1] - vert[c];
     if (c <= 1)
-      sum_lane_runs<4>(a, list, runs, g - first[c], st);
+      sum_lane_runs<4, kMarks>(a, list, runs, g - first[c], st, outdeg);
     else if (c == 2)
-      sum_lane_runs<8>(a, list, runs, g - first[c], st);
+      sum_lane_runs<8, kMarks>(a, list, runs, g - first[c], st, outdeg);
     else
-      sum_lane_runs<16>(a, list, runs, g - first[c], st);
+      sum_lane_runs<16, kMarks>(a, list, runs, g - first[c], st, outdeg);
   }
+  if (!kMarks) return;
+  outdeg = warp_sum(outdeg);
+  if (lane_id() == 0 && outdeg) atomicAdd(a.cnt + 1, (unsigned long long)outdeg);
 }
 
 // One run by a warp, 256 neighbours a step; stage: seq_at<8>(256) values, mask: 8 words.
@@ -462,15 +470,15 @@ __device__ __forceinline__ void sum_warp_runs(const SumArgs &a, double *stage, u
 
 // A round on its own: planning it costs two passes and the launches of three
 // streams, 12 us of a 40 us call on small graphs, and on uniform graphs there is
-// little to tell apart (10^6 vertices of degree 16, a fiftieth of them in the
-// frontier: 326 us a call by a plan, 237 so).  A lane per vertex of up to kSumShort
-// neighbours, 8 of its slots in flight; the longer runs are listed for the kernels
-// below.  At 16 / 24 / 32 / 64 neighbours: that graph 524 / 252 / 237 / 236 us a call,
-// Chung-Lu of 10^5 vertices 93 / 93 / 93 / 98, RMAT 2^20 / 2^24 draws 521 / 515 / 517 / 540.
+// little to tell apart (10^6 vertices of degree 16: 325 us a call by a plan, 290 so).
+// A lane per vertex of up to kSumShort neighbours, kBatch of its slots in flight; the
+// longer runs are listed for the other kernel.  At 32 neighbours instead of 64:
+// uniform 10^6 vertices of degree 24 / 32 / 48 330 / 371 / 451 -> 356 / 757 / 1229 us, Chung-Lu
+// and RMAT graphs as fast.
 // On a view with gaps (kGaps) so few neighbours may lie in a run of any length: a
 // lane takes it up to twice as many slots (a vector of runs has no more), its warp
 // at once up to kGapRun (a leaf's gap).
-constexpr uint32_t kSumShort = 32, kGapRun = 512;
+constexpr uint32_t kSumShort = 64, kGapRun = 512;
 enum { kRunLane, kRunGap, kRunWarp, kRunCta };
 template <bool kGaps>
 __device__ __forceinline__ int sum_run(const SumArgs &a, uint64_t v, uint64_t len) {
@@ -479,40 +487,35 @@ __device__ __forceinline__ int sum_run(const SumArgs &a, uint64_t v, uint64_t le
   return len <= kSumWarpMax ? kRunWarp : kRunCta;
 }
 
-// The long runs listed by a pass of its own: from kSumBeside slots on, so that
-// their kernels run beside the lanes (a call 517 -> 506 us on RMAT 2^20 / 2^24 draws,
-// 389 -> 334 on Chung-Lu of 10^6 vertices and degree 16).
+// Whether a round on its own is better planned, from 128 groups of 32 vertices: their
+// lanes' runs so unlike that most lanes would wait (the longest of 32 against their
+// mean: uniform graphs up to 2.7, Chung-Lu 2.2, for the hubs come first, RMAT 3.1 to
+// 6.1), or many too long for a lane (uniform from an average degree of about 56).
+constexpr int kSumProbes = 4;  // groups a warp
 template <bool kGaps>
-__global__ void __launch_bounds__(1024) k_sum_long(SumArgs a) {
-  __shared__ unsigned int cnt[2];
-  __shared__ unsigned long long at[2];
-  for (uint64_t base = blockIdx.x * 4096ull; base < a.n; base += gridDim.x * 4096ull) {
-    if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
-    __syncthreads();
-    int c[4];
-    unsigned int slot[4];
+__global__ void __launch_bounds__(1024) k_sum_probe(SumArgs a, unsigned long long *plan) {
+  __shared__ unsigned int s_sum, s_max, s_long;
+  if (threadIdx.x == 0) s_sum = s_max = s_long = 0;
+  __syncthreads();
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const uint64_t v = base + q * 1024 + threadIdx.x, len = v < a.n ? a.off[v + 1] - a.off[v] : 0;
-      const int run = sum_run<kGaps>(a, v, len);
-      c[q] = run == kRunCta ? 1 : run == kRunWarp ? 0 : -1;
-      slot[q] = c[q] >= 0 ? atomicAdd(cnt + c[q], 1u) : 0;
+  for (int q = 0; q < kSumProbes; q++) {
+    const uint32_t i = q * 32 + (threadIdx.x >> 5);
+    const uint64_t v = (((uint64_t)(i * 0x9E3779B1u) * ((a.n + 31) >> 5)) >> 32) * 32 + lane_id();
+    const uint64_t len = v < a.n ? a.off[v + 1] - a.off[v] : 0;
+    const uint32_t x = v < a.n ? min(kGaps ? a.deg[v] : (uint32_t)min(len, (uint64_t)kSumShort), kSumShort) : 0;
+    const uint32_t sum = __reduce_add_sync(kFull, x), top = __reduce_max_sync(kFull, x);
+    const uint32_t lng = __popc(__ballot_sync(kFull, len && sum_run<kGaps>(a, v, len) >= kRunWarp));
+    if (lane_id() == 0) {
+      atomicAdd(&s_sum, sum);
+      atomicAdd(&s_max, top);
+      atomicAdd(&s_long, lng);
     }
-    __syncthreads();
-    if (threadIdx.x < 2 && cnt[threadIdx.x])
-      at[threadIdx.x] = atomicAdd(a.plan.count + kSumWarp + threadIdx.x, (unsigned long long)cnt[threadIdx.x]);
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (c[q] >= 0) {
-        const uint64_t i = at[c[q]] + slot[q];
-        a.plan.list[c[q] ? a.n - 1 - i : i] = (uint32_t)(base + q * 1024 + threadIdx.x);
-      }
-    __syncthreads();
   }
+  __syncthreads();
+  if (threadIdx.x == 0) *plan = 32 * s_max > 3 * s_sum || 8 * s_long > 32 * kSumProbes * 32;
 }
 
-template <bool kDivide, bool kGaps>
+template <bool kDivide, bool kGaps, int kBatch>
 __global__ void __launch_bounds__(256, kDivide || kGaps ? 4 : 5) k_em_sum_direct(SumArgs a) {
   __shared__ double stages[kGaps ? 8 : 1][kGaps ? seq_at<8>(256) : 1];
   __shared__ uint32_t masks[8][8];
@@ -528,21 +531,21 @@ __global__ void __launch_bounds__(256, kDivide || kGaps ? 4 : 5) k_em_sum_direct
     if (len && run == kRunLane) {
       const uint32_t *const ids = a.slots + b;
       double acc = 0.0;
-      for (uint32_t j = 0; j < len; j += 8) {
-        uint32_t u[8];
-        double x[8];
+      for (uint32_t j = 0; j < len; j += kBatch) {
+        uint32_t u[kBatch];
+        double x[kBatch];
         unsigned in = 0;
 #pragma unroll
-        for (int q = 0; q < 8; q++) u[q] = j + q < len ? ids[j + q] : kSentinel;
+        for (int q = 0; q < kBatch; q++) u[q] = j + q < len ? ids[j + q] : kSentinel;
 #pragma unroll
-        for (int q = 0; q < 8; q++) in |= a.member(u[q]) ? 1u << q : 0u;
+        for (int q = 0; q < kBatch; q++) in |= a.member(u[q]) ? 1u << q : 0u;
         if (!in) continue;
 #pragma unroll
-        for (int q = 0; q < 8; q++) x[q] = (in >> q) & 1u ? a.value<kDivide>(u[q]) : 0.0;
+        for (int q = 0; q < kBatch; q++) x[q] = (in >> q) & 1u ? a.value<kDivide>(u[q]) : 0.0;
         if (!any) acc = a.sum[v];
         any = true;
 #pragma unroll
-        for (int q = 0; q < 8; q++)
+        for (int q = 0; q < kBatch; q++)
           if ((in >> q) & 1u) {
             zero |= seq_zero(acc);
             acc = __dadd_rn(acc, x[q]);
@@ -562,12 +565,10 @@ __global__ void __launch_bounds__(256, kDivide || kGaps ? 4 : 5) k_em_sum_direct
         }
       }
     }
-    if (!a.plan.listed) {
-      const uint64_t at = warp_append(run == kRunWarp, a.plan.count + kSumWarp);
-      if (run == kRunWarp) a.plan.list[at] = (uint32_t)v;
-      const uint64_t back = warp_append(run == kRunCta, a.plan.count + kSumCta);
-      if (run == kRunCta) a.plan.list[a.n - 1 - back] = (uint32_t)v;
-    }
+    const uint64_t at = warp_append(run == kRunWarp, a.plan.count + kSumWarp);
+    if (run == kRunWarp) a.plan.list[at] = (uint32_t)v;
+    const uint64_t back = warp_append(run == kRunCta, a.plan.count + kSumCta);
+    if (run == kRunCta) a.plan.list[a.n - 1 - back] = (uint32_t)v;
     emit_out(a.output && (a.zero_marks ? zero : any), (uint32_t)v, a.out_list, a.out_bits, a.deg, a.cnt, outdeg);
   }
   outdeg = warp_sum(outdeg);
@@ -812,7 +813,7 @@ int sum_plan(byo_graph *g, SumPlan *p) {
   BYO_TRY(ws(g, WS_DEFER, g->n + 1, &p->list));
   BYO_TRY(ws(g, WS_BUCKETS, kSumCounts, &p->count));
   BYO_CU(ctx, cudaMemsetAsync(p->count, 0, kSumCounts * 8, ctx->stream));
-  p->direct = p->listed = false;
+  p->direct = false;
   const dim3 grid(grid_for(ctx, (g->n + 3) / 4, 1024, 2));
   launch(ctx, k_sum_plan<false>, grid, dim3(1024), 0, (const uint64_t *)g->d_off, g->n, *p);
   launch(ctx, k_sum_plan<true>, grid, dim3(1024), 0, (const uint64_t *)g->d_off, g->n, *p);
@@ -820,14 +821,19 @@ int sum_plan(byo_graph *g, SumPlan *p) {
 }
 
 // A round of edgeMap: its counts on the device ([0..1] the members out and their
-// edges, [2] k_em_pull's long runs, from kEmCounts on those of a SumPlan).
-constexpr uint64_t kSumBeside = 1 << 22;
+// edges, [2] k_em_pull's long runs, [3] k_sum_probe's word, from kEmCounts on those
+// of a SumPlan).
 constexpr int kEmCounts = 8, kEmWords = kEmCounts + kSumCounts;
 struct EmRound {
   const SumPlan *plan;
   unsigned long long *cnt;
 };
 
+// A round on its own goes by a plan where most runs are too long for a lane (uniform
+// 10^5 vertices of degree 64 / 100: 106 / 130 us a call, 131 / 136 without), and from
+// kSumLarge slots on where k_sum_probe says so (8 us and a wait of the host: RMAT 2^24
+// vertices, 16 draws each, 2.0 ms a call by a plan, 2.4 without; 2^20 no difference).
+constexpr uint64_t kSumLarge = 1 << 23, kSumDense = 56, kSumDenseEdges = 1 << 22;
 // A dense round of a functor that sums (PR_F, PR_Delta_F): by a plan, or on its
 // own.
 template <bool kDivide>
@@ -846,36 +852,35 @@ int sum_round(byo_graph *g, SumArgs a, Frontier &in, Frontier &out, bool output,
   a.out_list = out.list;
   a.out_bits = out.bits;
   a.cnt = r.cnt;
-  if (!r.plan) {
+  const bool gaps = g->nslots != g->m;
+  bool planned = r.plan || (g->m > kSumDenseEdges && g->m > kSumDense * g->n);
+  if (!planned && g->nslots > kSumLarge) {
+    uint64_t *h = nullptr;
+    BYO_TRY(pinned(ctx, 4096, (void **)&h));
+    launch(ctx, gaps ? k_sum_probe<true> : k_sum_probe<false>, dim3(1), dim3(1024), 0, a, r.cnt + 3);
+    BYO_CU(ctx, cudaMemcpyAsync(h, r.cnt + 3, 8, cudaMemcpyDeviceToHost, ctx->stream));
+    BYO_CU(ctx, cudaStreamSynchronize(ctx->stream));
+    planned = *h != 0;
+  }
+  if (!planned) {
     a.plan.count = r.cnt + kEmCounts;
     a.plan.direct = true;
     BYO_TRY(ws(g, WS_DEFER, g->n + 1, &a.plan.list));
-    const bool gaps = g->nslots != g->m;
-    // the longest run there can be
-    const uint64_t longest = gaps ? g->nslots : std::min(g->n, g->m);
-    const dim3 lanes(grid_for(ctx, (g->n + 31) / 32 * 32, 256)), ctas(ctx->num_sms),
-        warps(grid_for(ctx, g->nslots / kSumShort * 32, 256, 4));
-    const auto direct = gaps ? k_em_sum_direct<kDivide, true> : k_em_sum_direct<kDivide, false>;
-    if (g->nslots <= kSumBeside) {
-      launch(ctx, direct, lanes, dim3(256), 0, a);
-      if (longest > kSumShort) launch(ctx, k_em_sum_ctas<kDivide, true>, ctas, dim3(kSumBlock), 0, a);
-      return check_launch(ctx, "edge_map");
-    }
-    a.plan.listed = true;
-    launch(ctx, gaps ? k_sum_long<true> : k_sum_long<false>, dim3(grid_for(ctx, (g->n + 3) / 4, 1024, 2)), dim3(1024), 0,
-           a);
-    BYO_TRY(side_fork(ctx, 0));
-    BYO_TRY(side_fork(ctx, 1));
-    k_em_sum_ctas<kDivide, false><<<ctas, kSumBlock, 0, ctx->side[0]>>>(a);
-    k_em_sum_warps<kDivide><<<warps, 256, 0, ctx->side[1]>>>(a);
-    ctx->launches += 2;
-    launch(ctx, direct, lanes, dim3(256), 0, a);
-    BYO_TRY(side_join(ctx, 0));
-    BYO_TRY(side_join(ctx, 1));
+    const bool thin = g->nslots < 6 * g->n;  // half of 8 would be past the run's end
+    const auto direct = gaps ? (thin ? k_em_sum_direct<kDivide, true, 4> : k_em_sum_direct<kDivide, true, 8>)
+                             : (thin ? k_em_sum_direct<kDivide, false, 4> : k_em_sum_direct<kDivide, false, 8>);
+    launch(ctx, direct, dim3(grid_for(ctx, (g->n + 31) / 32 * 32, 256)), dim3(256), 0, a);
+    // if the longest run that there can be is long
+    if ((gaps ? g->nslots : std::min(g->n, g->m)) > kSumShort)
+      launch(ctx, k_em_sum_ctas<kDivide, true>, dim3(ctx->num_sms), dim3(kSumBlock), 0, a);
     return check_launch(ctx, "edge_map");
   }
-  a.plan = *r.plan;
-  BYO_CU(ctx, cudaMemsetAsync(a.plan.count + 2 * kSumClasses, 0, 8, ctx->stream));
+  if (r.plan) {
+    a.plan = *r.plan;
+    BYO_CU(ctx, cudaMemsetAsync(a.plan.count + 2 * kSumClasses, 0, 8, ctx->stream));
+  } else {
+    BYO_TRY(sum_plan(g, &a.plan));
+  }
   // the three take vertices of their own: side by side, the longest runs' few
   // CTAs leave room for the rest
   BYO_TRY(side_fork(ctx, 0));
@@ -883,7 +888,8 @@ int sum_round(byo_graph *g, SumArgs a, Frontier &in, Frontier &out, bool output,
   k_em_sum_ctas<kDivide, false><<<ctx->num_sms, kSumBlock, 0, ctx->side[0]>>>(a);
   k_em_sum_warps<kDivide><<<grid_for(ctx, g->nslots / kSumLaneMax * 32, 256), 256, 0, ctx->side[1]>>>(a);
   ctx->launches += 2;
-  launch(ctx, k_em_sum_lanes, dim3(grid_for(ctx, g->n, 256)), dim3(256), 0, a);
+  launch(ctx, a.fb || output ? k_em_sum_lanes<true> : k_em_sum_lanes<false>, dim3(grid_for(ctx, g->n, 256)), dim3(256),
+         0, a);
   BYO_TRY(side_join(ctx, 0));
   BYO_TRY(side_join(ctx, 1));
   return check_launch(ctx, "edge_map");
