@@ -834,6 +834,7 @@ struct EmRound {
 // kSumLarge slots on where k_sum_probe says so (8 us and a wait of the host: RMAT 2^24
 // vertices, 16 draws each, 2.0 ms a call by a plan, 2.4 without; 2^20 no difference).
 constexpr uint64_t kSumLarge = 1 << 23, kSumDense = 56, kSumDenseEdges = 1 << 22;
+
 // A dense round of a functor that sums (PR_F, PR_Delta_F): by a plan, or on its
 // own.
 template <bool kDivide>
